@@ -13,9 +13,9 @@ DEFAULT = "/root/reference"
 
 
 def reference_dir():
-    """The reference checkout, or None when it is not on this machine."""
+    """The reference checkout, or None when its sources are not on this machine."""
     d = os.environ.get("CSP_REFERENCE_DIR") or DEFAULT
-    return d if os.path.isdir(d) else None
+    return d if os.path.isdir(os.path.join(d, "fvm_mpi", "src")) else None
 
 
 def reference_file(*parts):
