@@ -150,7 +150,7 @@ class Simulation:
         return out
 
     def autotune(self, repeats=3):
-        """Pick the staged kernel's tile shape by timing (csp_autotune); returns a dict."""
+        """Pick the step kernel's launch shape by timing (csp_autotune); returns a dict."""
         rep = abi.csp_tune_report()
         self._check(self.lib.csp_autotune(self.h, int(repeats), C.byref(rep)))
         cands = [dict(threads=rep.threads[i], segment=rep.segment[i], ms=rep.ms[i]) for i in range(rep.n)]

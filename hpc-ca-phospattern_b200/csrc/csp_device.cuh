@@ -1,5 +1,5 @@
 // csp_device.cuh -- device-side data layout and per-voxel arithmetic shared by the
-// voxel kernels (direct and TMA-staged) and the boundary kernel.
+// voxel kernels (direct and marching) and the boundary kernel.
 //
 // HBM layout of one realisation: for every species two FP32 buffers (the reference's
 // u1 / du pair, species.h:52-53, become a double buffer: a step reads the current
@@ -7,8 +7,11 @@
 // [nx][P] with P = ny*nz rounded up to a multiple of 128 elements, so each x-plane
 // starts on a 512-byte boundary (float) / 128-byte boundary (uint8) and can be moved by
 // 16-byte aligned bulk copies.  Within a plane the index is p = y*nz + z (z fastest,
-// species.c:1513).
+// species.c:1513), where nz is the row length nzv of the grid rounded up to a multiple of
+// 4: a group of 4 positions lies in one row, and every row starts on a 16-byte boundary
+// whatever the grid's size (the positions z >= nzv hold no voxel).
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -21,8 +24,19 @@ constexpr int NS = CSP_MAX_SPECIES;
 constexpr int NB = CSP_MAX_BUFFERS;
 constexpr int PLANE_ALIGN = 128;
 constexpr int DOMAIN_BITS = 7;      // domain id = domain byte & DOMAIN_BITS
-constexpr int CLASS_L = 1024;       // plane positions per chunk of the chunk class table
-constexpr unsigned char CLASS_MIXED = 0xff;
+constexpr unsigned char CODE_MIXED = 0xff;   // group code of a group that is neither uniform nor regular
+// A regular group (group code ND + i): one domain, in each of the directions y-, y+, x-, x+ one
+// neighbour domain for all four voxels (the groups along a domain sheet: nine in ten of a
+// dyad's boundary groups), and at most one SERCA flux each, across the same face.  Pattern i of
+// the realisation holds what they share.  code: bits 0-2 the domain, bits 3-20 the neighbours'
+// (z-: of the first voxel, z+: of the last), y-, y+, x-, x+, 3 bits each, the group's own for
+// those outside the box.  flux: PAT_NONE, or bits 0-2 the face's direction (0..5 in that
+// order), PAT_TO when the group is on the receiving side, bits 4-7 the voxels that take it.
+constexpr int NPAT = 128;
+enum : unsigned { PAT_NONE = 0xffffffffu, PAT_TO = 8u };
+struct GroupPattern {
+  unsigned code, flux;
+};
 // Surrogate domain kinds (RealDesc::sur_kind) and voxel classes (RealDesc::rx_class).
 enum : unsigned { RX_NONE = 0, RX_ELIGIBLE = 1, RX_STIFF = 2 };
 enum : unsigned { RX_CLASS_NONE = 0, RX_CLASS_EXPLICIT = 1, RX_CLASS_NETWORK = 2, RX_CLASS_PLAIN = 3 };
@@ -31,7 +45,8 @@ enum FluxKind : int { FLUX_NONE = 0, FLUX_RYR = 1, FLUX_P_RYR = 2, FLUX_SERCA = 
 
 // Constant description of one realisation (device resident, read-only in kernels).
 struct RealDesc {
-  int nx, ny, nz, P, plane;          // plane = ny*nz
+  int nx, ny, nz, P, plane;          // plane = ny*nz; nz = nzv rounded up to a multiple of 4
+  int nzv;                           // voxels per row
   int ns, nd, ndiff, nbuf;
   int reaction_substep, stochastic_substep;
   int dirichlet;
@@ -63,14 +78,6 @@ struct RealDesc {
   unsigned char* rx_class;           // [nx][P]; positions >= plane stay 0
   float sur_cs[ND][NS], sur_thr2[ND][NS];
   unsigned char sur_kind[ND];
-  // Density-boundary fluxes evaluated inside the voxel kernels.  A voxel's domain byte
-  // holds the domain id in bits 0-2 and a flux pattern index in bits 3-7 (0 = none).
-  // fpat[pattern][k] for neighbour direction k: 0 = no flux, else (slot + 1), with bit 7
-  // set when this voxel is the receiving ("to") side of the pair.
-  unsigned char fpat[32][6];
-  int fslot_species[4];
-  int fslot_kind[4];
-  double fslot_p[4][10];
   float init[ND][NS];                // initial values (Species_init_values, species.c:887-935)
   // Every field holds a value as its deviation from a base: u = base[d][s] + field, with d
   // the voxel's domain.  The base of a species that diffuses is one value for each set of
@@ -97,11 +104,10 @@ struct RealDesc {
   float qunit[ND][NS], qinv[ND][NS];
   float* u[2][NS];                   // the two buffers of every species
   const unsigned char* dom;          // [nx][P]
-  // Chunk class table [nx][ncls]: for plane x and chunk c (positions c*CLASS_L ...
-  // c*CLASS_L + CLASS_L - 1), the domain id when every voxel of planes x-1..x+1 within
-  // nz positions of the chunk lies in that domain with no flux pattern, else CLASS_MIXED.
-  const unsigned char* cls;
-  int ncls;
+  // Group codes [nx][P/4]: the domain id when the voxels of positions 4i..4i+3 and all
+  // their neighbours inside the box lie in it and none receives boundary flux, ND + i for a
+  // regular group of pattern i, else CODE_MIXED.
+  const unsigned char* gcode;
   long long total_steps;
   double dt, h, tabort;
   unsigned long long seed;           // Philox key of the realisation's channel draws
@@ -114,18 +120,24 @@ struct RealCtl {
   long long step;                    // steps taken; the running step has time_ind = step+1
   unsigned cur_mask[2];              // [step&1]: bit s = index of the current buffer of species s
   int stopped;
-  int open_count[2];                 // open channels after the step, by (step+1)&1
+  // open channels after step t at [t % 3]; the slot of step t + 2 is cleared when step t ends
+  int open_count[3];
   double last_closed;                // abort rule bookkeeping
 };
 
-// What a realisation's running step does, for the density-row kernel: written at creation
-// and by the step epilogue for the next step (one 16-byte load per row).
+// What a realisation's running step does (flags: STEP_*), for the voxel and density-row kernels: written at
+// creation and by the step epilogue for the next step (16-byte loads).
+enum : unsigned { STEP_REACT = 1u, STEP_REACT_FAST = 2u, STEP_GATE = 4u };
 struct alignas(16) StepRec {
   unsigned active;                   // not stopped
   unsigned cur;                      // bit s: index of the current buffer of species s
   unsigned updated;                  // species written by the step
   unsigned sub;                      // bit dsi: diffusive index dsi takes its substep (and its fluxes)
+  unsigned pre;                      // species that diffuse this step
+  unsigned flags;                    // STEP_REACT: a reaction step; STEP_REACT_FAST: by the per-species tables
+  unsigned pad[2];
 };
+static_assert(sizeof(StepRec) == 32, "two 16-byte loads");
 
 // A density-boundary row in 32 bytes (two 16-byte loads): the receiving voxel, the other
 // voxel of its first pair, the first pair's law with the SERCA scale inline, and the
@@ -172,8 +184,35 @@ struct FluxRow {
   unsigned char species, dsi, kind, owner, boundary, apply;
   unsigned char doms;     // first pair: domain ids of v0 (bits 0-2) and v1 (bits 3-5)
   unsigned char pad1;
+  int first_pair;         // index of the first pair
+  int pad2[3];
 };
-static_assert(sizeof(FluxRow) == 64, "a flux row is one 64-byte line");
+static_assert(sizeof(FluxRow) % 16 == 0, "whole 16-byte words");
+
+// A voxel of a group with CODE_MIXED.  code: bits 0-2 its domain id, bits 3-20 the ids of the
+// neighbours z-, z+, y-, y+, x-, x+ (3 bits each, its own for those outside the box), bits
+// 21-26 which of them are inside.  The first flux into it is inline, further ones are
+// items[more ...] up to the one marked MIX_LAST.
+// An item's meta: MIX_* flags (bits 0-7), species (8-15), dsi (16-23), domain ids of the voxel
+// (24-26) and of the pair's other voxel (27-29); vo: that voxel; pair: its FluxPair (channels
+// and laws other than the realisation's SERCA).
+// MIX_CHANNEL: an RyR / pRyR (MIX_PRYR) channel, in a voxel's first item only (MixVoxel::chan).
+enum : unsigned { MIX_LAST = 1u, MIX_APPLY = 2u, MIX_TO = 4u, MIX_SERCA = 8u, MIX_OWNER = 16u, MIX_CHANNEL = 0x20u,
+                  MIX_PRYR = 0x40u, MIX_NONE = 0x80u };
+struct alignas(16) MixItem {
+  int vo;
+  unsigned meta;                     // MIX_NONE: no flux
+  int pair;
+  int more;                          // MixVoxel::item: index of the next one
+};
+struct alignas(16) MixVoxel {
+  int v;                             // field index
+  unsigned code;
+  int r;                             // realisation (the device copy: the channel's index in its boundary and, from
+                                     // bit 24, the boundary)
+  int chan;                          // channel of the first item (global index)
+  MixItem item;
+};
 
 struct FluxEntry {
   int pair;
@@ -185,7 +224,38 @@ struct FluxEntry {
 struct FluxParams {
   double p[10];           // RyR_model::params layout (boundaryfluxes.h:54) / SERCA params
   double t_close;
+  double k1;              // RyR laws: 1 - K_0 of the realisation's dt and h (ryr_flux)
 };
+
+// The tables of one realisation that the step kernel keeps in shared memory.
+struct alignas(16) VoxDesc {
+  int nx, ny, nz, nzv, plane, P;
+  unsigned fixq;
+  int dirichlet, any_fixed, sur;
+  int pad[2];
+  // {-kon_dt, -koff_dt, a_dt, j0_dt} of the buffer bound to s in d (RealDesc::rk), each
+  // twice in one 64-bit word: a two-lane operand comes from shared memory as it is, instead
+  // of being packed by two moves per use
+  unsigned long long rk2[ND][NS][4];
+  float* u[2][NS];
+  const unsigned char* dom;
+  const unsigned char* gcode;
+  unsigned char* rx_class;
+  float cdiag[ND][NS];
+  float coef[NS][ND * ND];           // by species (RealDesc::coef is by diffusive index)
+  float fbase0[ND];                  // RealDesc::fbase of species 0
+  float qunit[ND][NS], qinv[ND][NS], dinit[ND][NS];
+  float sur_cs[ND][NS], sur_thr2[ND][NS];
+  double base0[ND];                  // RealDesc::base of species 0
+  double serca;                      // the SERCA law's scale (FluxParams::p[9])
+  FluxParams gate[2];                // RyR, pRyR
+  double dt, dts;                    // time step, gating step
+  unsigned long long seed;
+  unsigned stream;
+  GroupPattern pat[NPAT];
+  unsigned char rmask[ND], fixed_mask[ND], sur_kind[ND];
+};
+static_assert(sizeof(VoxDesc) % 16 == 0, "copied in 16-byte words");
 
 // Species updated at step time_ind, and the subset flagged before the reaction runs
 // (diffusion and boundary fluxes flag their species, species.c:1542, 1746).
@@ -323,9 +393,11 @@ __host__ __device__ inline double serca_flux_fast(double u0, double u1, double s
   return scale * (num / den);
 }
 
-__host__ __device__ inline double ryr_flux(double dt, double h, double u0, double u1, const double* params) {
-  const double K_0 = exp(-2 * dt * 1e15 / (2 * 96485.) * params[6] / (1300. - 0.1) / (h * h * h));
-  return (u0 - u1) * (1 - K_0) / 2;
+// RyR flux with k1 = 1 - K_0, K_0 = exp(-2 dt 1e15 / (2 F) i_unitary / (1300 - 0.1) / h^3), a
+// constant of the run (ryr_k1).
+inline double ryr_k1(double dt, double h, double i_unitary) {
+  return 1 - std::exp(-2 * dt * 1e15 / (2 * 96485.) * i_unitary / (1300. - 0.1) / (h * h * h));
 }
+__host__ __device__ inline double ryr_flux(double u0, double u1, double k1) { return (u0 - u1) * k1 / 2; }
 
 }  // namespace csp

@@ -1,11 +1,11 @@
 // csp_kernels.cuh -- the step kernels.
 //
+//   k_march           (csp_march.cuh) whole steps, any number of them in one launch.
 //   k_voxels_direct   one thread per voxel: diffusion of every species due this step,
 //                     buffer reactions, fixed values (species.c:1501-1702, 1037-1121).
-//   k_voxels_staged   (csp_staged.cuh) the same arithmetic over x-marching tiles staged
-//                     in shared memory by bulk TMA copies.
-//   k_boundaries      channel gating + boundary flux scatter + step epilogue
-//                     (species.c:1704-1957, boundaryfluxes.c:295-359, species.c:3384-3488).
+//   k_boundaries      channel gating + boundary flux scatter after the direct kernel
+//                     (species.c:1704-1957, boundaryfluxes.c:295-359).
+//   k_epilogue        step counter and abort rule (species.c:3384-3488).
 //   k_reduce_*        per (domain, species) min / max / FP64 sum (species.c:2785-2880).
 #pragma once
 #include <cfloat>
@@ -153,13 +153,6 @@ __host__ __device__ inline StepInfo step_info(const RealDesc& D, long long time_
 //  walked per bound species (table rtab); otherwise react_general.
 //  fixed values (species.c:1037-1077): fixed (domain, species) pairs and, with -f, the
 //  outer faces of species 0 are reset to their initial values.
-// Boundary flux of one pair, FP64 (boundaryfluxes.c:12-141), u0 on the "from" side.
-// fslot_p[slot][9] holds the SERCA scale dt*density*Q/(1e-24 h) (serca_flux_fast).
-__device__ __forceinline__ double pair_flux(const RealDesc& D, int slot, double u0, double u1) {
-  return D.fslot_kind[slot] == FLUX_SERCA ? serca_flux_fast(u0, u1, D.fslot_p[slot][9])
-                                          : ryr_flux(D.dt, D.h, u0, u1, D.fslot_p[slot]);
-}
-
 // Surrogate class of one voxel of domain d on a reaction step (RealDesc::sur) from the
 // increments the fast reactions apply (dJ_s = dt_r J_s, buffer_dj; ca = the voxel's Ca,
 // val = the stored deviations): the near-equilibrium test of the surrogate,
@@ -168,7 +161,7 @@ __device__ __forceinline__ double pair_flux(const RealDesc& D, int slot, double 
 // sur_thr2 - kon_dt (tot - b_s) |sum dJ| - (kon_dt ca + koff_dt) |dJ_s|
 // = fma(in, |dJ_s|, fma(nkon (cs - db), |sum dJ|, sur_thr2)), in = nkon ca + nkoff (the
 // voxel is near equilibrium when no margin is negative; a NaN margin counts as
-// non-negative, which keeps the explicit increment).  The staged kernel's two-lane form
+// non-negative, which keeps the explicit increment).  The step kernel's two-lane form
 // rounds every step the same way.
 template <int N>
 __device__ __forceinline__ unsigned rx_classify(const RealDesc& D, int d, float ca, const float (&val)[N]) {
@@ -203,9 +196,7 @@ __device__ __forceinline__ unsigned rx_classify(const RealDesc& D, int d, float 
 template <int N, bool SUR = false, class LoadU, class LoadD>
 __device__ __forceinline__ void voxel_update(const RealDesc& D, const StepInfo& si, unsigned valid, bool on_face,
                                              LoadU ld, LoadD ldd, float (&out)[N], unsigned* cls = nullptr) {
-  const int braw = ldd(6);
-  const int d = braw & DOMAIN_BITS;
-  const int pat = braw >> 3;
+  const int d = ldd(6) & DOMAIN_BITS;
   const unsigned fq = D.fixq & si.updated;        // fixed-point species: out[] holds the increment
   float val[N];
 #pragma unroll
@@ -235,24 +226,6 @@ __device__ __forceinline__ void voxel_update(const RealDesc& D, const StepInfo& 
       }
       const float* c = &D.coef[D.dsi_of[s]][d * ND];
       out[s] = uniform ? diffuse_uniform(c[d], u, un) : diffuse_general(c, dn, u, un);
-      if (pat) {
-        // density-boundary fluxes across this voxel's faces (Species_step_boundary_fluxes,
-        // species.c:1751-1807: du[to] += J, du[from] -= J), after diffusion, before reactions
-        double acc = 0.0;
-        bool any = false;
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-          const int code = D.fpat[pat][k];
-          if (!code) continue;
-          const int slot = (code & 0x7f) - 1;
-          if (D.fslot_species[slot] != s) continue;
-          const double self = (double)u + D.base[d][s], other = (double)un[k] + D.base[dn[k]][s];
-          if (code & 0x80) acc += pair_flux(D, slot, other, self);
-          else acc -= pair_flux(D, slot, self, other);
-          any = true;
-        }
-        if (any) out[s] = (float)((double)out[s] + acc);
-      }
     }
   }
   if (si.react) {
@@ -283,19 +256,19 @@ __device__ __forceinline__ void voxel_update(const RealDesc& D, const StepInfo& 
 }
 
 // One thread per voxel; blockIdx.y = realisation.
-__global__ void __launch_bounds__(256) k_voxels_direct(const RealDesc* __restrict__ descs, RealCtl* __restrict__ ctl,
+__global__ void __launch_bounds__(256) k_voxels_direct(const RealDesc* __restrict__ descs,
+                                                        const RealCtl* __restrict__ ctl,
                                                         int* __restrict__ err) {
   __shared__ StepInfo s_si;
   __shared__ unsigned s_cur;
   const int r = blockIdx.y;
   const RealDesc& D = descs[r];
-  RealCtl& C = ctl[r];
+  const RealCtl& C = ctl[r];
   if (C.stopped) return;
   if (threadIdx.x == 0) {
     const long long k = C.step;
     s_si = step_info(D, k + 1);
     s_cur = C.cur_mask[k & 1];
-    if (blockIdx.x == 0) C.cur_mask[(k + 1) & 1] = s_cur ^ s_si.updated;
   }
   __syncthreads();
   const StepInfo si = s_si;
@@ -308,8 +281,9 @@ __global__ void __launch_bounds__(256) k_voxels_direct(const RealDesc* __restric
   const int p = v - x * plane;
   const int y = p / nz;
   const int z = p - y * nz;
+  if (z >= D.nzv) return;
   const long long idx = (long long)x * D.P + p;
-  const unsigned valid = (z > 0 ? 1u : 0u) | (z < nz - 1 ? 2u : 0u) | (y > 0 ? 4u : 0u) |
+  const unsigned valid = (z > 0 ? 1u : 0u) | (z < D.nzv - 1 ? 2u : 0u) | (y > 0 ? 4u : 0u) |
                          (y < D.ny - 1 ? 8u : 0u) | (x > 0 ? 16u : 0u) | (x < D.nx - 1 ? 32u : 0u);
   // out-of-box neighbours read the voxel itself, so every address stays inside the field
   const long long off[6] = {(valid & 1u) ? -1ll : 0ll, (valid & 2u) ? 1ll : 0ll,
@@ -337,16 +311,20 @@ __device__ __forceinline__ int gate(const FluxParams& fp, int state, double c0, 
                                     unsigned long long seed, unsigned r, unsigned ch, unsigned boundary,
                                     long long time_ind) {
   const double* p = fp.p;
-  if (p[8] > 0) {
-    if (p[8] <= t + dts) return 0;
-    return state;
-  }
-  const double kc = fmax(fmin(pow(c0 / p[0], p[5]), p[1]), p[7]);
-  const double ko = fmax(fmin(pow(c0 / p[9], p[2]), p[3]), p[4]);
+  if (p[8] > 0) return p[8] <= t + dts ? 0 : state;
+  if (state != 0 && state != 1) return state;
+  // closed: opens with rate ko = clamp(pow(c0 / p[9], p[2]), p[4], p[3]); open: closes with
+  // kc = clamp(pow(c0 / p[0], p[5]), p[7], p[1]).  The draw is compared with the clamp's bounds
+  // first: above the upper one nothing happens whatever the rate, up to the lower one it does,
+  // and dts times the bounds is about 1e-5, so nearly every step is decided without the power
+  // (with the same outcome: the product is monotone in the rate)
+  const double lo = state == 0 ? p[4] : p[7], hi = fmax(state == 0 ? p[3] : p[1], lo);
   const double rv = channel_uniform(seed, r, ch, boundary, time_ind);
-  if (state == 0) return rv <= dts * ko ? 1 : 0;
-  if (state == 1) return rv <= dts * kc ? 0 : 1;
-  return state;
+  if (rv > dts * hi) return state;
+  if (rv <= dts * lo) return 1 - state;
+  const double rate = state == 0 ? fmax(fmin(pow(c0 / p[9], p[2]), p[3]), p[4])
+                                 : fmax(fmin(pow(c0 / p[0], p[5]), p[1]), p[7]);
+  return rv <= dts * rate ? 1 - state : state;
 }
 
 // Flux of one pair at this step, with the channel gated first (a discrete pair flows
@@ -357,8 +335,8 @@ template <bool CH>
 __device__ __forceinline__ bool pair_step(const RealDesc& D, RealCtl* ctl_r, int species, int kind, int dsi,
                                           int channel, int local_channel, int boundary, int owner, long long v0,
                                           long long v1, int doms, const FluxParams& fp,
-                                          const float* __restrict__ uold, const float* __restrict__ ca,
-                                          unsigned char* __restrict__ states, int nch, long long k, bool stoch,
+                                          const float* uold, const float* ca, unsigned char* states, int nch,
+                                          long long k, bool stoch,
                                           double& J) {
   const long long ti = k + 1;
   const int d0 = doms & DOMAIN_BITS, d1 = (doms >> 3) & DOMAIN_BITS;
@@ -366,18 +344,18 @@ __device__ __forceinline__ bool pair_step(const RealDesc& D, RealCtl* ctl_r, int
     const int s_old = states[(k & 1) * (long long)nch + channel];
     int s_new = s_old;
     if (stoch && kind != FLUX_SERCA)
-      s_new = gate(fp, s_old, (double)__ldg(ca + v1) + D.base[d1][0], (double)ti * D.dt, D.dt * D.stochastic_substep,
+      s_new = gate(fp, s_old, (double)ca[v1] + D.base[d1][0], (double)ti * D.dt, D.dt * D.stochastic_substep,
                    D.seed, D.stream, (unsigned)local_channel, (unsigned)boundary, ti);
     if (owner) {
       states[((k + 1) & 1) * (long long)nch + channel] = (unsigned char)s_new;
-      if (s_new == 1) atomicAdd(&ctl_r->open_count[(k + 1) & 1], 1);
+      if (s_new == 1) atomicAdd(&ctl_r->open_count[(k + 1) % 3], 1);
     }
     if (s_new != 1) return false;
   }
   if (ti % D.substeps[dsi] != 0) return false;
-  const double u0 = (double)__ldg(uold + v0) + D.base[d0][species];
-  const double u1 = (double)__ldg(uold + v1) + D.base[d1][species];
-  J = kind == FLUX_SERCA ? serca_flux_fast(u0, u1, fp.p[9]) : ryr_flux(D.dt, D.h, u0, u1, fp.p);
+  const double u0 = (double)uold[v0] + D.base[d0][species];
+  const double u1 = (double)uold[v1] + D.base[d1][species];
+  J = kind == FLUX_SERCA ? serca_flux_fast(u0, u1, fp.p[9]) : ryr_flux(u0, u1, fp.k1);
   return true;
 }
 
@@ -437,10 +415,13 @@ __global__ void __launch_bounds__(256, CH ? 4 : 8) k_boundaries(const RealDesc* 
 __host__ __device__ inline void write_steprec(const RealDesc& D, const RealCtl& C, StepRec& R) {
   unsigned pre, updated, sub;
   step_masks(D, C.step + 1, pre, updated, sub);
+  const StepInfo si = step_info(D, C.step + 1);
   R.active = C.stopped ? 0u : 1u;
   R.cur = C.cur_mask[C.step & 1];
   R.updated = updated;
   R.sub = sub;
+  R.pre = si.pre;
+  R.flags = (si.react ? STEP_REACT : 0u) | (si.react_fast ? STEP_REACT_FAST : 0u);
 }
 
 // Density-boundary rows (voxels touched by density pairs only: the SERCA sheets), one
@@ -481,7 +462,7 @@ __global__ void __launch_bounds__(256, 8) k_density_rows(const RealDesc* __restr
     const bool to = meta1 & DROW_TO;
     const double u0 = to ? uo : us, u1 = to ? us : uo;
     const double J = (meta1 & DROW_SERCA) ? serca_flux_fast(u0, u1, __hiloint2double(b.y, b.x))
-                                          : ryr_flux(D.dt, D.h, u0, u1, params[meta0 & 0xffffu].p);
+                                          : ryr_flux(u0, u1, params[meta0 & 0xffffu].k1);
     acc += to ? J : -J;
     any = true;
     if (write_from) unew[a.y] = (float)((double)nvo + -J);       // the "from" voxel's own row
@@ -494,12 +475,24 @@ __global__ void __launch_bounds__(256, 8) k_density_rows(const RealDesc* __restr
     const FluxParams& fp = params[pr.param];
     const double u0 = (double)__ldg(uold + pr.v0) + D.base[pr.doms & DOMAIN_BITS][sp];
     const double u1 = (double)__ldg(uold + pr.v1) + D.base[(pr.doms >> 3) & DOMAIN_BITS][sp];
-    const double J = pr.kind == FLUX_SERCA ? serca_flux_fast(u0, u1, fp.p[9]) : ryr_flux(D.dt, D.h, u0, u1, fp.p);
+    const double J = pr.kind == FLUX_SERCA ? serca_flux_fast(u0, u1, fp.p[9]) : ryr_flux(u0, u1, fp.k1);
     acc += (double)en.sign * J;
     any = true;
   }
   if (any && write) unew[a.x] = (float)((double)nv + acc);
 }
+
+// The boundary work: voxels with a channel pair (the longest chains), the others, and what
+// they read.
+struct MixArgs {
+  const MixVoxel* chan;
+  const MixVoxel* vox;
+  const MixItem* items;
+  const FluxPair* pairs;
+  const FluxParams* params;
+  unsigned char* states;             // [2][nch]
+  int nch;
+};
 
 // Step epilogue, one thread per realisation, after the boundary kernel: advance the
 // step counter, apply the abort rule (species.c:3476-3486) on the openness counted by
@@ -520,8 +513,9 @@ __global__ void k_epilogue(const RealDesc* __restrict__ descs, RealCtl* __restri
   const RealDesc& D = descs[r];
   const long long k = C.step;
   const long long ti = k + 1;
-  const int open = C.open_count[(k + 1) & 1];
-  C.open_count[k & 1] = 0;
+  const int open = C.open_count[ti % 3];
+  C.open_count[(ti + 2) % 3] = 0;
+  C.cur_mask[ti & 1] = rec[r].cur ^ rec[r].updated;
   C.step = ti;
   if (D.has_channels && D.tabort != 0) {
     const double tt = (double)ti * D.dt;
@@ -537,6 +531,49 @@ __global__ void k_epilogue(const RealDesc* __restrict__ descs, RealCtl* __restri
   if (flags) flags[r] = C.stopped;
 }
 
+// Initial fields of one realisation: species blockIdx.y of the first buffers (consecutive
+// fields of `elems` floats from u on), every position from its domain's value.
+struct InitTable {
+  float v[ND][NS];
+};
+__global__ void k_init_fields(const unsigned char* __restrict__ dom, float* __restrict__ u, size_t elems,
+                              long long quads, const __grid_constant__ InitTable init) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= quads) return;
+  const int s = blockIdx.y;
+  const uchar4 d = reinterpret_cast<const uchar4*>(dom)[i];
+  reinterpret_cast<float4*>(u + s * elems)[i] = make_float4(init.v[d.x][s], init.v[d.y][s], init.v[d.z][s],
+                                                            init.v[d.w][s]);
+}
+
+// Group codes of one realisation (RealDesc::gcode), one thread per group, from its domain
+// bytes.
+__global__ void k_group_codes(const unsigned char* __restrict__ dom, unsigned char* __restrict__ code, int nx, int ny,
+                              int nz, int nzv, int P) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= (long long)nx * (P / 4)) return;
+  const int x = (int)(i / (P / 4)), p = (int)(i - (long long)x * (P / 4)) * 4;
+  const int y = p / nz, z0 = p - y * nz;
+  unsigned char c = CODE_MIXED;
+  if (y < ny && z0 < nzv) {
+    const unsigned char* g = dom + (long long)x * P + p;
+    const unsigned char d = g[0];
+    bool same = true;
+    for (int j = 0; j < 4 && z0 + j < nzv; j++) {
+      const unsigned char* v = g + j;
+      same = same && v[0] == d;
+      if (z0 + j > 0) same = same && v[-1] == d;
+      if (z0 + j < nzv - 1) same = same && v[1] == d;
+      if (y > 0) same = same && v[-nz] == d;
+      if (y < ny - 1) same = same && v[nz] == d;
+      if (x > 0) same = same && v[-(long long)P] == d;
+      if (x < nx - 1) same = same && v[P] == d;
+    }
+    if (same) c = d;
+  }
+  code[i] = c;
+}
+
 // Output reductions: partial min / max / sum over a block for one species of one
 // realisation, then a fixed-order final pass (deterministic FP64 sums).
 __global__ void __launch_bounds__(256) k_reduce_partial(const RealDesc* __restrict__ descs,
@@ -550,8 +587,9 @@ __global__ void __launch_bounds__(256) k_reduce_partial(const RealDesc* __restri
   for (int d = 0; d < ND; d++) { mn[d] = FLT_MAX; mx[d] = FLT_MIN; sm[d] = 0.0; }
   const long long nvox = (long long)D.nx * D.plane;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvox; v += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(v / D.plane);
-    const long long idx = (long long)x * D.P + (v - (long long)x * D.plane);
+    const int x = (int)(v / D.plane), p = (int)(v - (long long)x * D.plane);
+    if (p % D.nz >= D.nzv) continue;
+    const long long idx = (long long)x * D.P + p;
     const int d = D.dom[idx] & DOMAIN_BITS;
     const double val = ((D.fixq >> s & 1u) ? (double)q_bits(u[idx]) * D.qunit[d][s] : (double)u[idx]) + D.base[d][s];
 #pragma unroll

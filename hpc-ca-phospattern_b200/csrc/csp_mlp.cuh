@@ -34,7 +34,8 @@
 #include <cuda_runtime.h>
 
 #include "csp_device.cuh"
-#include "csp_staged.cuh"   // mbarrier helpers and the bounded wait
+#include "csp_kernels.cuh"  // buffer_dj, the fixed-point fields, step_info
+#include "csp_ptx.cuh"      // mbarrier helpers and the bounded wait
 
 namespace csp {
 
@@ -753,7 +754,7 @@ __device__ __forceinline__ void rx_fallback(const RxConst& kc, int n, double dt,
 
 __device__ __forceinline__ bool rx_on_face(const RealDesc& D, int x, int p) {
   const int c1 = p / D.nz, c2 = p - c1 * D.nz;
-  return x == 0 || x == D.nx - 1 || c1 == 0 || c1 == D.ny - 1 || c2 == 0 || c2 == D.nz - 1;
+  return x == 0 || x == D.nx - 1 || c1 == 0 || c1 == D.ny - 1 || c2 == 0 || c2 == D.nzv - 1;
 }
 
 // One voxel's old state: deviations dev[] (Ca and the slots' species) and the values
@@ -1252,7 +1253,9 @@ __global__ void k_mlp_harvest(const RealDesc* __restrict__ descs, const RealCtl*
   const long long nvox = (long long)D.nx * D.P;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvox;
        v += (long long)gridDim.x * blockDim.x) {
-    if ((int)(v % D.P) >= D.plane) continue;
+    const int c0 = (int)(v / D.P), p = (int)(v - (long long)c0 * D.P);
+    const int c1 = p / D.nz, c2 = p - c1 * D.nz;
+    if (p >= D.plane || c2 >= D.nzv) continue;
     const int d = D.dom[v] & DOMAIN_BITS;
     if (!((elig[r] >> d) & 1u)) continue;
     const float c = __fadd_rn(D.fbase[d][0], D.u[cur & 1u][0][v]);
@@ -1263,7 +1266,10 @@ __global__ void k_mlp_harvest(const RealDesc* __restrict__ descs, const RealCtl*
       atomicAdd(&s_hist[max(bin, 0)], 1u);
       continue;
     }
-    unsigned ctr[4] = {(unsigned)v, (unsigned)(v >> 32), (unsigned)r, 0x68727374u}, rr[4];
+    // the draw's counter is the voxel's index in rows without padding
+    const long long vi = (long long)c0 * ((D.ny * D.nzv + PLANE_ALIGN - 1) / PLANE_ALIGN * PLANE_ALIGN) +
+                         c1 * D.nzv + c2;
+    unsigned ctr[4] = {(unsigned)vi, (unsigned)(vi >> 32), (unsigned)r, 0x68727374u}, rr[4];
     philox4x32(ctr, (unsigned)seed, (unsigned)(seed >> 32), rr);
     if (((double)rr[0] + 0.5) * (1.0 / 4294967296.0) >= prob[max(bin, 0)]) continue;
     const unsigned long long slot = atomicAdd(cursor, 1ull);

@@ -3,9 +3,7 @@
 // Host side: derive every per-realisation constant from the model and options exactly
 // as the reference setup does (species.c:95-884, geometry.c:96-344,
 // boundaryfluxes.c:361-605), build the boundary-flux rows, allocate HBM, and drive the
-// step kernels (direct launches, or replay of a captured CUDA graph of STEPS_PER_GRAPH
-// steps: the kernels read the step index from device memory, so one graph serves
-// every cycle).
+// step kernel.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,7 +21,7 @@
 #include <vector>
 
 #include "csp_kernels.cuh"
-#include "csp_staged.cuh"
+#include "csp_march.cuh"
 #include "csp_mlp.cuh"
 
 using namespace csp;
@@ -31,6 +29,7 @@ using namespace csp;
 namespace {
 
 constexpr int STEPS_PER_GRAPH = 16;
+constexpr int64_t MARCH_STEPS_MAX = 4096;   // steps per launch of the step kernel (a launch stays below a second)
 constexpr int PHASE_SAMPLE = 16;            // steps timed per advance call (csp_set_phase_timing)
 thread_local char g_create_error[512];
 
@@ -45,7 +44,10 @@ struct HostReal {
   size_t field_elems;             // n0*P
   int perm[3];                    // device axis i holds physical axis perm[i]
   int nphys[3];                   // species voxels per physical axis
-  std::vector<unsigned char> cls; // chunk class table (RealDesc::cls)
+  std::vector<GroupPattern> pat;  // regular groups (GroupPattern)
+  double serca = 0.0;             // scale of the SERCA law (FluxParams::p[9])
+  FluxParams gate[2] = {};        // RyR, pRyR
+  std::vector<double> acc;        // prefix sums of the planes' costs (march_cut)
   // padded linear device index of physical species voxel (x, y, z)
   long long dev_index(int x, int y, int z) const {
     const int c[3] = {x, y, z};
@@ -85,29 +87,53 @@ static void choose_axes(const csp_model& m, int perm[3]) {
   perm[2] = swap ? rest[0] : rest[1];
 }
 
-// Chunk class table of one realisation from its device-layout domain bytes (see
-// RealDesc::cls).
-static void chunk_classes(const RealDesc& D, const std::vector<unsigned char>& dom, std::vector<unsigned char>& cls) {
-  const int nch = (D.plane + CLASS_L - 1) / CLASS_L;
-  cls.assign((size_t)D.nx * nch, CLASS_MIXED);
-  std::vector<unsigned char> pu((size_t)D.nx * nch, CLASS_MIXED);
-  for (int q = 0; q < D.nx; q++)
-    for (int c = 0; c < nch; c++) {
-      const int lo = std::max(0, c * CLASS_L - D.nz), hi = std::min(D.plane, c * CLASS_L + CLASS_L + D.nz);
-      const unsigned char* row = dom.data() + (size_t)q * D.P;
-      const unsigned char d = row[lo];
-      bool same = d <= DOMAIN_BITS;
-      for (int p = lo + 1; same && p < hi; p++) same = row[p] == d;
-      if (same) pu[(size_t)q * nch + c] = d;
+// The step kernel's tables of one realisation (VoxDesc) from its descriptor, its patterns
+// and its SERCA scale.
+static VoxDesc make_vox_desc(const HostReal& hr) {
+  const RealDesc& D = hr.desc;
+  VoxDesc v;
+  memset(&v, 0, sizeof v);
+  std::copy(hr.pat.begin(), hr.pat.end(), v.pat);
+  v.serca = hr.serca;
+  v.gate[0] = hr.gate[0];
+  v.gate[1] = hr.gate[1];
+  v.dt = D.dt;
+  v.dts = D.dt * D.stochastic_substep;
+  v.seed = D.seed;
+  v.stream = D.stream;
+  for (int d = 0; d < ND; d++) v.base0[d] = D.base[d][0];
+  v.nx = D.nx; v.ny = D.ny; v.nz = D.nz; v.nzv = D.nzv; v.plane = D.plane; v.P = D.P;
+  v.fixq = D.fixq;
+  v.dirichlet = D.dirichlet;
+  v.sur = D.sur;
+  auto twice = [](float f) {
+    unsigned b;
+    memcpy(&b, &f, sizeof b);
+    return (unsigned long long)b << 32 | b;
+  };
+  for (int d = 0; d < ND; d++) {
+    v.rmask[d] = D.rmask[d];
+    v.fixed_mask[d] = D.fixed_mask[d];
+    v.sur_kind[d] = D.sur_kind[d];
+    v.any_fixed |= D.fixed_mask[d];
+    v.fbase0[d] = D.fbase[d][0];
+    for (int s = 0; s < NS; s++) {
+      const float4 k = D.rk[d][s];
+      v.rk2[d][s][0] = twice(k.x); v.rk2[d][s][1] = twice(k.y);
+      v.rk2[d][s][2] = twice(k.z); v.rk2[d][s][3] = twice(k.w);
     }
-  for (int x = 0; x < D.nx; x++)
-    for (int c = 0; c < nch; c++) {
-      const unsigned char d = pu[(size_t)x * nch + c];
-      if (d == CLASS_MIXED) continue;
-      if (x > 0 && pu[(size_t)(x - 1) * nch + c] != d) continue;
-      if (x + 1 < D.nx && pu[(size_t)(x + 1) * nch + c] != d) continue;
-      cls[(size_t)x * nch + c] = d;
-    }
+  }
+  for (int s = 0; s < NS; s++)
+    if (D.dsi_of[s] >= 0) memcpy(v.coef[s], D.coef[D.dsi_of[s]], sizeof v.coef[s]);
+  memcpy(v.u, D.u, sizeof v.u);
+  v.dom = D.dom; v.gcode = D.gcode; v.rx_class = D.rx_class;
+  memcpy(v.cdiag, D.cdiag, sizeof v.cdiag);
+  memcpy(v.qunit, D.qunit, sizeof v.qunit);
+  memcpy(v.qinv, D.qinv, sizeof v.qinv);
+  memcpy(v.dinit, D.dinit, sizeof v.dinit);
+  memcpy(v.sur_cs, D.sur_cs, sizeof v.sur_cs);
+  memcpy(v.sur_thr2, D.sur_thr2, sizeof v.sur_thr2);
+  return v;
 }
 
 }  // namespace
@@ -121,8 +147,9 @@ struct csp_handle {
   // device memory
   float* d_fields = nullptr;
   unsigned char* d_dom = nullptr;
-  unsigned char* d_cls = nullptr;
+  unsigned char* d_gcode = nullptr;  // group codes of every realisation (RealDesc::gcode)
   RealDesc* d_desc = nullptr;
+  VoxDesc* d_vdesc = nullptr;
   RealCtl* d_ctl = nullptr;
   FluxRow* d_rows = nullptr;
   FluxEntry* d_entries = nullptr;
@@ -150,6 +177,12 @@ struct csp_handle {
   // rows are realisation-major: the rows of realisation r are [first[r], first[r+1]) of the
   // compact density rows, the density-only FluxRows and the channel FluxRows
   std::vector<int> drow_first, krow_first, crow_first;
+  // voxels at domain boundaries (MixArgs), without and with a channel pair, and their flux
+  // items; realisation-major like the rows
+  MixVoxel* d_mix = nullptr;
+  MixVoxel* d_mixc = nullptr;
+  MixItem* d_items = nullptr;
+  std::vector<int> mix_first, mixc_first;
   // csp_run_states: host-to-device stream, staging (two input and two output slots), per
   // step stop flags
   cudaStream_t in_stream = nullptr;
@@ -161,7 +194,7 @@ struct csp_handle {
   int max_plane_vox = 0;
   long long max_vox = 0;
   long long max_field = 0;           // max n0*P (padded planes)
-  int kernel = 0;                 // 0 staged, 1 direct
+  int kernel = 0;                 // 0 march, 1 direct
   int inject_wait = 0;            // csp_test_wait_timeout armed (direct launches, no graph)
   // csp_set_phase_timing: the first steps of every advance call run as direct launches
   // with events between the step's kernels; the sample's per-phase device time, scaled to
@@ -172,11 +205,14 @@ struct csp_handle {
   int64_t phase_call_steps = 0;
   double phase_ms[CSP_NUM_PHASES] = {};
   int64_t phase_steps = 0;
-  StagedPlan plan;
+  // launches of the step kernel: the variant, its resident CTAs, and the teams and units for
+  // every range of realisations asked for so far
+  int ms = 5;
+  unsigned fixq = 0;
+  int ctas = 0;
+  size_t l2 = 0;
+  std::vector<MarchPlan> plans;
   cudaGraphExec_t graph = nullptr;
-  int graph_kernel = -1;
-  int graph_plan = -1;
-  int plan_epoch = 0;                       // bumped when the autotuner replaces the plan
   int graph_surrogate = 0;
   int graph_sur_tc = 0;
   // learned reaction surrogate (csp_set_surrogate)
@@ -355,9 +391,84 @@ int derive(const csp_model& m, const csp_options& o, Derived& dv, std::string& e
   return CSP_OK;
 }
 
-struct PairHost {
-  FluxPair p;
-};
+// The voxels of realisation r's groups that carry CODE_MIXED, in index order.
+void mix_voxels(const RealDesc& D, int r, const unsigned char* code,
+                const std::vector<unsigned char>& dom, std::vector<MixVoxel>& out) {
+  for (int x = 0; x < D.nx; x++)
+    for (int y = 0; y < D.ny; y++) {
+      const int row = x * D.P + y * D.nz;
+      for (int g = 0; g < D.nz / 4; g++) {
+        if (code[row / 4 + g] != CODE_MIXED) continue;
+        for (int z = 4 * g; z < std::min(4 * g + 4, D.nzv); z++) {
+          const int v = row + z;
+          const unsigned valid = (z > 0 ? 1u : 0u) | (z < D.nzv - 1 ? 2u : 0u) | (y > 0 ? 4u : 0u) |
+                                 (y < D.ny - 1 ? 8u : 0u) | (x > 0 ? 16u : 0u) | (x < D.nx - 1 ? 32u : 0u);
+          const int off[6] = {-1, 1, -D.nz, D.nz, -D.P, D.P};
+          const unsigned d = dom[v] & DOMAIN_BITS;
+          unsigned c = d | valid << 21;
+          for (int k = 0; k < 6; k++)
+            c |= ((valid >> k & 1u) ? dom[v + off[k]] & (unsigned)DOMAIN_BITS : d) << (3 + 3 * k);
+          out.push_back({v, c, r, 0, {0, MIX_NONE, 0, 0}});
+        }
+      }
+    }
+}
+
+// Prefix sums of the cost of a realisation's planes (MARCH_US_*): a warp's 128 positions cost
+// what the dearest of their groups does.
+void plane_costs(HostReal& hr, const unsigned char* code, const std::vector<GroupPattern>& pat) {
+  const RealDesc& D = hr.desc;
+  double of[256];
+  for (int c = 0; c < 256; c++)
+    of[c] = c < ND || c == CODE_MIXED          ? MARCH_US_PLANE
+            : c - ND >= (int)pat.size()        ? MARCH_US_PLANE
+            : pat[c - ND].flux == PAT_NONE     ? MARCH_US_REGULAR
+                                               : MARCH_US_FLUX;
+  const int groups = D.plane / 4;
+  hr.acc.assign(1, 0.0);
+  for (int x = 0; x < D.nx; x++) {
+    const unsigned char* row = code + (size_t)x * (D.P / 4);
+    double sum = 0.0;
+    int cols = 0;
+    for (int g = 0; g < groups; g += 32, cols++) {
+      double w = 0.0;
+      for (int i = g; i < std::min(g + 32, groups); i++) w = std::max(w, of[row[i]]);
+      sum += w;
+    }
+    hr.acc.push_back(hr.acc.back() + sum / cols);
+  }
+}
+
+// Whether the four voxels m[0..3] of a group make a regular group (GroupPattern), and what
+// they share.
+bool regular_group(const RealDesc& D, const MixVoxel* m, GroupPattern& g) {
+  const unsigned yx = 0xfffu << 9;                     // neighbours y-, y+, x-, x+
+  const unsigned d = m[0].code & 7u;
+  for (int j = 1; j < 4; j++)
+    if ((m[j].code & 7u) != d || ((m[j].code ^ m[0].code) & yx)) return false;
+  // z inside the group is its own domain; the ends come from the first and the last voxel
+  g.code = ((m[0].code & ~(7u << 6)) | (m[3].code & (7u << 6))) & 0x1fffffu;
+  g.flux = PAT_NONE;
+  int have = 0;
+  for (int j = 0; j < 4; j++) have += !(m[j].item.meta & MIX_NONE);
+  if (have == 0) return true;
+  if (have != 4) return false;
+  const int off[6] = {-1, 1, -D.nz, D.nz, -D.P, D.P};
+  const MixItem& a = m[0].item;
+  int k = 0;
+  while (k < 6 && m[0].v + off[k] != a.vo) k++;
+  if (k == 6 || !(a.meta & MIX_SERCA) || (a.meta >> 8 & 0xffu) != 0) return false;
+  g.flux = (unsigned)k | ((a.meta & MIX_TO) ? PAT_TO : 0u);
+  for (int j = 0; j < 4; j++) {
+    const MixItem& b = m[j].item;
+    if (!(b.meta & MIX_LAST) || ((b.meta ^ a.meta) & ~(MIX_APPLY | MIX_LAST)) || b.vo != m[j].v + off[k] ||
+        !((m[j].code >> (21 + k)) & 1u) || (b.meta >> 27 & 7u) != ((m[j].code >> (3 + 3 * k)) & 7u))
+      return false;
+    if (b.meta & MIX_APPLY) g.flux |= 0x10u << j;
+  }
+  // (across z, inside the group, the other side's base would be another voxel's)
+  return k >= 2;
+}
 
 }  // namespace
 
@@ -407,6 +518,7 @@ static void ryr_params(FluxParams& fp, const csp_ryr_params& p, double t_close) 
   fp.p[4] = p.k_min_open; fp.p[5] = p.n_close; fp.p[6] = p.i_unitary; fp.p[7] = p.k_min_close;
   fp.p[8] = t_close; fp.p[9] = p.Kd_open;
   fp.t_close = t_close;
+  fp.k1 = 0.0;
 }
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }
@@ -428,9 +540,10 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     choose_axes(models[r], hr0.perm);
     hr0.nphys[0] = dv[r].nx; hr0.nphys[1] = dv[r].ny; hr0.nphys[2] = dv[r].nz;
     const int n0 = hr0.nphys[hr0.perm[0]], n1 = hr0.nphys[hr0.perm[1]], n2 = hr0.nphys[hr0.perm[2]];
-    const int plane = n1 * n2;
-    const int P = round_up(plane, PLANE_ALIGN);
-    if ((long long)n0 * P >= (1ll << 31)) { delete h; return fail(nullptr, CSP_EINVAL, "realisation %d: grid too large (2^31 voxels per field)", r); }
+    const long long plane_ll = (long long)n1 * round_up(n2, 4);
+    const long long P_ll = (plane_ll + PLANE_ALIGN - 1) / PLANE_ALIGN * PLANE_ALIGN;
+    const int plane = (int)plane_ll, P = (int)P_ll;
+    if (n0 * P_ll >= (1ll << 31)) { delete h; return fail(nullptr, CSP_EINVAL, "realisation %d: grid too large (2^31 voxels per field)", r); }
     hr0.field_elems = (size_t)n0 * P;
     field_total += hr0.field_elems * 2 * models[r].num_species;
     dom_total += hr0.field_elems;
@@ -447,7 +560,9 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   }
   if (cudaMalloc(&h->d_fields, field_total * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&h->d_dom, dom_total + 256) != cudaSuccess ||
+      cudaMalloc(&h->d_gcode, dom_total / 4 + 16) != cudaSuccess ||
       cudaMalloc(&h->d_desc, n * sizeof(RealDesc)) != cudaSuccess ||
+      cudaMalloc(&h->d_vdesc, n * sizeof(VoxDesc)) != cudaSuccess ||
       cudaMalloc(&h->d_ctl, n * sizeof(RealCtl)) != cudaSuccess ||
       cudaMalloc(&h->d_err, sizeof(int)) != cudaSuccess) {
     csp_destroy(h);
@@ -459,13 +574,13 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   cudaMemsetAsync(h->d_dom, 0, dom_total + 256, h->stream);
 
   std::vector<FluxPair> pairs;
-  std::vector<char> fused;           // pair evaluated inside the voxel kernels
   std::vector<FluxParams> params;
   std::vector<unsigned char> states0;
   std::vector<RealCtl> ctl(n);
   size_t foff = 0, doff = 0;
-  std::vector<float> hostf;
   std::vector<unsigned char> hostd;
+  std::vector<unsigned char> codes(dom_total / 4);      // group codes of every realisation
+  std::vector<MixVoxel> mix;
   for (int r = 0; r < n; r++) {
     const csp_model& m = models[r];
     const csp_options& o = options[r];
@@ -476,7 +591,8 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     const int nd = m.num_domains;
     hr.nd = nd;
     // device axes (choose_axes): nx / ny / nz below are device axes 0 / 1 / 2
-    D.nx = hr.nphys[hr.perm[0]]; D.ny = hr.nphys[hr.perm[1]]; D.nz = hr.nphys[hr.perm[2]];
+    D.nx = hr.nphys[hr.perm[0]]; D.ny = hr.nphys[hr.perm[1]]; D.nzv = hr.nphys[hr.perm[2]];
+    D.nz = round_up(D.nzv, 4);
     D.plane = D.ny * D.nz;
     D.P = round_up(D.plane, PLANE_ALIGN);
     D.ns = m.num_species; D.nd = nd; D.ndiff = d.ndiff; D.nbuf = d.nbuf;
@@ -588,6 +704,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
         foff += hr.field_elems;
       }
     D.dom = h->d_dom + doff;
+    D.gcode = h->d_gcode + doff / 4;
     doff += hr.field_elems;
     hr.dV = d.h * d.h * d.h;
     // species voxel domains (species.c:596-605) and the initial state (species.c:887-935)
@@ -603,19 +720,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
         }
     for (size_t i = 0; i < (size_t)m.N[0] * m.N[1] * m.N[2]; i++) gcount[m.voxels[i]]++;
     for (int dd = 0; dd < ND; dd++) hr.volumes[dd] = dd < nd ? gcount[dd] * m.h_geom * m.h_geom * m.h_geom : 0.0;
-    hostf.assign(hr.field_elems, 0.f);
-    for (int s = 0; s < m.num_species; s++) {
-      for (size_t i = 0; i < hr.field_elems; i++) {
-        const int dd = hostd[i];
-        hostf[i] = D.dinit[dd][s];                                                   // init - base
-        if (D.fixq >> s & 1u) {
-          const int32_t q = (int32_t)std::lrint((double)D.dinit[dd][s] * D.qinv[dd][s]);
-          memcpy(&hostf[i], &q, sizeof q);
-        }
-      }
-      cudaMemcpyAsync(D.u[0][s], hostf.data(), hr.field_elems * sizeof(float), cudaMemcpyHostToDevice, h->stream);
-      cudaStreamSynchronize(h->stream);
-    }
     // -- boundaries, flux map and channels (boundaryfluxes.c:361-605) --
     hr.boundary_channel_base.assign(m.num_boundaries, -1);
     hr.boundary_nch.assign(m.num_boundaries, 0);
@@ -660,6 +764,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       memset(&fp, 0, sizeof fp);
       if (kind == FLUX_RYR) ryr_params(fp, m.ryr, t_close_of(o, "ryr"));
       else if (kind == FLUX_P_RYR) ryr_params(fp, m.p_ryr, t_close_of(o, "p_ryr"));
+      if (kind != FLUX_SERCA) fp.k1 = ryr_k1(d.dt, d.h, fp.p[6]);
       else {
         fp.p[0] = m.serca.v_cyt_to_A_sr; fp.p[1] = m.serca.density; fp.p[2] = m.serca.scale; fp.t_close = -1;
         // serca_flux (boundaryfluxes.c:73-84): dt * density*v*Q * h^2 / (1e-24 h^3)
@@ -667,6 +772,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       }
       const int pidx = (int)params.size();
       params.push_back(fp);
+      if (kind != FLUX_SERCA) hr.gate[kind == FLUX_RYR ? 0 : 1] = fp;
       const csp_boundary& gb = m.boundaries[bi];
       const std::vector<unsigned>& bv = bvox[bi];
       const int np = (int)(bv.size() / 6);
@@ -682,111 +788,35 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
         p.v1 = lin(&bv[6 * i + 3]);
         p.doms = (hostd[p.v0] & DOMAIN_BITS) | (hostd[p.v1] & DOMAIN_BITS) << 3;
         pairs.push_back(p);
-        fused.push_back(0);
-      }
-    }
-    int64_t nfused = 0;
-    // -- density-boundary pairs joining two face-adjacent voxels are evaluated inside the
-    // voxel kernels: per voxel a 6-direction code vector, deduplicated into <= 31 patterns
-    // stored in the domain byte (bits 3-7).  Anything that does not fit stays a flux row.
-    {
-      std::vector<size_t> cand;
-      for (size_t i = 0; i < pairs.size(); i++) {
-        const FluxPair& p = pairs[i];
-#ifdef CSP_FUSE_DENSITY
-        if (p.r == r && p.kind == FLUX_SERCA && p.inner && p.channel < 0) cand.push_back(i);
-#endif
-      }
-      int nslot = 0;
-      int slot_boundary[4] = {-1, -1, -1, -1};
-      auto dev_coords = [&](long long v, int c[3]) {
-        c[0] = (int)(v / D.P);
-        const int rem = (int)(v - (long long)c[0] * D.P);
-        c[1] = rem / D.nz;
-        c[2] = rem - c[1] * D.nz;
-      };
-      bool ok = true;
-      // candidate pairs that can be fused: (pair, slot, k_from, k_to)
-      struct Cand { size_t i; int slot, kf, kt; };
-      std::vector<Cand> cands;
-      for (size_t i : cand) {
-        const FluxPair& p = pairs[i];
-        int a[3], b[3];
-        dev_coords(p.v0, a);
-        dev_coords(p.v1, b);
-        int axis = -1, nd_ = 0;
-        for (int q = 0; q < 3; q++)
-          if (a[q] != b[q]) { nd_++; axis = q; }
-        if (nd_ != 1 || std::abs(a[axis] - b[axis]) != 1) continue;   // not face-adjacent
-        int slot = -1;
-        for (int q = 0; q < nslot; q++)
-          if (slot_boundary[q] == p.boundary) slot = q;
-        if (slot < 0) {
-          if (nslot == 4) continue;
-          slot = nslot++;
-          slot_boundary[slot] = p.boundary;
-          D.fslot_species[slot] = p.species;
-          D.fslot_kind[slot] = p.kind;
-          for (int q = 0; q < 10; q++) D.fslot_p[slot][q] = params[p.param].p[q];
-        }
-        // direction k: device axis 2 -> 0/1, axis 1 -> 2/3, axis 0 -> 4/5 (minus / plus)
-        const int kbase = 2 * (2 - axis);
-        cands.push_back({i, slot, kbase + (b[axis] > a[axis] ? 1 : 0), kbase + (b[axis] > a[axis] ? 0 : 1)});
-      }
-      // per-voxel code vectors; pairs touching voxels whose pattern is not among the 31
-      // most frequent ones go back to the boundary kernel, until the patterns fit
-      std::vector<char> keep(cands.size(), 1);
-      std::unordered_map<long long, std::array<unsigned char, 6>> vc;
-      std::map<std::array<unsigned char, 6>, int> patterns;
-      for (int iter = 0; iter < 64; iter++) {
-        vc.clear();
-        for (size_t q = 0; q < cands.size(); q++) {
-          if (!keep[q]) continue;
-          const FluxPair& p = pairs[cands[q].i];
-          auto& c0 = vc[p.v0];
-          auto& c1 = vc[p.v1];
-          if (c0[cands[q].kf] || c1[cands[q].kt]) { keep[q] = 0; continue; }   // face already used
-          c0[cands[q].kf] = (unsigned char)(cands[q].slot + 1);
-          c1[cands[q].kt] = (unsigned char)((cands[q].slot + 1) | 0x80);
-        }
-        std::map<std::array<unsigned char, 6>, long long> freq;
-        for (auto& kv : vc) freq[kv.second]++;
-        patterns.clear();
-        if ((int)freq.size() <= 31) {
-          for (auto& kv : freq) patterns.emplace(kv.first, (int)patterns.size() + 1);
-          break;
-        }
-        std::vector<std::pair<long long, std::array<unsigned char, 6>>> byf;
-        for (auto& kv : freq) byf.push_back({kv.second, kv.first});
-        std::stable_sort(byf.begin(), byf.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-        std::map<std::array<unsigned char, 6>, int> top;
-        for (int q = 0; q < 31; q++) top.emplace(byf[q].second, 1);
-        for (size_t q = 0; q < cands.size(); q++) {
-          if (!keep[q]) continue;
-          const FluxPair& p = pairs[cands[q].i];
-          if (!top.count(vc[p.v0]) || !top.count(vc[p.v1])) keep[q] = 0;
-        }
-      }
-      std::vector<size_t> taken;
-      for (size_t q = 0; q < cands.size(); q++)
-        if (keep[q]) taken.push_back(cands[q].i);
-      if (patterns.empty() && !vc.empty()) ok = false;
-      if (getenv("CSP_DEBUG"))
-        fprintf(stderr, "csp: realisation %d: %zu density pairs, %zu fused, %zu flux patterns\n", r, cand.size(),
-                ok ? taken.size() : (size_t)0, patterns.size());
-      if (ok && !taken.empty()) {
-        memset(D.fpat, 0, sizeof D.fpat);
-        for (auto& kv : patterns)
-          for (int k = 0; k < 6; k++) D.fpat[kv.second][k] = kv.first[k];
-        for (auto& kv : vc) hostd[kv.first] = (unsigned char)(hostd[kv.first] | (patterns[kv.second] << 3));
-        for (size_t i : taken) fused[i] = 1;
-        nfused = (int64_t)taken.size();
       }
     }
     cudaMemcpyAsync((void*)D.dom, hostd.data(), hr.field_elems, cudaMemcpyHostToDevice, h->stream);
-    chunk_classes(D, hostd, hr.cls);
-    D.ncls = (D.plane + CLASS_L - 1) / CLASS_L;
-    cudaStreamSynchronize(h->stream);
+    {
+      InitTable init;
+      for (int dd = 0; dd < ND; dd++)
+        for (int s = 0; s < NS; s++) {
+          init.v[dd][s] = D.dinit[dd][s];                                            // init - base
+          if (D.fixq >> s & 1u) {
+            const int32_t q = (int32_t)std::lrint((double)D.dinit[dd][s] * D.qinv[dd][s]);
+            memcpy(&init.v[dd][s], &q, sizeof q);
+          }
+        }
+      const long long quads = (long long)hr.field_elems / 4;
+      k_init_fields<<<dim3((unsigned)((quads + 255) / 256), (unsigned)D.ns), 256, 0, h->stream>>>(
+          D.dom, D.u[0][0], hr.field_elems, quads, init);
+    }
+    // group codes, then the voxels of the groups that are not uniform or receive flux
+    {
+      const long long groups = (long long)D.nx * (D.P / 4);
+      const size_t first = (size_t)(D.dom - h->d_dom) / 4;
+      k_group_codes<<<(unsigned)((groups + 255) / 256), 256, 0, h->stream>>>(D.dom, h->d_gcode + first, D.nx, D.ny, D.nz,
+                                                                             D.nzv, D.P);
+      cudaMemcpyAsync(codes.data() + first, h->d_gcode + first, groups, cudaMemcpyDeviceToHost, h->stream);
+      cudaStreamSynchronize(h->stream);
+      for (size_t i = pairs.size(); i-- > 0 && pairs[i].r == r;)
+        codes[first + pairs[i].v0 / 4] = codes[first + pairs[i].v1 / 4] = CODE_MIXED;
+      mix_voxels(D, r, codes.data() + first, hostd, mix);
+    }
     // initial channel states (BoundaryFluxes_init_stochastic_boundaries, boundaryfluxes.c:544-605)
     int ndiscrete = 0;
     for (int bi = 0; bi < m.num_boundaries; bi++) ndiscrete += m.boundaries[bi].type == CSP_BOUNDARY_DISCRETE;
@@ -835,7 +865,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     // info
     csp_info& in = hr.info;
     memset(&in, 0, sizeof in);
-    in.fused_pairs = nfused;
     in.n[0] = d.nx; in.n[1] = d.ny; in.n[2] = d.nz;
     in.subdivisions = d.S; in.h = d.h; in.dt = d.dt;
     in.num_species = m.num_species; in.num_diffusive = d.ndiff;
@@ -856,7 +885,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   std::vector<Side> sides;
   for (int i = 0; i < (int)pairs.size(); i++) {
     const FluxPair& p = pairs[i];
-    if (fused[i]) continue;
     sides.push_back({p.r, p.species, p.v1, i, 1.f, p.channel >= 0 ? 1 : 0});
     if (p.inner) sides.push_back({p.r, p.species, p.v0, i, -1.f, 0});
   }
@@ -880,6 +908,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       row.local_channel = p0.local_channel; row.sign = sides[i].sign;
       row.dsi = (unsigned char)p0.dsi; row.kind = (unsigned char)p0.kind; row.owner = (unsigned char)sides[i].owner;
       row.boundary = (unsigned char)p0.boundary;
+      row.first_pair = sides[i].pair;
       row.doms = (unsigned char)p0.doms;
     }
     j = i + 1;
@@ -900,11 +929,104 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     ph[rr.perm[0]] = c0; ph[rr.perm[1]] = c1; ph[rr.perm[2]] = c2;
     const int S = dv[row.r].S;
     const unsigned char dd = models[row.r].voxels[((size_t)(ph[0] / S) * models[row.r].N[1] + ph[1] / S) * models[row.r].N[2] + ph[2] / S];
-    const bool face = c0 == 0 || c0 == D.nx - 1 || c1 == 0 || c1 == D.ny - 1 || c2 == 0 || c2 == D.nz - 1;
+    const bool face = c0 == 0 || c0 == D.nx - 1 || c1 == 0 || c1 == D.ny - 1 || c2 == 0 || c2 == D.nzv - 1;
     row.apply = !((D.fixed_mask[dd] >> row.species) & 1u) && !(D.dirichlet && row.species == 0 && face);
     rows.push_back(row);
     h->real[row.r].info.flux_rows++;
     i = j;
+  }
+  // the same fluxes by voxel (MixArgs): rows are in (realisation, species, voxel)
+  // order, the items of a voxel in (species, pair) order
+  std::vector<MixItem> items;
+  std::vector<MixVoxel> mixc;           // voxels with a channel pair
+  std::vector<int> places;              // MixVoxel::r of their device copies
+  std::vector<std::vector<GroupPattern>> pats(n);
+  std::vector<int> serca(n, -1);
+  for (const FluxPair& p : pairs)
+    if (p.kind == FLUX_SERCA) serca[p.r] = p.param;
+  {
+    // realisations that may have regular groups: the step kernel's variants with run-time
+    // masks (another realisation's model may select them for the batch) do not know them
+    bool batch = true;
+    for (int r = 0; r < n; r++)
+      batch = batch && h->real[r].desc.ns <= 5 && (h->real[r].desc.fixq & ~(1u << 4)) == 0;
+    std::vector<char> regular(n, 0);
+    for (int r = 0; r < n; r++) regular[r] = batch && march_masks_known(h->real[r].desc);
+    std::vector<int> order(rows.size());
+    for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+      return rows[a].r != rows[b].r ? rows[a].r < rows[b].r : rows[a].v < rows[b].v;
+    });
+    std::vector<MixVoxel> rest;
+    size_t q = 0;
+    MixVoxel group[4] = {};             // the voxels of the group in hand
+    bool chan_of[4] = {};
+    int place_of[4] = {};
+    int ng = 0;
+    auto flush = [&]() {
+      const int r = group[0].r;
+      const RealDesc& D = h->real[r].desc;
+      GroupPattern g;
+      if (ng == 4 && regular[r] && !chan_of[0] && !chan_of[1] && !chan_of[2] && !chan_of[3] &&
+          regular_group(D, group, g)) {
+        std::vector<GroupPattern>& P = pats[r];
+        size_t i = 0;
+        while (i < P.size() && (P[i].code != g.code || P[i].flux != g.flux)) i++;
+        if (i < (size_t)NPAT) {
+          if (i == P.size()) P.push_back(g);
+          codes[(size_t)(D.dom - h->d_dom) / 4 + group[0].v / 4] = (unsigned char)(ND + i);
+          ng = 0;
+          return;
+        }
+      }
+      for (int j = 0; j < ng; j++) {
+        (chan_of[j] ? mixc : rest).push_back(group[j]);
+        if (chan_of[j]) places.push_back(place_of[j]);
+      }
+      ng = 0;
+    };
+    for (MixVoxel m : mix) {
+      bool channel = false, first = true;      // first: only the inline item so far
+      int place = 0;
+      if (ng > 0 && (group[0].r != m.r || group[0].v / 4 != m.v / 4)) flush();
+      while (q < order.size() && rows[order[q]].r == m.r && rows[order[q]].v == m.v) {
+        const FluxRow& rw = rows[order[q++]];
+        auto add = [&](int pair, float sign, int owner) {
+          const FluxPair& p = pairs[pair];
+          const bool to = sign > 0.f, chan = p.channel >= 0;
+          const unsigned d0 = p.doms & DOMAIN_BITS, d1 = (p.doms >> 3) & DOMAIN_BITS;
+          MixItem it;
+          it.vo = (int)(to ? p.v0 : p.v1);
+          it.pair = pair;
+          it.more = 0;
+          it.meta = (rw.apply ? MIX_APPLY : 0u) | (to ? MIX_TO : 0u) |
+                    (p.kind == FLUX_SERCA && !chan && p.param == serca[m.r] ? MIX_SERCA : 0u) | (owner ? MIX_OWNER : 0u) |
+                    (unsigned)p.species << 8 | (unsigned)p.dsi << 16 | (to ? d1 : d0) << 24 | (to ? d0 : d1) << 27;
+          if (m.item.meta & MIX_NONE) {
+            if (chan && p.kind != FLUX_SERCA && p.local_channel < (1 << 24) && p.boundary < 128) {
+              it.meta |= MIX_CHANNEL | (p.kind == FLUX_P_RYR ? MIX_PRYR : 0u);
+              m.chan = p.channel;
+              place = p.local_channel | p.boundary << 24;
+            }
+            m.item = it;
+          } else {
+            MixItem& prev = first ? m.item : items.back();
+            prev.more = (int)items.size();
+            first = false;
+            items.push_back(it);
+          }
+          channel = channel || chan;
+        };
+        add(rw.first_pair, rw.sign, rw.owner);
+        for (int e = rw.more_begin; e < rw.more_end; e++) add(entries[e].pair, entries[e].sign, entries[e].owner);
+      }
+      if (!(m.item.meta & MIX_NONE)) (first ? m.item : items.back()).meta |= MIX_LAST;
+      group[ng] = m;
+      place_of[ng] = place;
+      chan_of[ng++] = channel;
+    }
+    if (ng) flush();
+    mix.swap(rest);
   }
   h->nrows = (int)rows.size();
   // rows touched by density pairs only first (gating-free launch), channel rows after
@@ -976,6 +1098,8 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       for (int i = count - 1; i >= 0; i--) f[r_of(i)] = i;
       for (int r = n - 1; r >= 0; r--) f[r] = std::min(f[r], f[r + 1]);
     };
+    firsts(h->mix_first, (int)mix.size(), [&](int i) { return mix[i].r; });
+    firsts(h->mixc_first, (int)mixc.size(), [&](int i) { return mixc[i].r; });
     firsts(h->drow_first, h->ndrows, [&](int i) { return drows[i].r; });
     firsts(h->krow_first, h->nrows_density, [&](int i) { return rows[i].r; });
     firsts(h->crow_first, h->nrows - h->nrows_density, [&](int i) { return rows[h->nrows_density + i].r; });
@@ -988,25 +1112,27 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   };
   std::vector<unsigned char> st2(2 * (size_t)std::max(h->nch, 1), 0);
   std::copy(states0.begin(), states0.end(), st2.begin());
-  size_t cls_total = 0;
-  for (int r = 0; r < n; r++) cls_total += h->real[r].cls.size();
-  std::vector<unsigned char> cls_all;
-  cls_all.reserve(cls_total);
-  for (int r = 0; r < n; r++) cls_all.insert(cls_all.end(), h->real[r].cls.begin(), h->real[r].cls.end());
-  if (!upload((void**)&h->d_cls, cls_all.empty() ? nullptr : cls_all.data(), cls_all.size())) {
-    csp_destroy(h);
-    return fail(nullptr, CSP_ENOMEM, "device allocation of the chunk class table failed");
-  }
   std::vector<RealDesc> descs(n);
-  for (int r = 0, off = 0; r < n; r++) {
-    h->real[r].desc.cls = h->d_cls + off;
-    off += (int)h->real[r].cls.size();
+  std::vector<VoxDesc> vdescs(n);
+  for (int r = 0; r < n; r++) {
     descs[r] = h->real[r].desc;
+    h->real[r].pat = pats[r];
+    if (serca[r] >= 0) h->real[r].serca = params[serca[r]].p[9];
+    vdescs[r] = make_vox_desc(h->real[r]);
   }
+  if (cudaMemcpyAsync(h->d_gcode, codes.data(), codes.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
+    csp_destroy(h);
+    return fail(nullptr, CSP_ECUDA, "group code upload");
+  }
+  for (size_t i = 0; i < mixc.size(); i++) mixc[i].r = places[i];
+  for (int r = 0; r < n; r++) plane_costs(h->real[r], codes.data() + (size_t)(h->real[r].desc.dom - h->d_dom) / 4, pats[r]);
   std::vector<StepRec> recs(n);
   for (int r = 0; r < n; r++) write_steprec(descs[r], ctl[r], recs[r]);
   bool ok = upload((void**)&h->d_rec, recs.data(), recs.size() * sizeof(StepRec)) &&
             (drows.empty() || upload((void**)&h->d_drows, drows.data(), drows.size() * sizeof(DensityRow))) &&
+            upload((void**)&h->d_mix, mix.empty() ? nullptr : mix.data(), mix.size() * sizeof(MixVoxel)) &&
+            upload((void**)&h->d_mixc, mixc.empty() ? nullptr : mixc.data(), mixc.size() * sizeof(MixVoxel)) &&
+            upload((void**)&h->d_items, items.empty() ? nullptr : items.data(), items.size() * sizeof(MixItem)) &&
             upload((void**)&h->d_rows, rows.empty() ? nullptr : rows.data(), rows.size() * sizeof(FluxRow)) &&
             upload((void**)&h->d_entries, entries.empty() ? nullptr : entries.data(), entries.size() * sizeof(FluxEntry)) &&
             upload((void**)&h->d_pairs, pairs.empty() ? nullptr : pairs.data(), pairs.size() * sizeof(FluxPair)) &&
@@ -1014,6 +1140,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
             upload((void**)&h->d_states, st2.data(), st2.size());
   if (!ok) { csp_destroy(h); return fail(nullptr, CSP_ENOMEM, "device allocation of flux tables failed"); }
   if ((e = cudaMemcpyAsync(h->d_desc, descs.data(), n * sizeof(RealDesc), cudaMemcpyHostToDevice, h->stream)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(h->d_vdesc, vdescs.data(), n * sizeof(VoxDesc), cudaMemcpyHostToDevice, h->stream)) != cudaSuccess ||
       (e = cudaMemcpyAsync(h->d_ctl, ctl.data(), n * sizeof(RealCtl), cudaMemcpyHostToDevice, h->stream)) != cudaSuccess) {
     csp_destroy(h);
     return fail(nullptr, CSP_ECUDA, "descriptor upload: %s", cudaGetErrorString(e));
@@ -1024,8 +1151,29 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     csp_destroy(h);
     return fail(nullptr, CSP_ENOMEM, "device allocation of reduction buffers failed");
   }
-  h->plan = staged_plan(descs);
-  if (staged_prepare(h->plan) != cudaSuccess) h->kernel = 1;
+  {
+    int ns = 0, dev = 0, sms = 0, per_sm = 0, l2 = 0;
+    for (const RealDesc& D : descs) {
+      ns = std::max(ns, D.ns);
+      h->fixq |= D.fixq;
+    }
+    h->ms = ns <= 5 ? 5 : 8;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+    for (int sur = 0; sur < 2 && e == cudaSuccess; sur++) {
+      int k = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, march_kernel(h->ms, h->fixq, sur != 0), MARCH_T,
+                                                        sizeof(MarchShared));
+      per_sm = sur == 0 ? k : std::min(per_sm, k);
+    }
+    if (e != cudaSuccess || per_sm < 1) {
+      csp_destroy(h);
+      return fail(nullptr, CSP_ECUDA, "step kernel: %s", e != cudaSuccess ? cudaGetErrorString(e) : "does not fit an SM");
+    }
+    h->ctas = per_sm * sms;
+    h->l2 = (size_t)l2;
+  }
   e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) { csp_destroy(h); return fail(nullptr, CSP_ECUDA, "setup: %s", cudaGetErrorString(e)); }
   *out = h;
@@ -1035,14 +1183,190 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
 // The kernels of one step, for the realisations [r0, r1) (r1 < 0: all of them, the
 // launches csp_advance captures).  Realisations are independent, so stepping a range
 // gives that range exactly what a step of the whole batch gives it.
-static void launch_voxels(csp_handle* h, int r0 = 0, int r1 = -1) {
-  if (r1 < 0) r1 = h->n;
-  if (h->kernel == 1) {
-    dim3 grid((unsigned)((h->max_vox + 255) / 256), (unsigned)(r1 - r0));
-    k_voxels_direct<<<grid, 256, 0, h->stream>>>(h->d_desc + r0, h->d_ctl + r0, h->d_err);
-  } else {
-    staged_launch(h->plan, h->d_desc, h->d_ctl, h->d_err, h->stream, h->inject_wait != 0, r0, r1, h->surrogate != 0);
+// The fields of a realisation that its steps read and write: both buffers of every species,
+// group codes.
+static double working_set(const RealDesc& D) { return (double)D.nx * D.P * (8.0 * D.ns + 0.25); }
+
+// Teams, their realisations and units for the realisations [r0, r1).  The number of teams is
+// the one with the least estimated time (march_cost; each realisation to the team with the
+// least so far, longest first) among those whose realisations in flight fit in
+// MARCH_L2_SHARE of the L2 cache together (one team always may): with more, each step
+// streams through HBM again (40 grids of 100x100x50: 2, 3, 4, 5, 6 in flight take 211, 183, 205, 243,
+// 267 us per step; three are 0.46 of the 132 MB).  teams / nseg > 0: fixed (csp_autotune).
+constexpr double MARCH_L2_SHARE = 0.5;
+static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPlan& pl) {
+  const int n = r1 - r0;
+  std::vector<int> order(n);
+  for (int i = 0; i < n; i++) order[i] = r0 + i;
+  auto desc = [&](int r) -> const RealDesc& { return h->real[r].desc; };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return working_set(desc(a)) > working_set(desc(b)); });
+  auto columns = [&](int r) { return (desc(r).plane + MARCH_COL - 1) / MARCH_COL; };
+  auto tiles_of = [&](int r) {
+    return (h->mixc_first[r + 1] - h->mixc_first[r] + 31) / 32 + (h->mix_first[r + 1] - h->mix_first[r] + 31) / 32;
+  };
+  int most = 0;
+  for (double sum = 0.0; most < std::min(n, h->ctas);) {
+    sum += working_set(desc(order[most]));
+    if (most > 0 && sum > MARCH_L2_SHARE * (double)h->l2) break;
+    most++;
   }
+  // no more CTAs than the largest realisation has work for, one plane per unit
+  long long need = 1;
+  for (int i = 0; i < n; i++)
+    need = std::max<long long>(need, (long long)desc(order[i]).nx * columns(order[i]) + tiles_of(order[i]));
+  const int W = MARCH_T / 32;
+  auto size_of = [&](int t) { return (int)std::max<long long>(1, std::min<long long>(h->ctas / t, (need + W - 1) / W)); };
+  auto deal = [&](int t, std::vector<std::vector<int>>* out) {
+    const int size = size_of(t);
+    std::vector<double> load(t, 0.0);
+    double last = 0.0;
+    for (int i = 0; i < n; i++) {
+      const RealDesc& D = desc(order[i]);
+      const bool same = i > 0 && D.nx == desc(order[i - 1]).nx && D.plane == desc(order[i - 1]).plane;
+      if (!same) last = march_cost(columns(order[i]), h->real[order[i]].acc, tiles_of(order[i]), size, nullptr);
+      const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      load[k] += last;
+      if (out) (*out)[k].push_back(order[i]);
+    }
+    return *std::max_element(load.begin(), load.end());
+  };
+  int best = std::max(1, std::min({teams, n, h->ctas}));
+  if (teams <= 0) {
+    double tb = 1e300;
+    for (int t = 1; t <= most; t += t < 16 ? 1 : t / 8) {
+      const double c = deal(t, nullptr);
+      if (c < tb) {
+        tb = c;
+        best = t;
+      }
+    }
+  }
+  pl.r0 = r0;
+  pl.r1 = r1;
+  pl.teams = best;
+  pl.size = size_of(best);
+  std::vector<std::vector<int>> team(best);
+  deal(best, &team);
+  std::vector<MarchReal> real;
+  std::vector<int> first(1, 0), cuts, one;
+  for (const auto& t : team) {
+    for (int r : t) {
+      MarchReal m;
+      m.r = r;
+      m.ncol = columns(r);
+      m.nseg = nseg;
+      march_cost(m.ncol, h->real[r].acc, tiles_of(r), pl.size, &m.nseg);
+      if (real.empty()) pl.nseg = m.nseg;
+      march_cut(h->real[r].acc, m.nseg, &one);
+      m.cut0 = (int)cuts.size();
+      cuts.insert(cuts.end(), one.begin(), one.end());
+      m.chan0 = h->mixc_first[r];
+      m.nchan = h->mixc_first[r + 1] - m.chan0;
+      m.vox0 = h->mix_first[r];
+      m.nvox = h->mix_first[r + 1] - m.vox0;
+      real.push_back(m);
+    }
+    first.push_back((int)real.size());
+  }
+  if (cudaMalloc(&pl.d_real, real.size() * sizeof(MarchReal)) != cudaSuccess ||
+      cudaMalloc(&pl.d_first, first.size() * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&pl.d_cuts, cuts.size() * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&pl.d_arrived, (size_t)best * 32 * sizeof(unsigned)) != cudaSuccess)
+    return fail(h, CSP_ENOMEM, "launch plan of %d realisations", n);
+  CUDA_TRY(h, cudaMemcpyAsync(pl.d_real, real.data(), real.size() * sizeof(MarchReal), cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(h, cudaMemcpyAsync(pl.d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(h, cudaMemcpyAsync(pl.d_cuts, cuts.data(), cuts.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(h, cudaMemsetAsync(pl.d_arrived, 0, (size_t)best * 32 * sizeof(unsigned), h->stream));
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  return CSP_OK;
+}
+
+static void free_plan(MarchPlan& p) {
+  cudaFree(p.d_real);
+  cudaFree(p.d_first);
+  cudaFree(p.d_cuts);
+  cudaFree(p.d_arrived);
+  p = MarchPlan();
+}
+
+static int plan_for(csp_handle* h, int r0, int r1, const MarchPlan** out) {
+  for (const MarchPlan& p : h->plans)
+    if (p.r0 == r0 && p.r1 == r1) {
+      *out = &p;
+      return CSP_OK;
+    }
+  MarchPlan p;
+  const int rc = make_plan(h, r0, r1, 0, 0, p);
+  if (rc) {
+    free_plan(p);
+    return rc;
+  }
+  h->plans.push_back(p);
+  *out = &h->plans.back();
+  return CSP_OK;
+}
+
+// nsteps steps of a plan's realisations, or (without MARCH_ADVANCE) parts of the current one.
+// Launched cooperatively when its CTAs wait for one another.  flags: MarchArgs.
+static cudaError_t launch_march(csp_handle* h, const MarchPlan& pl, long long nsteps, unsigned what, int* flags = nullptr) {
+  MarchArgs a;
+  memset(&a, 0, sizeof a);
+  a.descs = h->d_desc;
+  a.vdescs = h->d_vdesc;
+  a.ctl = h->d_ctl;
+  a.rec = h->d_rec;
+  a.real = pl.d_real;
+  a.first = pl.d_first;
+  a.cuts = pl.d_cuts;
+  a.size = pl.size;
+  a.nsteps = nsteps;
+  a.what = what;
+  a.mix.chan = h->d_mixc;
+  a.mix.vox = h->d_mix;
+  a.mix.items = h->d_items;
+  a.mix.pairs = h->d_pairs;
+  a.mix.params = h->d_params;
+  a.mix.states = h->d_states;
+  a.mix.nch = std::max(h->nch, 1);
+  a.arrived = pl.d_arrived;
+  a.flags = flags;
+  a.flag_stride = h->n;
+  a.err = h->d_err;
+  a.inject = h->inject_wait;
+  MarchKernel k = march_kernel(h->ms, h->fixq, h->surrogate != 0);
+  const unsigned grid = (unsigned)(pl.teams * pl.size);
+  if (pl.size == 1 || !(what & (MARCH_ADVANCE | MARCH_REPEAT))) {
+    k<<<grid, MARCH_T, sizeof(MarchShared), h->stream>>>(a);
+    return cudaGetLastError();
+  }
+  cudaError_t e = cudaMemsetAsync(pl.d_arrived, 0, (size_t)pl.teams * 32 * sizeof(unsigned), h->stream);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&a};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(grid), dim3(MARCH_T), args,
+                                     sizeof(MarchShared), h->stream);
+}
+
+static void launch_density_rows(csp_handle* h, int r0, int r1);
+static void launch_channel_rows(csp_handle* h, int r0, int r1);
+static void launch_direct(csp_handle* h, int r0, int r1) {
+  dim3 grid((unsigned)((h->max_vox + 255) / 256), (unsigned)(r1 - r0));
+  k_voxels_direct<<<grid, 256, 0, h->stream>>>(h->d_desc + r0, h->d_ctl + r0, h->d_err);
+}
+
+// Every voxel of the realisations [r0, r1) in their current step, the fluxes included: the
+// step kernel, or the direct kernel followed by the flux-row kernels.
+static int launch_voxels(csp_handle* h, int r0, int r1) {
+  if (h->kernel == 1) {
+    launch_direct(h, r0, r1);
+    launch_density_rows(h, r0, r1);
+    launch_channel_rows(h, r0, r1);
+  } else {
+    const MarchPlan* pl;
+    const int rc = plan_for(h, r0, r1, &pl);
+    if (rc) return rc;
+    CUDA_TRY(h, launch_march(h, *pl, 1, MARCH_STEP & ~MARCH_ADVANCE));
+  }
+  return CSP_OK;
 }
 
 // The flux-row kernels of one step: density-boundary rows (SERCA), then the channel rows
@@ -1119,61 +1443,109 @@ static void launch_epilogue(csp_handle* h, int r0, int r1, int* step_flags) {
                                                            step_flags, h->surrogate ? h->d_sur_queue : nullptr);
 }
 
-static void launch_boundaries(csp_handle* h, int r0 = 0, int r1 = -1, int* step_flags = nullptr) {
-  if (r1 < 0) r1 = h->n;
-  launch_density_rows(h, r0, r1);
-  launch_channel_rows(h, r0, r1);
+static void launch_boundaries(csp_handle* h, int r0, int r1, int* step_flags = nullptr) {
   launch_surrogate(h, r0, r1);
   launch_epilogue(h, r0, r1, step_flags);
 }
 
-// One step of every realisation with an event before and after each phase (CSP_PHASE_*).
-static void launch_step_timed(csp_handle* h, cudaEvent_t* ev) {
+// One step of every realisation with an event before and after each phase (CSP_PHASE_*); the
+// step kernel runs once per phase, so that each has a time.
+static int launch_step_timed(csp_handle* h, cudaEvent_t* ev) {
+  const MarchPlan* pl = nullptr;
+  if (h->kernel != 1) {
+    const int rc = plan_for(h, 0, h->n, &pl);
+    if (rc) return rc;
+  }
   cudaEventRecord(ev[0], h->stream);
-  launch_voxels(h);
+  if (pl) CUDA_TRY(h, launch_march(h, *pl, 1, MARCH_UNITS)); else launch_direct(h, 0, h->n);
   cudaEventRecord(ev[1 + CSP_PHASE_VOXELS], h->stream);
-  launch_density_rows(h, 0, h->n);
+  if (pl) CUDA_TRY(h, launch_march(h, *pl, 1, MARCH_VOXELS)); else launch_density_rows(h, 0, h->n);
   cudaEventRecord(ev[1 + CSP_PHASE_DENSITY], h->stream);
-  launch_channel_rows(h, 0, h->n);
+  if (pl) CUDA_TRY(h, launch_march(h, *pl, 1, MARCH_CHANNELS)); else launch_channel_rows(h, 0, h->n);
   cudaEventRecord(ev[1 + CSP_PHASE_CHANNELS], h->stream);
   launch_surrogate(h, 0, h->n);
   cudaEventRecord(ev[1 + CSP_PHASE_SURROGATE], h->stream);
   launch_epilogue(h, 0, h->n, nullptr);
   cudaEventRecord(ev[1 + CSP_PHASE_EPILOGUE], h->stream);
+  return CSP_OK;
 }
 
-static cudaError_t launch_step(csp_handle* h, int r0 = 0, int r1 = -1, int* step_flags = nullptr) {
-  launch_voxels(h, r0, r1);
+static int launch_step(csp_handle* h, int r0, int r1, int* step_flags = nullptr) {
+  const int rc = launch_voxels(h, r0, r1);
+  if (rc) return rc;
   launch_boundaries(h, r0, r1, step_flags);
-  return cudaGetLastError();
+  CUDA_TRY(h, cudaGetLastError());
+  return CSP_OK;
 }
 
-static int ensure_graph(csp_handle* h) {
-  if (h->graph && h->graph_kernel == h->kernel && h->graph_surrogate == h->surrogate && h->graph_sur_tc == h->sur_tc &&
-      h->graph_plan == h->plan_epoch)
+// Steps of [r0, r1) from now on, at most `left`, of which the surrogate has nothing to do with
+// any: up to the next reaction step of one of them.  steps0: the host's step counts when the
+// call began, `done` steps ago.
+static int64_t steps_without_reaction(const csp_handle* h, int r0, int r1, int64_t done, int64_t left) {
+  int64_t m = left;
+  for (int r = r0; r < r1 && m > 0; r++) {
+    const RealDesc& D = h->real[r].desc;
+    if (D.nbuf == 0) continue;
+    const int64_t s = h->real[r].info.step + done;
+    m = std::min<int64_t>(m, D.reaction_substep - 1 - s % D.reaction_substep);
+  }
+  return m;
+}
+
+// nsteps steps of [r0, r1); step_flags (nullable, device): every realisation's stop flag after
+// every step, [nsteps][n].  The step kernel takes all of them in one launch; with the
+// surrogate on, those between two reaction steps.
+static int launch_steps(csp_handle* h, int r0, int r1, int64_t nsteps, int* step_flags) {
+  if (nsteps <= 0) return CSP_OK;
+  if (h->kernel == 1) {
+    for (int64_t i = 0; i < nsteps; i++) {
+      const int rc = launch_step(h, r0, r1, step_flags ? step_flags + i * h->n + r0 : nullptr);
+      if (rc) return rc;
+    }
     return CSP_OK;
+  }
+  const MarchPlan* pl;
+  int rc = plan_for(h, r0, r1, &pl);
+  if (rc) return rc;
+  for (int64_t i = 0; i < nsteps;) {
+    int64_t m = std::min<int64_t>(nsteps - i, MARCH_STEPS_MAX);
+    if (h->surrogate) m = steps_without_reaction(h, r0, r1, i, m);
+    if (m > 0) {
+      CUDA_TRY(h, launch_march(h, *pl, m, MARCH_STEP, step_flags ? step_flags + i * h->n : nullptr));
+      i += m;
+      continue;
+    }
+    rc = launch_step(h, r0, r1, step_flags ? step_flags + i * h->n + r0 : nullptr);
+    if (rc) return rc;
+    i++;
+  }
+  return CSP_OK;
+}
+
+// The direct kernel's steps as a graph (the kernels read the step index from device memory, so
+// one graph serves every call).
+static int ensure_graph(csp_handle* h) {
+  if (h->graph && h->graph_surrogate == h->surrogate && h->graph_sur_tc == h->sur_tc) return CSP_OK;
   if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
   cudaGraph_t g;
   CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   for (int i = 0; i < STEPS_PER_GRAPH; i++) {
-    cudaError_t e = launch_step(h);
-    if (e != cudaSuccess) {
+    const int rc = launch_step(h, 0, h->n);
+    if (rc) {
       cudaStreamEndCapture(h->stream, &g);
-      return fail(h, CSP_ECUDA, "capture: %s", cudaGetErrorString(e));
+      return rc;
     }
   }
   CUDA_TRY(h, cudaStreamEndCapture(h->stream, &g));
   cudaError_t e = cudaGraphInstantiate(&h->graph, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) { h->graph = nullptr; return fail(h, CSP_ECUDA, "graph instantiate: %s", cudaGetErrorString(e)); }
-  h->graph_kernel = h->kernel;
-  h->graph_plan = h->plan_epoch;
   h->graph_surrogate = h->surrogate;
   h->graph_sur_tc = h->sur_tc;
   return CSP_OK;
 }
 
-// The timed sample of the last advance call, scaled to the call's steps, into phase_ms.
+// The last advance call's device time, in the proportions of its timed sample, into phase_ms.
 static void add_phase_sample(csp_handle* h) {
   if (!h->phase_sampled) return;
   double ms[CSP_NUM_PHASES] = {};
@@ -1184,8 +1556,11 @@ static void add_phase_sample(csp_handle* h) {
       if (cudaEventElapsedTime(&t, ev[p], ev[p + 1]) == cudaSuccess) ms[p] += t;
     }
   }
-  const double scale = (double)h->phase_call_steps / h->phase_sampled;
-  for (int p = 0; p < CSP_NUM_PHASES; p++) h->phase_ms[p] += ms[p] * scale;
+  float call = 0.f;
+  double sum = 0.0;
+  for (int p = 0; p < CSP_NUM_PHASES; p++) sum += ms[p];
+  if (sum > 0.0 && cudaEventElapsedTime(&call, h->ev0, h->ev1) == cudaSuccess)
+    for (int p = 0; p < CSP_NUM_PHASES; p++) h->phase_ms[p] += call * ms[p] / sum;
   h->phase_steps += h->phase_call_steps;
   h->phase_sampled = 0;
 }
@@ -1214,9 +1589,12 @@ extern "C" int csp_profile_advance(csp_handle* h, int64_t nsteps, float* voxel_m
   for (auto& e : ev) CUDA_TRY(h, cudaEventCreate(&e));
   for (int64_t i = 0; i < nsteps; i++) {
     cudaEventRecord(ev[3 * i], h->stream);
-    launch_voxels(h);
+    if (int rc = launch_voxels(h, 0, h->n)) {
+      for (auto& x : ev) cudaEventDestroy(x);
+      return rc;
+    }
     cudaEventRecord(ev[3 * i + 1], h->stream);
-    launch_boundaries(h);
+    launch_boundaries(h, 0, h->n);
     cudaEventRecord(ev[3 * i + 2], h->stream);
   }
   cudaError_t le = cudaGetLastError();
@@ -1237,8 +1615,13 @@ extern "C" int csp_profile_advance(csp_handle* h, int64_t nsteps, float* voxel_m
 }
 
 static int launch_advance(csp_handle* h, int64_t nsteps) {
-  if (!h->inject_wait) {
+  const bool direct = h->kernel == 1;
+  if (direct) {
     int rc = ensure_graph(h);
+    if (rc) return rc;
+  } else {
+    const MarchPlan* pl;
+    int rc = plan_for(h, 0, h->n, &pl);
     if (rc) return rc;
   }
   CUDA_TRY(h, cudaEventRecord(h->ev0, h->stream));
@@ -1246,17 +1629,25 @@ static int launch_advance(csp_handle* h, int64_t nsteps) {
   h->phase_sampled = 0;
   if (h->phase_timing && left > 0) {
     const int ns = (int)std::min<int64_t>(left, PHASE_SAMPLE);
-    for (int i = 0; i < ns; i++) launch_step_timed(h, &h->phase_ev[i * (CSP_NUM_PHASES + 1)]);
+    for (int i = 0; i < ns; i++) {
+      const int rc = launch_step_timed(h, &h->phase_ev[i * (CSP_NUM_PHASES + 1)]);
+      if (rc) return rc;
+    }
     CUDA_TRY(h, cudaGetLastError());
     h->phase_sampled = ns;
     h->phase_call_steps = nsteps;
     left -= ns;
   }
-  while (!h->inject_wait && left >= STEPS_PER_GRAPH) {
+  while (direct && left >= STEPS_PER_GRAPH) {
     CUDA_TRY(h, cudaGraphLaunch(h->graph, h->stream));
     left -= STEPS_PER_GRAPH;
   }
-  while (left-- > 0) CUDA_TRY(h, launch_step(h));
+  // (the surrogate's reaction steps are counted from the host's step counts)
+  const int64_t taken = nsteps - left;
+  for (int r = 0; r < h->n && taken; r++) h->real[r].info.step += taken;
+  const int rc = launch_steps(h, 0, h->n, left, nullptr);
+  for (int r = 0; r < h->n && taken; r++) h->real[r].info.step -= taken;
+  if (rc) return rc;
   CUDA_TRY(h, cudaEventRecord(h->ev1, h->stream));
   return CSP_OK;
 }
@@ -1573,8 +1964,8 @@ static int run_states(csp_handle* h, const T* const* uin, int64_t nsteps, T* con
       k_state_in<T><<<blocks_of(m.nvox * m.ns), 256, 0, cs>>>(in_slot + off[r], m);
     }
     if (e == cudaSuccess) e = cudaEventRecord(in_free[k], cs);
-    for (int64_t st = 0; st < nsteps && e == cudaSuccess; st++)
-      e = launch_step(h, r0, r1, step_flags ? h->d_stepflags + st * h->n + r0 : nullptr);
+    if (e == cudaSuccess && launch_steps(h, r0, r1, nsteps, step_flags ? h->d_stepflags : nullptr) != CSP_OK)
+      e = cudaErrorLaunchFailure;
     if (e == cudaSuccess && g >= 2) e = cudaStreamWaitEvent(cs, out_free[k], 0);
     for (int r = r0; r < r1 && e == cudaSuccess; r++) {
       const StateMap m = make_state_map(h, r);
@@ -1724,7 +2115,8 @@ struct LinescanMap {
   double base[ND];           // the species' field base per domain
   int fixq;                  // the species is stored in fixed point: value = base + q * qunit
   double qunit[ND];
-  int nd[3];                 // device extents (n0, n1, n2)
+  int nd[3];                 // device extents (n0, n1, row stride)
+  int nzv;                   // voxels per row
   int P;
   int phys_of_dev[3];        // physical axis of each device axis
   int axis;                  // scanned physical axis
@@ -1744,6 +2136,7 @@ __global__ void k_linescan_bins(LinescanMap m, double* __restrict__ bins) {
     const int c0 = (int)(v / plane);
     const long long rem = v - c0 * plane;
     const int c1 = (int)(rem / m.nd[2]), c2 = (int)(rem - (long long)c1 * m.nd[2]);
+    if (c2 >= m.nzv) continue;
     const long long dv = (long long)c0 * m.P + rem;
     const int dom = m.dom[dv] & DOMAIN_BITS;
     if (m.num_domains > 0 && dom >= m.num_domains) continue;
@@ -1801,6 +2194,7 @@ extern "C" int csp_linescan(csp_handle* h, int32_t r, int32_t species, int32_t a
   }
   m.fixq = (D.fixq >> species) & 1u;
   m.nd[0] = D.nx; m.nd[1] = D.ny; m.nd[2] = D.nz;
+  m.nzv = D.nzv;
   m.P = D.P;
   for (int i = 0; i < 3; i++) m.phys_of_dev[i] = hr.perm[i];
   m.axis = axis;
@@ -1901,9 +2295,7 @@ extern "C" int csp_get_phase_times(const csp_handle* h, double* ms, int64_t* ste
 
 extern "C" int csp_test_wait_timeout(csp_handle* h, int32_t on) {
   if (!h) return CSP_EINVAL;
-  if (on && (h->kernel != 0 || !h->plan.ok || !h->plan.launch_inject))
-    return fail(h, CSP_EINVAL, "the staged voxel kernel with the test hook is not in use");
-  // the hook's variant does not classify voxels for the surrogate
+  if (on && h->kernel != 0) return fail(h, CSP_EINVAL, "the step kernel with the test hook is not in use");
   if (on && h->surrogate) return fail(h, CSP_EINVAL, "the test hook does not run with the surrogate on");
   h->inject_wait = on ? 1 : 0;
   return CSP_OK;
@@ -1912,127 +2304,110 @@ extern "C" int csp_test_wait_timeout(csp_handle* h, int32_t on) {
 extern "C" int csp_set_kernel(csp_handle* h, int32_t which) {
   if (!h || which < 0 || which > 1) return CSP_EINVAL;
   CSP_NOT_PENDING(h);
-  if (which == 0 && !h->plan.ok) return fail(h, CSP_ENOTSUP, "staged kernel unavailable for this batch");
   h->kernel = which;
   return CSP_OK;
 }
 
-// ---- autotuner of the staged kernel's tile shape ----
-// Candidates: threads per CTA (positions per chunk = 4 x threads) and x planes per work
-// unit.  Each candidate's voxel kernel runs `repeats` times at the current step: the
-// kernel reads the current buffers and writes the next ones, so repeating it is free of
-// side effects (the real step writes the same values), and every tiling gives bitwise
-// equal fields.  The fastest plan replaces the current one.
+// ---- autotuner ----
+// Candidates: the number of teams of the step kernel (realisations in flight) and the x
+// segments per realisation, around the estimate's choice, and the direct kernel.  Each runs TUNE_STEPS steps
+// `repeats` times at the current step without going on (MARCH_REPEAT: the buffers read stay
+// current, the next ones are written again; the channels' gating is left out), so that the
+// fields' place in L2 or HBM counts as in a run; no side effect stays, and every candidate
+// gives bitwise equal fields.
+constexpr int TUNE_STEPS = 4;
 extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep) {
   if (!h) return CSP_EINVAL;
   CSP_NOT_PENDING(h);
   if (repeats < 1) repeats = 3;
-  std::vector<RealDesc> descs(h->n);
-  for (int r = 0; r < h->n; r++) descs[r] = h->real[r].desc;
-  int cand[CSP_TUNE_MAX][2] = {{256, 0}, {256, 16}, {256, 32}, {256, 1 << 20}, {128, 0}, {128, 32}};
-  int ncand = 6;
-  // two more segment lengths for 256 threads from a cost model: rounds of work units over
-  // the resident CTAs times the planes a unit stages (its segment and two halo planes)
-  {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long ctas = 2ll * sms, L = 1024;
-    double best[2] = {1e300, 1e300};
-    int bseg[2] = {0, 0};
-    for (int seg = 8; seg <= 64; seg++) {
-      if (seg == 16 || seg == 32) continue;
-      long long units = 0;
-      for (const RealDesc& D : descs) units += (long long)((D.nx + seg - 1) / seg) * ((D.plane + L - 1) / L);
-      const double cost = (double)((units + ctas - 1) / ctas) * (seg + 2);
-      if (cost < best[0]) {
-        best[1] = best[0]; bseg[1] = bseg[0];
-        best[0] = cost; bseg[0] = seg;
-      } else if (cost < best[1]) {
-        best[1] = cost; bseg[1] = seg;
-      }
-    }
-    for (int k = 0; k < 2 && ncand < CSP_TUNE_MAX; k++)
-      if (bseg[k]) { cand[ncand][0] = 256; cand[ncand][1] = bseg[k]; ncand++; }
+  for (MarchPlan& p : h->plans) free_plan(p);
+  h->plans.clear();
+  const MarchPlan* def;
+  int rc = plan_for(h, 0, h->n, &def);
+  if (rc) return rc;
+  const int t0 = def->teams, seg0 = def->nseg, nx0 = h->real[0].desc.nx;
+  int cand[CSP_TUNE_MAX][2];
+  int ncand = 0;
+  auto add = [&](int t, int s) {
+    t = std::max(1, std::min(t, h->n));
+    s = std::max(0, s);
+    for (int i = 0; i < ncand; i++)
+      if (cand[i][0] == t && (cand[i][1] ? cand[i][1] : seg0) == (s ? s : seg0)) return;
+    if (ncand < CSP_TUNE_MAX - 1) { cand[ncand][0] = t; cand[ncand][1] = s; ncand++; }
+  };
+  add(t0, 0);
+  if (h->n == 1) {
+    for (int s : {seg0 + 1, seg0 - 1, seg0 * 5 / 4, seg0 * 3 / 4, seg0 * 3 / 2}) add(1, s);
+  } else {
+    for (int t : {t0 - 1, t0 + 1, t0 * 5 / 4, t0 * 3 / 4}) add(t, 0);
+    add(t0, seg0 * 5 / 4 + 1);
+    add(t0, seg0 * 3 / 4);
   }
   cudaEvent_t e0, e1;
   CUDA_TRY(h, cudaEventCreate(&e0));
   CUDA_TRY(h, cudaEventCreate(&e1));
-  int best = -1;
-  float best_ms = 0.f;
-  StagedPlan best_plan;
   csp_tune_report local;
   memset(&local, 0, sizeof local);
-  for (int i = 0; i < ncand && i < CSP_TUNE_MAX - 1; i++) {
-    StagedPlan pl = staged_plan(descs, cand[i][0], cand[i][1]);
-    local.threads[local.n] = cand[i][0];
-    local.segment[local.n] = pl.g.seg;
-    local.ms[local.n] = -1.f;
-    if (staged_prepare(pl) != cudaSuccess) {
-      staged_release(pl);
-      local.n++;
-      continue;
-    }
-    staged_launch(pl, h->d_desc, h->d_ctl, h->d_err, h->stream);      // warm-up
+  int best = -1;
+  MarchPlan best_plan;
+  bool direct = false;
+  cudaError_t e = cudaSuccess;
+  auto timed = [&](auto launch, float* ms) {
     cudaEventRecord(e0, h->stream);
-    for (int k = 0; k < repeats; k++) staged_launch(pl, h->d_desc, h->d_ctl, h->d_err, h->stream);
+    launch();                                                   // warm-up
     cudaEventRecord(e1, h->stream);
-    cudaError_t e = cudaEventSynchronize(e1);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      staged_release(pl);
-      if (best >= 0) staged_release(best_plan);
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      return fail(h, CSP_ECUDA, "autotune: %s", cudaGetErrorString(e));
-    }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    ms /= repeats;
-    local.ms[local.n] = ms;
-    if (best < 0 || ms < best_ms) {
-      if (best >= 0) staged_release(best_plan);
-      best = local.n;
-      best_ms = ms;
+    cudaError_t w = cudaEventSynchronize(e1);
+    if (w != cudaSuccess) return w;
+    cudaEventElapsedTime(ms, e0, e1);
+    *ms /= TUNE_STEPS;
+    if (best >= 0 && *ms > 2.f * local.ms[best]) return cudaGetLastError();    // far behind already
+    cudaEventRecord(e0, h->stream);
+    for (int k = 0; k < repeats; k++) launch();
+    cudaEventRecord(e1, h->stream);
+    cudaError_t x = cudaEventSynchronize(e1);
+    if (x == cudaSuccess) x = cudaGetLastError();
+    cudaEventElapsedTime(ms, e0, e1);
+    *ms /= (float)repeats * TUNE_STEPS;
+    return x;
+  };
+  for (int i = 0; i < ncand && e == cudaSuccess && rc == CSP_OK; i++) {
+    MarchPlan pl;
+    rc = make_plan(h, 0, h->n, cand[i][0], cand[i][1], pl);
+    if (rc) { free_plan(pl); break; }
+    const int k = local.n++;
+    local.threads[k] = MARCH_T;
+    local.segment[k] = (nx0 + pl.nseg - 1) / pl.nseg;
+    e = timed([&]() { launch_march(h, pl, TUNE_STEPS, MARCH_UNITS | MARCH_VOXELS | MARCH_REPEAT); }, &local.ms[k]);
+    if (e == cudaSuccess && (best < 0 || local.ms[k] < local.ms[best])) {
+      free_plan(best_plan);
+      best = k;
       best_plan = pl;
     } else {
-      staged_release(pl);
+      free_plan(pl);
     }
-    local.n++;
   }
-  // the direct kernel (recomputes the same step, like the staged candidates)
-  bool direct = false;
-  {
-    const int i = local.n;
-    local.threads[i] = 256;
-    local.segment[i] = -1;
-    dim3 grid((unsigned)((h->max_vox + 255) / 256), (unsigned)h->n);
-    k_voxels_direct<<<grid, 256, 0, h->stream>>>(h->d_desc, h->d_ctl, h->d_err);
-    cudaEventRecord(e0, h->stream);
-    for (int k = 0; k < repeats; k++) k_voxels_direct<<<grid, 256, 0, h->stream>>>(h->d_desc, h->d_ctl, h->d_err);
-    cudaEventRecord(e1, h->stream);
-    cudaError_t e = cudaEventSynchronize(e1);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      if (best >= 0) staged_release(best_plan);
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      return fail(h, CSP_ECUDA, "autotune: %s", cudaGetErrorString(e));
-    }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    local.ms[i] = ms / repeats;
-    if (best < 0 || local.ms[i] < best_ms) direct = true;
-    local.n++;
+  if (e == cudaSuccess && rc == CSP_OK) {
+    // the direct kernel with its density rows, which only write the next buffers too
+    const int k = local.n++;
+    local.threads[k] = 256;
+    local.segment[k] = -1;
+    e = timed([&]() {
+      for (int s = 0; s < TUNE_STEPS; s++) {
+        launch_direct(h, 0, h->n);
+        launch_density_rows(h, 0, h->n);
+      }
+    }, &local.ms[k]);
+    direct = e == cudaSuccess && local.ms[k] < local.ms[best];
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  if (best >= 0) {
-    staged_release(h->plan);
-    h->plan = best_plan;
+  if (e != cudaSuccess || rc != CSP_OK) {
+    free_plan(best_plan);
+    return rc != CSP_OK ? rc : fail(h, CSP_ECUDA, "autotune: %s", cudaGetErrorString(e));
   }
-  h->plan_epoch++;
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  free_plan(h->plans[0]);
+  h->plans[0] = best_plan;
   h->kernel = direct ? 1 : 0;
   local.chosen = direct ? local.n - 1 : best;
   if (rep) *rep = local;
@@ -2160,7 +2535,10 @@ extern "C" int csp_set_surrogate(csp_handle* h, const float* params, double tol)
     }
     descs[r] = D;
   }
+  std::vector<VoxDesc> vdescs(h->n);
+  for (int r = 0; r < h->n; r++) vdescs[r] = make_vox_desc(h->real[r]);
   CUDA_TRY(h, cudaMemcpyAsync(h->d_desc, descs.data(), h->n * sizeof(RealDesc), cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(h, cudaMemcpyAsync(h->d_vdesc, vdescs.data(), h->n * sizeof(VoxDesc), cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return CSP_OK;
 }
@@ -2464,9 +2842,9 @@ extern "C" void csp_destroy(csp_handle* h) {
   if (!h) return;
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->graph) cudaGraphExecDestroy(h->graph);
-  staged_release(h->plan);
-  cudaFree(h->d_fields); cudaFree(h->d_dom); cudaFree(h->d_cls); cudaFree(h->d_desc); cudaFree(h->d_ctl);
-  cudaFree(h->d_rec); cudaFree(h->d_drows);
+  for (MarchPlan& p : h->plans) free_plan(p);
+  cudaFree(h->d_fields); cudaFree(h->d_dom); cudaFree(h->d_gcode); cudaFree(h->d_desc); cudaFree(h->d_vdesc); cudaFree(h->d_ctl);
+  cudaFree(h->d_rec); cudaFree(h->d_drows); cudaFree(h->d_mix); cudaFree(h->d_mixc); cudaFree(h->d_items);
   cudaFree(h->d_rows); cudaFree(h->d_entries); cudaFree(h->d_pairs); cudaFree(h->d_params);
   cudaFree(h->d_states); cudaFree(h->d_err); cudaFree(h->d_red); cudaFree(h->d_red_out);
   cudaFree(h->d_stage);

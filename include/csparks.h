@@ -273,9 +273,9 @@ int csp_get_stream(const csp_handle* h, void** stream);
 /* Device time in ms of the last csp_advance call (CUDA events on the handle stream). */
 int csp_last_advance_ms(const csp_handle* h, float* ms);
 
-/* Advance like csp_advance, but launch the two kernels of every step one by one with CUDA
- * events around each launch (no graph); voxel_ms / boundary_ms receive the summed device
- * times of the voxel kernel and of the boundary / gating kernel. */
+/* Advance like csp_advance, but with a launch per step and CUDA events around its parts:
+ * voxel_ms receives the summed device times of the voxels' updates with their boundary fluxes
+ * and gating, boundary_ms those of the surrogate's corrections and the step counter. */
 int csp_profile_advance(csp_handle* h, int64_t nsteps, float* voxel_ms, float* boundary_ms);
 
 /* Per-phase device times of the step (the counterpart of the reference's -v timing buckets
@@ -285,29 +285,29 @@ int csp_profile_advance(csp_handle* h, int64_t nsteps, float* voxel_ms, float* b
  * reactions and fixed values (species.c:1501-1702), CSP_PHASE_DENSITY = density-boundary
  * (SERCA) fluxes, CSP_PHASE_CHANNELS = RyR/pRyR gating with the channel fluxes
  * (species.c:1704-1957), CSP_PHASE_SURROGATE = the learned reaction increments,
- * CSP_PHASE_EPILOGUE = step counter and abort rule.  While enabled, the first 16 steps of
- * every csp_advance / csp_advance_async call run as direct launches with CUDA events
- * between the kernels; their per-phase time, scaled to the call's steps, is accumulated
- * (an estimate: the other steps replay the captured graph untimed).  ms[CSP_NUM_PHASES]
- * receives the accumulated milliseconds, steps the steps they stand for. */
+ * CSP_PHASE_EPILOGUE = step counter and abort rule.  A density pair along a domain sheet is
+ * evaluated with the sheet's voxels, in CSP_PHASE_VOXELS.  While enabled, the first 16 steps
+ * of every csp_advance / csp_advance_async call run as one launch per phase with CUDA events
+ * between them; the call's device time is divided in the proportions of this sample (an
+ * estimate: the other steps run whole, many to a launch) and accumulated.
+ * ms[CSP_NUM_PHASES] receives the accumulated milliseconds, steps the steps they stand for. */
 enum { CSP_PHASE_VOXELS = 0, CSP_PHASE_DENSITY, CSP_PHASE_CHANNELS, CSP_PHASE_SURROGATE, CSP_PHASE_EPILOGUE,
        CSP_NUM_PHASES };
 int csp_set_phase_timing(csp_handle* h, int32_t on);
 int csp_get_phase_times(const csp_handle* h, double* ms, int64_t* steps);
 
-/* Test hook for the failure path of the staged voxel kernel's bounded waits.  While armed
- * (on != 0), every launch of the staged kernel makes one thread of its first CTA wait on an
- * mbarrier that nothing completes, with a 1 ms limit; that CTA then leaves its x loop as
- * one (the decision is taken at the end-of-plane barrier), waits for its own bulk copies
- * in flight, sets the timeout bit of the device error word and returns, and csp_advance
- * returns CSP_EDEVICE with csp_status naming the timeout.  The handle's fields are
+/* Test hook for the failure path of the step kernel's bounded waits.  While armed (on != 0),
+ * every launch of the step kernel makes one thread of its first CTA wait for an arrival that
+ * nothing makes, with a 1 ms limit; the thread then sets the timeout bit of the device error
+ * word and the CTA leaves, the CTAs that wait for it at a barrier see the bit and leave too,
+ * and csp_advance returns CSP_EDEVICE with csp_status naming the timeout.  The handle's fields are
  * undefined afterwards and the error stays set; the device and other handles stay usable.
  * No counterpart in the reference: it has no device and aborts on any error
  * (fvm_mpi/src/utils.h:21-27). */
 int csp_test_wait_timeout(csp_handle* h, int32_t on);
 
-/* Select the voxel kernel: 0 = staged (TMA bulk copies into shared memory, default),
- * 1 = direct (one thread per voxel, global loads).  Both give bitwise equal results. */
+/* Select the kernels: 0 = the step kernel (whole steps, many to a launch, default), 1 = direct
+ * (one thread per voxel, then the boundary rows).  Both give bitwise equal results. */
 int csp_set_kernel(csp_handle* h, int32_t which);
 
 /* Linescan of species `species` of realisation r along physical axis `axis` (0 x, 1 y,
@@ -395,17 +395,15 @@ int csp_surrogate_counts(const csp_handle* h, int64_t* voxels, int64_t* network,
 int csp_set_surrogate_tensor_cores(csp_handle* h, int32_t kind);
 
 /* ---- autotuner ----
- * Times candidate tile shapes of the staged voxel kernel (threads per CTA, x planes per
- * work unit) and the direct kernel (segment = -1: one thread per voxel, every plane at
- * once, which wins on batches too small to give the staged kernel's work units to every
- * CTA slot) at the current step and keeps the fastest; fields are the same for every
- * candidate.  No counterpart in the reference (its OpenMP loops have no tile parameters). */
+ * Times candidates of the step kernel (realisations in flight at once, x segments per
+ * realisation) and the direct kernel (segment = -1) at the current step and keeps the
+ * fastest; fields are the same for every candidate.  No counterpart in the reference (its OpenMP loops have no tile parameters). */
 #define CSP_TUNE_MAX 10
 typedef struct csp_tune_report {
   int32_t n;                       /* candidates tried */
   int32_t threads[CSP_TUNE_MAX];
-  int32_t segment[CSP_TUNE_MAX];   /* x planes per work unit */
-  float ms[CSP_TUNE_MAX];          /* voxel-kernel time per launch (-1: did not fit) */
+  int32_t segment[CSP_TUNE_MAX];   /* x planes per work unit (mean, first realisation) */
+  float ms[CSP_TUNE_MAX];          /* time per step */
   int32_t chosen;                  /* index of the plan in use */
 } csp_tune_report;
 int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* report);
