@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <array>
 #include <map>
+#include <mutex>
 #include <unordered_map>
 #include <cmath>
 #include <cstdarg>
@@ -2567,35 +2568,77 @@ extern "C" int csp_surrogate_counts(const csp_handle* hc, int64_t* voxels, int64
 
 static cudaError_t mlp_grad_launch(const float* dp, const float* dx, const float* dt, long long n, float* dg,
                                    float* dl, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MLP_GRAD_SMEM);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  const unsigned blocks = (unsigned)((n + MLP_TB - 1) / MLP_TB);
-  k_mlp_grad<<<blocks, MLP_TB, MLP_GRAD_SMEM, st>>>(dp, dx, dt, n, 1.f / (float)(n * MLP_OUT), dg, dl);
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpGradSmem));
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  // two CTAs fit an SM; each walks its share of the tiles, two at least: with one (7 us less
+  // below 20,000 samples) twice as many rounded partial sums meet in each weight
+  const unsigned blocks = (unsigned)std::min<long long>((n + 2 * MLP_TB - 1) / (2 * MLP_TB), 2ll * sms);
+  k_mlp_grad<<<blocks, MLP_GT, sizeof(MlpGradSmem), st>>>(dp, dx, dt, n, 1.f / (float)(n * MLP_OUT), dg, dl);
   return cudaGetLastError();
+}
+
+// csp_mlp_gradient's device memory: a pool per device that keeps up to GRAD_POOL_KEEP bytes
+// from call to call (a cudaMalloc and cudaFree of them cost 0.5 ms, the kernel 0.2) and gives
+// the rest back when a call ends; csp_destroy gives back what is not in use.
+constexpr unsigned long long GRAD_POOL_KEEP = 64ull << 20;
+constexpr int GRAD_POOL_DEVICES = 64;
+static std::mutex g_grad_pool_mu;
+static cudaMemPool_t g_grad_pool[GRAD_POOL_DEVICES] = {};
+
+static cudaError_t grad_pool(cudaMemPool_t* pool) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= GRAD_POOL_DEVICES) return cudaDeviceGetDefaultMemPool(pool, dev);
+  std::lock_guard<std::mutex> lock(g_grad_pool_mu);
+  if (!g_grad_pool[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t made = nullptr;
+    e = cudaMemPoolCreate(&made, &props);
+    unsigned long long keep = GRAD_POOL_KEEP;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) return e;
+    g_grad_pool[dev] = made;
+  }
+  *pool = g_grad_pool[dev];
+  return cudaSuccess;
+}
+
+static void grad_pool_trim() {
+  std::lock_guard<std::mutex> lock(g_grad_pool_mu);
+  for (cudaMemPool_t p : g_grad_pool)
+    if (p) cudaMemPoolTrimTo(p, 0);
 }
 
 extern "C" int csp_mlp_gradient(const float* params, const float* x, const float* t, int64_t n, float* grad,
                                 float* loss) {
   if (!params || !x || !t || !grad || !loss || n <= 0) return fail(nullptr, CSP_EINVAL, "bad argument");
-  float *dp = nullptr, *dx = nullptr, *dt = nullptr, *dg = nullptr;
-  const size_t nb = (MLP_NPARAM + 1) * sizeof(float);
-  cudaError_t e = cudaMalloc(&dp, nb);
-  if (e == cudaSuccess) e = cudaMalloc(&dx, n * MLP_IN * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dt, n * MLP_OUT * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dg, nb);
-  if (e == cudaSuccess) e = cudaMemcpy(dp, params, MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dx, x, n * MLP_IN * sizeof(float), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dt, t, n * MLP_OUT * sizeof(float), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(dg, 0, nb);
+  // one allocation: parameters, gradient and loss, inputs, targets
+  const size_t np = (MLP_NPARAM + 1 + 63) / 64 * 64;
+  const size_t nx = ((size_t)n * MLP_IN + 63) / 64 * 64;
+  float* dp = nullptr;
+  cudaMemPool_t pool = nullptr;
+  cudaError_t e = grad_pool(&pool);
+  if (e == cudaSuccess)
+    e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dp), (2 * np + nx + (size_t)n * MLP_OUT) * sizeof(float), pool, 0);
+  float *dg = dp + np, *dx = dg + np, *dt = dx + nx;
+  std::vector<float> out(MLP_NPARAM + 1);
+  if (e == cudaSuccess) e = cudaMemsetAsync(dg, 0, np * sizeof(float), 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dp, params, MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, n * MLP_IN * sizeof(float), cudaMemcpyHostToDevice, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, n * MLP_OUT * sizeof(float), cudaMemcpyHostToDevice, 0);
   if (e == cudaSuccess) e = mlp_grad_launch(dp, dx, dt, n, dg, dg + MLP_NPARAM, 0);
-  if (e == cudaSuccess) e = cudaMemcpy(grad, dg, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(loss, dg + MLP_NPARAM, sizeof(float), cudaMemcpyDeviceToHost);
-  cudaFree(dp); cudaFree(dx); cudaFree(dt); cudaFree(dg);
+  if (e == cudaSuccess) e = cudaMemcpy(out.data(), dg, out.size() * sizeof(float), cudaMemcpyDeviceToHost);
+  if (dp) cudaFreeAsync(dp, 0);
   if (e != cudaSuccess) return fail(nullptr, CSP_ECUDA, "mlp gradient: %s", cudaGetErrorString(e));
+  std::memcpy(grad, out.data(), MLP_NPARAM * sizeof(float));
+  *loss = out[MLP_NPARAM];
   return CSP_OK;
 }
 
@@ -2840,6 +2883,7 @@ extern "C" int csp_mlp_train(csp_handle* h, int32_t r, const csp_mlp_config* cfg
 
 extern "C" void csp_destroy(csp_handle* h) {
   if (!h) return;
+  grad_pool_trim();
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->graph) cudaGraphExecDestroy(h->graph);
   for (MarchPlan& p : h->plans) free_plan(p);
