@@ -289,10 +289,9 @@ class Simulation:
 
     def snapshot_wait(self):
         """Wait for snapshot_async; returns a copy of the fields ([species][x][y][z], FP64)."""
-        p = C.POINTER(C.c_double)()
-        self._check(self.lib.csp_snapshot_wait(self.h, C.byref(p)))
-        n = int(np.prod(self._snap_shape))
-        return np.ctypeslib.as_array(p, shape=(n,)).reshape(self._snap_shape).copy()
+        u = np.empty(getattr(self, "_snap_shape", 1))
+        self._check(self.lib.csp_snapshot_read(self.h, u.ctypes.data_as(C.POINTER(C.c_double))))
+        return u
 
     def profile(self, nsteps):
         """Advance nsteps with per-kernel CUDA events: (voxel_ms, boundary_ms) summed."""

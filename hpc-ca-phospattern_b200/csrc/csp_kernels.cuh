@@ -574,72 +574,141 @@ __global__ void k_group_codes(const unsigned char* __restrict__ dom, unsigned ch
   code[i] = c;
 }
 
-// Output reductions: partial min / max / sum over a block for one species of one
-// realisation, then a fixed-order final pass (deterministic FP64 sums).
-__global__ void __launch_bounds__(256) k_reduce_partial(const RealDesc* __restrict__ descs,
-                                                         const RealCtl* __restrict__ ctl, int r, int s,
-                                                         double* __restrict__ part /*[nblk][3][ND]*/) {
+// Output reductions: min / max / sum per domain and species of one realisation, blockIdx.y =
+// species, then a final pass in a fixed order (deterministic FP64 sums).
+// Bound by reading the fields once (5 bytes per voxel and species).  A thread takes four
+// voxels at a time, in one domain nearly always (its byte tells the others' lane), reduces
+// the stored deviations and adds the domain's base at the end: min and max in FP32 (or
+// integers), whose order is the values', and the sum as sum(deviations) + count * base.
+// 4 M voxels x 5 species through csp_reduce_outputs: 78 us (a launch, a one-warp final pass, a
+// copy and a wait per species, with FP64 selects over all domains per voxel: 500 us).
+constexpr int RED_BLOCKS = 296, RED_T = 256;
+struct RedPart {
+  double sum;
+  float mn, mx;                     // fixed point: the integers' bits
+  unsigned long long n;             // voxels
+};
+
+__device__ __forceinline__ void red_join(RedPart& a, const RedPart& b, bool fixq) {
+  if (fixq) {
+    a.mn = __int_as_float(min(__float_as_int(a.mn), __float_as_int(b.mn)));
+    a.mx = __int_as_float(max(__float_as_int(a.mx), __float_as_int(b.mx)));
+  } else {
+    a.mn = fminf(a.mn, b.mn);       // (NaN: the other one)
+    a.mx = fmaxf(a.mx, b.mx);
+  }
+  a.sum += b.sum;
+  a.n += b.n;
+}
+
+__device__ __forceinline__ RedPart red_shuffle(const RedPart& a, int o) {
+  RedPart b;
+  b.sum = __shfl_xor_sync(0xffffffffu, a.sum, o);
+  b.mn = __shfl_xor_sync(0xffffffffu, a.mn, o);
+  b.mx = __shfl_xor_sync(0xffffffffu, a.mx, o);
+  b.n = __shfl_xor_sync(0xffffffffu, a.n, o);
+  return b;
+}
+
+__device__ __forceinline__ RedPart red_empty(bool fixq) {
+  RedPart a;
+  a.sum = 0.0;
+  a.mn = fixq ? __int_as_float(0x7fffffff) : __int_as_float(0x7f800000);
+  a.mx = fixq ? __int_as_float((int)0x80000000) : __int_as_float((int)0xff800000);
+  a.n = 0;
+  return a;
+}
+
+__global__ void __launch_bounds__(RED_T) k_reduce_partial(const RealDesc* __restrict__ descs,
+                                                          const RealCtl* __restrict__ ctl, int r,
+                                                          RedPart* __restrict__ part /*[species][ND][gridDim.x]*/) {
   const RealDesc& D = descs[r];
+  const int s = blockIdx.y;
   const unsigned cur = ctl[r].cur_mask[ctl[r].step & 1];
   const float* __restrict__ u = D.u[(cur >> s) & 1u][s];
-  double mn[ND], mx[ND], sm[ND];
+  const bool fixq = D.fixq >> s & 1u;
+  RedPart acc[ND];
 #pragma unroll
-  for (int d = 0; d < ND; d++) { mn[d] = FLT_MAX; mx[d] = FLT_MIN; sm[d] = 0.0; }
-  const long long nvox = (long long)D.nx * D.plane;
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvox; v += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(v / D.plane), p = (int)(v - (long long)x * D.plane);
-    if (p % D.nz >= D.nzv) continue;
-    const long long idx = (long long)x * D.P + p;
-    const int d = D.dom[idx] & DOMAIN_BITS;
-    const double val = ((D.fixq >> s & 1u) ? (double)q_bits(u[idx]) * D.qunit[d][s] : (double)u[idx]) + D.base[d][s];
+  for (int d = 0; d < ND; d++) acc[d] = red_empty(fixq);
+  auto add = [&](const RedPart& a, unsigned d) {
 #pragma unroll
-    for (int dd = 0; dd < ND; dd++) {
-      if (dd == d) {
-        mn[dd] = val < mn[dd] ? val : mn[dd];
-        mx[dd] = val > mx[dd] ? val : mx[dd];
-        sm[dd] += val;
-      }
+    for (int dd = 0; dd < ND; dd++)
+      if (dd == (int)d) red_join(acc[dd], a, fixq);
+  };
+  auto value = [&](float f) { return fixq ? (double)__float_as_int(f) : (double)f; };
+  const unsigned rowg = (unsigned)D.nz / 4, planeg = (unsigned)D.plane / 4;      // groups of four per row, plane
+  const long long groups = (long long)D.nx * planeg;
+  for (long long g = (long long)blockIdx.x * RED_T + threadIdx.x; g < groups; g += (long long)gridDim.x * RED_T) {
+    const long long x = groups < (1ll << 32) ? (unsigned)g / planeg : g / planeg;
+    const unsigned p = (unsigned)(g - x * planeg);
+    const int z = (int)(p % rowg) * 4;
+    const long long idx = x * D.P + (long long)p * 4;
+    const unsigned dom = *reinterpret_cast<const unsigned*>(D.dom + idx) & DOMAIN_BITS * 0x01010101u;
+    const float4 f = *reinterpret_cast<const float4*>(u + idx);
+    const float fv[4] = {f.x, f.y, f.z, f.w};
+    if (z + 4 <= D.nzv && dom == (dom & 0xffu) * 0x01010101u) {
+      RedPart a;
+      a.mn = a.mx = f.x;
+      a.sum = value(f.x);
+      a.n = 4;
+#pragma unroll
+      for (int j = 1; j < 4; j++) red_join(a, RedPart{value(fv[j]), fv[j], fv[j], 0u}, fixq);
+      add(a, dom & 0xffu);
+    } else {
+      for (int j = 0; j < 4 && z + j < D.nzv; j++)
+        add(RedPart{value(fv[j]), fv[j], fv[j], 1u}, dom >> (8 * j) & 0xffu);
     }
   }
-  __shared__ double red[3][ND][256];
+  __shared__ RedPart red[RED_T / 32][ND];
 #pragma unroll
-  for (int d = 0; d < ND; d++) { red[0][d][threadIdx.x] = mn[d]; red[1][d][threadIdx.x] = mx[d]; red[2][d][threadIdx.x] = sm[d]; }
+  for (int d = 0; d < ND; d++) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) red_join(acc[d], red_shuffle(acc[d], o), fixq);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][d] = acc[d];
+  }
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-#pragma unroll
-      for (int d = 0; d < ND; d++) {
-        double a = red[0][d][threadIdx.x + w];
-        if (a < red[0][d][threadIdx.x]) red[0][d][threadIdx.x] = a;
-        a = red[1][d][threadIdx.x + w];
-        if (a > red[1][d][threadIdx.x]) red[1][d][threadIdx.x] = a;
-        red[2][d][threadIdx.x] += red[2][d][threadIdx.x + w];
-      }
-    }
-    __syncthreads();
-  }
   if (threadIdx.x < ND) {
-    const int d = threadIdx.x;
-    part[(blockIdx.x * 3 + 0) * ND + d] = red[0][d][0];
-    part[(blockIdx.x * 3 + 1) * ND + d] = red[1][d][0];
-    part[(blockIdx.x * 3 + 2) * ND + d] = red[2][d][0];
+    RedPart a = red[0][threadIdx.x];
+    for (int w = 1; w < RED_T / 32; w++) red_join(a, red[w][threadIdx.x], fixq);
+    part[((size_t)s * ND + threadIdx.x) * gridDim.x + blockIdx.x] = a;
   }
 }
 
-__global__ void k_reduce_final(const double* __restrict__ part, int nblk, double dV,
-                               double* __restrict__ out /*[3][ND]*/) {
-  const int d = threadIdx.x;
-  if (d >= ND) return;
-  double mn = FLT_MAX, mx = FLT_MIN, sm = 0.0;
-  for (int b = 0; b < nblk; b++) {
-    const double a = part[(b * 3 + 0) * ND + d], c = part[(b * 3 + 1) * ND + d];
-    mn = a < mn ? a : mn;
-    mx = c > mx ? c : mx;
-    sm += part[(b * 3 + 2) * ND + d];
+// One warp per domain and block per species: the blocks' parts, then the domain's base, into
+// out[species][min, max, total][ND]; blocks from ns on copy the realisation's channel states.
+__global__ void __launch_bounds__(32 * ND) k_reduce_final(const RealDesc* __restrict__ descs,
+                                                          const RealCtl* __restrict__ ctl, int r,
+                                                          const RedPart* __restrict__ part, int nblk, double dV,
+                                                          double* __restrict__ out,
+                                                          const unsigned char* __restrict__ states, int nch_all,
+                                                          int ch0, int nch, unsigned char* __restrict__ open) {
+  const RealDesc& D = descs[r];
+  if ((int)blockIdx.x >= D.ns) {
+    const unsigned char* now = states + (ctl[r].step & 1) * (long long)nch_all + ch0;
+    for (int i = ((int)blockIdx.x - D.ns) * (int)blockDim.x + (int)threadIdx.x; i < nch;
+         i += ((int)gridDim.x - D.ns) * (int)blockDim.x)
+      open[i] = now[i];
+    return;
   }
-  out[0 * ND + d] = mn;
-  out[1 * ND + d] = mx;
-  out[2 * ND + d] = sm * dV;
+  const int s = blockIdx.x, d = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool fixq = D.fixq >> s & 1u;
+  RedPart a = red_empty(fixq);
+  for (int b = lane; b < nblk; b += 32) red_join(a, part[((size_t)s * ND + d) * nblk + b], fixq);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) red_join(a, red_shuffle(a, o), fixq);
+  if (lane) return;
+  double mn = FLT_MAX, mx = FLT_MIN, sum = 0.0;
+  if (a.n) {
+    const double unit = fixq ? (double)D.qunit[d][s] : 1.0, base = D.base[d][s];
+    const double lo = (fixq ? (double)__float_as_int(a.mn) : (double)a.mn) * unit + base;
+    const double hi = (fixq ? (double)__float_as_int(a.mx) : (double)a.mx) * unit + base;
+    mn = lo < mn ? lo : mn;
+    mx = hi > mx ? hi : mx;
+    sum = a.sum * unit + (double)a.n * base;
+  }
+  out[(s * 3 + 0) * ND + d] = mn;
+  out[(s * 3 + 1) * ND + d] = mx;
+  out[(s * 3 + 2) * ND + d] = sum * dV;
 }
 
 }  // namespace csp

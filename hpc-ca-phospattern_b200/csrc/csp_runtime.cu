@@ -8,6 +8,8 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
+#include <condition_variable>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -19,6 +21,7 @@
 #include <ctime>
 #include <random>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "csp_kernels.cuh"
@@ -158,8 +161,10 @@ struct csp_handle {
   FluxParams* d_params = nullptr;
   unsigned char* d_states = nullptr;
   int* d_err = nullptr;
-  double* d_red = nullptr;
+  RedPart* d_red = nullptr;
   double* d_red_out = nullptr;
+  double* d_line = nullptr;             // csp_linescan: weights and bins
+  size_t line_elems = 0;
   void* d_stage = nullptr;           // host-state staging of upload / download (one realisation)
   size_t stage_bytes = 0;
   // asynchronous snapshots: FP64 fields converted on the handle stream into d_snap, copied
@@ -169,6 +174,10 @@ struct csp_handle {
   size_t snap_elems = 0;
   cudaStream_t snap_stream = nullptr;
   cudaEvent_t ev_snap = nullptr, ev_copy = nullptr;
+  cudaEvent_t ev_snap_sp[NS] = {};      // the species' copies of the pending snapshot
+  size_t snap_nvox = 0;                 // its voxels, species and their mask
+  int snap_ns = 0;
+  uint32_t snap_mask = 0;
   bool snap_pending = false;
   bool advance_pending = false;
   int nrows = 0, nch = 0;
@@ -1146,9 +1155,8 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     csp_destroy(h);
     return fail(nullptr, CSP_ECUDA, "descriptor upload: %s", cudaGetErrorString(e));
   }
-  const int red_blocks = 296;
-  if (cudaMalloc(&h->d_red, red_blocks * 3 * ND * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->d_red_out, 3 * ND * sizeof(double)) != cudaSuccess) {
+  if (cudaMalloc(&h->d_red, (size_t)RED_BLOCKS * NS * ND * sizeof(RedPart)) != cudaSuccess ||
+      cudaMalloc(&h->d_red_out, 3 * NS * ND * sizeof(double) + std::max(h->nch, 1)) != cudaSuccess) {
     csp_destroy(h);
     return fail(nullptr, CSP_ENOMEM, "device allocation of reduction buffers failed");
   }
@@ -2046,8 +2054,13 @@ extern "C" int csp_snapshot_async(csp_handle* h, int32_t r, uint32_t species_mas
     const size_t off = (size_t)sp * m.nvox;
     CUDA_TRY(h, cudaMemcpyAsync(h->h_snap + off, h->d_snap + off, (size_t)m.nvox * sizeof(double),
                                 cudaMemcpyDeviceToHost, h->snap_stream));
+    if (!h->ev_snap_sp[sp]) CUDA_TRY(h, cudaEventCreateWithFlags(&h->ev_snap_sp[sp], cudaEventDisableTiming));
+    CUDA_TRY(h, cudaEventRecord(h->ev_snap_sp[sp], h->snap_stream));
   }
   CUDA_TRY(h, cudaEventRecord(h->ev_copy, h->snap_stream));
+  h->snap_nvox = (size_t)m.nvox;
+  h->snap_ns = m.ns;
+  h->snap_mask = species_mask;
   h->snap_pending = true;
   return CSP_OK;
 }
@@ -2058,6 +2071,76 @@ extern "C" int csp_snapshot_wait(csp_handle* h, const double** u) {
   h->snap_pending = false;
   CUDA_TRY(h, cudaEventSynchronize(h->ev_copy));
   *u = h->h_snap;
+  return CSP_OK;
+}
+
+// The pending snapshot into the caller's memory, each species as its copy from the device ends.
+// Fresh memory costs more to touch than the bytes to move (160 MB by one thread: 30 ms, half of
+// it the pages' first touch), so SNAP_THREADS host threads share it: 6.2 ms, 3.1 of them the
+// copy from the device (8 threads 7.7, 24 threads 6.1; pieces of 512 KB 7.4).  A piece is long
+// enough to cover a large page; below four pieces a thread is not worth its start (~50 us).
+constexpr size_t SNAP_PIECE = 2u << 20;
+constexpr unsigned SNAP_THREADS = 12;
+
+extern "C" int csp_snapshot_read(csp_handle* h, double* u) {
+  if (!h || !u) return CSP_EINVAL;
+  if (!h->snap_pending) return fail(h, CSP_EINVAL, "no snapshot is pending");
+  h->snap_pending = false;
+  const size_t sp_bytes = h->snap_nvox * sizeof(double);
+  const size_t pieces = (sp_bytes + SNAP_PIECE - 1) / SNAP_PIECE;      // per species
+  std::vector<int> order;
+  for (int sp = 0; sp < h->snap_ns; sp++)
+    if (h->snap_mask >> sp & 1u) order.push_back(sp);
+  const size_t total = pieces * order.size();
+  std::mutex mu;
+  std::condition_variable cv;
+  size_t ready = 0;                    // species of `order` that have arrived
+  std::atomic<size_t> next{0};
+  std::atomic<bool> stop{false};
+  auto work = [&](bool wait) {
+    while (!stop.load()) {
+      if (!wait && next.load() >= pieces * ready) return;      // (the main thread: only what is there)
+      const size_t i = next.fetch_add(1);
+      if (i >= total) return;
+      const size_t k = i / pieces;
+      if (wait) {
+        std::unique_lock<std::mutex> lock(mu);
+        cv.wait(lock, [&]() { return ready > k || stop.load(); });
+        if (ready <= k) return;
+      }
+      const size_t o = (i - k * pieces) * SNAP_PIECE, n = std::min(SNAP_PIECE, sp_bytes - o);
+      std::memcpy(reinterpret_cast<char*>(u) + (size_t)order[k] * sp_bytes + o,
+                  reinterpret_cast<const char*>(h->h_snap) + (size_t)order[k] * sp_bytes + o, n);
+    }
+  };
+  const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+  const size_t nthreads = std::min<size_t>({SNAP_THREADS, (size_t)cores, total / 4});
+  std::vector<std::thread> threads;
+  try {
+    threads.reserve(nthreads);
+    for (size_t t = 0; t < nthreads; t++) threads.emplace_back(work, true);
+  } catch (...) {                      // no more threads: those that started do the work, or this one
+  }
+  cudaError_t e = cudaSuccess;
+  for (size_t k = 0; k < order.size() && e == cudaSuccess; k++) {
+    e = cudaEventSynchronize(h->ev_snap_sp[order[k]]);
+    if (e != cudaSuccess) break;
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      ready = k + 1;
+    }
+    cv.notify_all();
+    if (threads.empty())
+      while (next.load() < pieces * ready) work(false);
+  }
+  if (e != cudaSuccess) {
+    std::lock_guard<std::mutex> lock(mu);
+    stop = true;
+  }
+  cv.notify_all();
+  for (std::thread& t : threads) t.join();
+  if (e == cudaSuccess) e = cudaEventSynchronize(h->ev_copy);
+  if (e != cudaSuccess) return fail(h, CSP_ECUDA, "snapshot: %s", cudaGetErrorString(e));
   return CSP_OK;
 }
 
@@ -2111,45 +2194,75 @@ extern "C" int csp_set_channel_states(csp_handle* h, int32_t r, int32_t boundary
 // index i of A (FP64 bins in shared memory, then one global add per bin and block), and
 // the host finishes out[a] = sum_i S[i] g((a - i) h).
 struct LinescanMap {
-  const float* f;
+  const float* f[2];         // both buffers of the species
+  const RealCtl* ctl;        // the realisation's progress block: which one is current
+  int species;
   const unsigned char* dom;
   double base[ND];           // the species' field base per domain
   int fixq;                  // the species is stored in fixed point: value = base + q * qunit
   double qunit[ND];
-  int nd[3];                 // device extents (n0, n1, row stride)
-  int nzv;                   // voxels per row
+  int n0, n1;                // device extents
+  int nz, nzv;               // row stride, voxels per row
   int P;
-  int phys_of_dev[3];        // physical axis of each device axis
-  int axis;                  // scanned physical axis
+  int axis;                  // the scanned device axis
   int num_domains;           // > 0: only voxels with domain id < num_domains
-  const double* w[3];        // per physical axis weights (the scanned axis: unused)
+  const double* w[3];        // per device axis weights (the scanned axis: ones)
   int nbins;
 };
 
-__global__ void k_linescan_bins(LinescanMap m, double* __restrict__ bins) {
+// Weighted sums of a species over the planes of the scanned axis, added to bins.
+// Bound by reading field and domain bytes once.  A warp takes whole rows: along the scanned
+// row axis (2) each lane keeps the sums of its voxels over the warp's rows, else the row's sum
+// goes to its plane's bin by one add.  4 M voxels through csp_linescan: 76-94 us (a shared FP64
+// atomic per voxel, the device buffer allocated per call and nbins^2 exponentials on the
+// host: 280-420 us).
+constexpr int LINE_T = 256, LINE_Z = 8;      // LINE_Z * 32 voxels of a row at a time
+__global__ void __launch_bounds__(LINE_T) k_linescan_bins(LinescanMap m, double* __restrict__ bins) {
   extern __shared__ double sb[];
-  for (int i = threadIdx.x; i < m.nbins; i += blockDim.x) sb[i] = 0.0;
+  for (int i = threadIdx.x; i < m.nbins; i += LINE_T) sb[i] = 0.0;
   __syncthreads();
-  const long long plane = (long long)m.nd[1] * m.nd[2];
-  const long long total = (long long)m.nd[0] * plane;
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total;
-       v += (long long)gridDim.x * blockDim.x) {
-    const int c0 = (int)(v / plane);
-    const long long rem = v - c0 * plane;
-    const int c1 = (int)(rem / m.nd[2]), c2 = (int)(rem - (long long)c1 * m.nd[2]);
-    if (c2 >= m.nzv) continue;
-    const long long dv = (long long)c0 * m.P + rem;
-    const int dom = m.dom[dv] & DOMAIN_BITS;
-    if (m.num_domains > 0 && dom >= m.num_domains) continue;
-    int pc[3];
-    pc[m.phys_of_dev[0]] = c0; pc[m.phys_of_dev[1]] = c1; pc[m.phys_of_dev[2]] = c2;
-    double w = (m.fixq ? (double)__float_as_int(m.f[dv]) * m.qunit[dom] : (double)m.f[dv]) + m.base[dom];
-    for (int a = 0; a < 3; a++)
-      if (a != m.axis) w *= m.w[a][pc[a]];
-    atomicAdd(&sb[pc[m.axis]], w);
+  const int lane = threadIdx.x & 31;
+  const unsigned cur = m.ctl->cur_mask[m.ctl->step & 1];
+  const float* __restrict__ f = m.f[(cur >> m.species) & 1u];
+  const long long rows = (long long)m.n0 * m.n1;
+  const int warps = (int)gridDim.x * (LINE_T / 32);
+  const int w0 = (int)blockIdx.x * (LINE_T / 32) + (int)(threadIdx.x >> 5);
+  // the warp's rows, neighbours in memory
+  const long long r0 = rows * w0 / warps, r1 = rows * (w0 + 1) / warps;
+  auto value = [&](long long v) {
+    const int d = m.dom[v] & DOMAIN_BITS;
+    if (m.num_domains > 0 && d >= m.num_domains) return 0.0;
+    const float x = f[v];
+    return (m.fixq ? (double)__float_as_int(x) * m.qunit[d] : (double)x) + m.base[d];
+  };
+  for (int z0 = 0; z0 < m.nzv; z0 += 32 * LINE_Z) {
+    double acc[LINE_Z] = {}, wz[LINE_Z];
+#pragma unroll
+    for (int j = 0; j < LINE_Z; j++) wz[j] = z0 + 32 * j + lane < m.nzv ? m.w[2][z0 + 32 * j + lane] : 0.0;
+    for (long long row = r0; row < r1; row++) {
+      const int c0 = (int)(row / m.n1), c1 = (int)(row - (long long)c0 * m.n1);
+      const long long o = (long long)c0 * m.P + (long long)c1 * m.nz + z0 + lane;
+      const double wr = m.w[0][c0] * m.w[1][c1];
+      double sum = 0.0;
+#pragma unroll
+      for (int j = 0; j < LINE_Z; j++) {
+        if (z0 + 32 * j + lane >= m.nzv) break;
+        const double v = value(o + 32 * j);
+        if (m.axis == 2) acc[j] += v * wr;
+        else sum += v * wz[j];
+      }
+      if (m.axis == 2) continue;
+#pragma unroll
+      for (int k = 16; k; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+      if (lane == 0) atomicAdd(&sb[m.axis == 0 ? c0 : c1], sum * wr);
+    }
+    if (m.axis != 2) continue;
+#pragma unroll
+    for (int j = 0; j < LINE_Z; j++)
+      if (z0 + 32 * j + lane < m.nzv) atomicAdd(&sb[z0 + 32 * j + lane], acc[j]);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < m.nbins; i += blockDim.x)
+  for (int i = threadIdx.x; i < m.nbins; i += LINE_T)
     if (sb[i] != 0.0) atomicAdd(&bins[i], sb[i]);
 }
 
@@ -2168,54 +2281,61 @@ extern "C" int csp_linescan(csp_handle* h, int32_t r, int32_t species, int32_t a
   if (axis < 0 || axis > 2) return fail(h, CSP_ERANGE, "axis %d out of range", axis);
   const int nA = hr.nphys[axis];
   if ((size_t)nA * sizeof(double) > 48 * 1024) return fail(h, CSP_ENOTSUP, "linescan axis of %d voxels", nA);
-  RealCtl c;
-  int rc = read_ctl(h, r, c);
-  if (rc) return rc;
-  const unsigned cur = c.cur_mask[c.step & 1];
   const double hs = hr.info.h;
-  // weights of the two fixed axes, then one device buffer: [w0 | w1 | w2 | bins]
+  // one device buffer: [weights of the device axes | bins]
   std::vector<double> host;
   size_t woff[3];
-  for (int a = 0; a < 3; a++) {
-    woff[a] = host.size();
-    for (int i = 0; i < hr.nphys[a]; i++)
-      host.push_back(a == axis ? 0.0 : gauss_weight(offsets_nm[a] - i * hs, conv[a]));
+  int dev_axis = 0;
+  for (int i = 0; i < 3; i++) {
+    const int a = hr.perm[i];
+    if (a == axis) dev_axis = i;
+    woff[i] = host.size();
+    for (int k = 0; k < hr.nphys[a]; k++)
+      host.push_back(a == axis ? 1.0 : gauss_weight(offsets_nm[a] - k * hs, conv[a]));
   }
   const size_t boff = host.size();
   host.resize(boff + nA, 0.0);
-  double* dbuf = nullptr;
-  if (cudaMalloc(&dbuf, host.size() * sizeof(double)) != cudaSuccess)
-    return fail(h, CSP_ENOMEM, "linescan buffer");
+  if (host.size() > h->line_elems) {
+    cudaFree(h->d_line);
+    h->d_line = nullptr;
+    h->line_elems = 0;
+    if (cudaMalloc(&h->d_line, host.size() * sizeof(double)) != cudaSuccess)
+      return fail(h, CSP_ENOMEM, "linescan buffer");
+    h->line_elems = host.size();
+  }
   LinescanMap m;
-  m.f = D.u[(cur >> species) & 1u][species];
+  m.f[0] = D.u[0][species];
+  m.f[1] = D.u[1][species];
+  m.ctl = h->d_ctl + r;
+  m.species = species;
   m.dom = D.dom;
   for (int dd = 0; dd < ND; dd++) {
     m.base[dd] = D.base[dd][species];
     m.qunit[dd] = D.qunit[dd][species];
   }
   m.fixq = (D.fixq >> species) & 1u;
-  m.nd[0] = D.nx; m.nd[1] = D.ny; m.nd[2] = D.nz;
+  m.n0 = D.nx;
+  m.n1 = D.ny;
+  m.nz = D.nz;
   m.nzv = D.nzv;
   m.P = D.P;
-  for (int i = 0; i < 3; i++) m.phys_of_dev[i] = hr.perm[i];
-  m.axis = axis;
+  m.axis = dev_axis;
   m.num_domains = num_domains;
-  for (int a = 0; a < 3; a++) m.w[a] = dbuf + woff[a];
+  for (int i = 0; i < 3; i++) m.w[i] = h->d_line + woff[i];
   m.nbins = nA;
-  cudaError_t e = cudaMemcpyAsync(dbuf, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) {
-    k_linescan_bins<<<592, 256, nA * sizeof(double), h->stream>>>(m, dbuf + boff);
-    e = cudaGetLastError();
-  }
-  std::vector<double> bins(nA);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(bins.data(), dbuf + boff, nA * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(dbuf);
-  if (e != cudaSuccess) return fail(h, CSP_ECUDA, "linescan: %s", cudaGetErrorString(e));
+  std::vector<double> bins(nA), table(nA);
+  CUDA_TRY(h, cudaMemcpyAsync(h->d_line, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  const long long rows = (long long)D.nx * D.ny;
+  const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(592, rows / (LINE_T / 32)));
+  k_linescan_bins<<<blocks, LINE_T, nA * sizeof(double), h->stream>>>(m, h->d_line + boff);
+  CUDA_TRY(h, cudaGetLastError());
+  // the scanned axis' weights by distance, while the device sums
+  for (int a = 0; a < nA; a++) table[a] = gauss_weight(a * hs, conv[axis]);
+  CUDA_TRY(h, cudaMemcpyAsync(bins.data(), h->d_line + boff, nA * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   for (int a = 0; a < nA; a++) {
     double acc = 0.0;
-    for (int i = 0; i < nA; i++) acc += bins[i] * gauss_weight((a - i) * hs, conv[axis]);
+    for (int i = 0; i < nA; i++) acc += bins[i] * table[a < i ? i - a : a - i];
     out[a] = acc;
   }
   return CSP_OK;
@@ -2228,27 +2348,37 @@ extern "C" int csp_reduce_outputs(csp_handle* h, int32_t r, double* min_values, 
   if (r < 0 || r >= h->n) return fail(h, CSP_ERANGE, "realisation %d out of range", r);
   const HostReal& hr = h->real[r];
   const RealDesc& D = hr.desc;
-  const int nblk = 296;
-  double out[3 * ND];
-  for (int s = 0; s < D.ns; s++) {
-    k_reduce_partial<<<nblk, 256, 0, h->stream>>>(h->d_desc, h->d_ctl, r, s, h->d_red);
-    k_reduce_final<<<1, 32, 0, h->stream>>>(h->d_red, nblk, hr.dV, h->d_red_out);
-    CUDA_TRY(h, cudaGetLastError());
-    CUDA_TRY(h, cudaMemcpyAsync(out, h->d_red_out, sizeof out, cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    for (int d = 0; d < hr.nd; d++) {
-      if (min_values) min_values[d * D.ns + s] = out[0 * ND + d];
-      if (max_values) max_values[d * D.ns + s] = out[1 * ND + d];
-      if (total_values) total_values[d * D.ns + s] = out[2 * ND + d];
-    }
+  // the realisation's channels: one range of the state bytes
+  int ch0 = 0, nch = 0;
+  for (size_t b = 0; openness && b < hr.boundary_channel_base.size(); b++) {
+    if (hr.boundary_channel_base[b] < 0) continue;
+    if (nch == 0) ch0 = hr.boundary_channel_base[b];
+    ch0 = std::min(ch0, hr.boundary_channel_base[b]);
+    nch += hr.boundary_nch[b];
   }
+  const long long groups = (long long)D.nx * (D.plane / 4);
+  const int nblk = (int)std::max<long long>(1, std::min<long long>(RED_BLOCKS, (groups + RED_T - 1) / RED_T));
+  unsigned char* d_open = reinterpret_cast<unsigned char*>(h->d_red_out + 3 * NS * ND);
+  k_reduce_partial<<<dim3(nblk, D.ns), RED_T, 0, h->stream>>>(h->d_desc, h->d_ctl, r, h->d_red);
+  k_reduce_final<<<D.ns + (nch ? (nch + 1023) / 1024 : 0), 32 * ND, 0, h->stream>>>(
+      h->d_desc, h->d_ctl, r, h->d_red, nblk, hr.dV, h->d_red_out, h->d_states, std::max(h->nch, 1), ch0, nch, d_open);
+  CUDA_TRY(h, cudaGetLastError());
+  std::vector<double> out((3 * NS * ND * sizeof(double) + nch + 7) / 8);
+  CUDA_TRY(h, cudaMemcpyAsync(out.data(), h->d_red_out, 3 * NS * ND * sizeof(double) + nch, cudaMemcpyDeviceToHost,
+                              h->stream));
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  for (int s = 0; s < D.ns; s++)
+    for (int d = 0; d < hr.nd; d++) {
+      if (min_values) min_values[d * D.ns + s] = out[(s * 3 + 0) * ND + d];
+      if (max_values) max_values[d * D.ns + s] = out[(s * 3 + 1) * ND + d];
+      if (total_values) total_values[d * D.ns + s] = out[(s * 3 + 2) * ND + d];
+    }
   if (openness) {
-    int off = 0;
+    const unsigned char* open = reinterpret_cast<const unsigned char*>(out.data() + 3 * NS * ND);
     for (size_t b = 0; b < hr.boundary_channel_base.size(); b++) {
       if (hr.boundary_channel_base[b] < 0) continue;
-      int rc = csp_get_channel_states(h, r, (int)b, openness + off);
-      if (rc) return rc;
-      off += hr.boundary_nch[b];
+      const unsigned char* p = open + (hr.boundary_channel_base[b] - ch0);
+      for (int i = 0; i < hr.boundary_nch[b]; i++) *openness++ = p[i];
     }
   }
   return CSP_OK;
@@ -2890,7 +3020,7 @@ extern "C" void csp_destroy(csp_handle* h) {
   cudaFree(h->d_fields); cudaFree(h->d_dom); cudaFree(h->d_gcode); cudaFree(h->d_desc); cudaFree(h->d_vdesc); cudaFree(h->d_ctl);
   cudaFree(h->d_rec); cudaFree(h->d_drows); cudaFree(h->d_mix); cudaFree(h->d_mixc); cudaFree(h->d_items);
   cudaFree(h->d_rows); cudaFree(h->d_entries); cudaFree(h->d_pairs); cudaFree(h->d_params);
-  cudaFree(h->d_states); cudaFree(h->d_err); cudaFree(h->d_red); cudaFree(h->d_red_out);
+  cudaFree(h->d_states); cudaFree(h->d_err); cudaFree(h->d_red); cudaFree(h->d_red_out); cudaFree(h->d_line);
   cudaFree(h->d_stage);
   if (h->in_stream) { cudaStreamSynchronize(h->in_stream); cudaStreamDestroy(h->in_stream); }
   cudaFree(h->d_pipe); cudaFree(h->d_stepflags);
@@ -2899,6 +3029,8 @@ extern "C" void csp_destroy(csp_handle* h) {
   cudaFreeHost(h->h_snap);
   if (h->ev_snap) cudaEventDestroy(h->ev_snap);
   if (h->ev_copy) cudaEventDestroy(h->ev_copy);
+  for (cudaEvent_t ev : h->ev_snap_sp)
+    if (ev) cudaEventDestroy(ev);
   if (h->snap_stream) cudaStreamDestroy(h->snap_stream);
   cudaFree(h->d_mlp); cudaFree(h->d_mlp_cnt); cudaFree(h->d_sur_list); cudaFree(h->d_sur_counts);
   cudaFree(h->d_sur_tiles); cudaFree(h->d_sur_queue); cudaFree(h->d_rx_class);

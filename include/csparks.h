@@ -252,6 +252,10 @@ int csp_advance_wait(csp_handle* h, int32_t* stop_flags);
 int csp_snapshot_async(csp_handle* h, int32_t r, uint32_t species_mask);
 int csp_snapshot_wait(csp_handle* h, const double** u);
 
+/* csp_snapshot_wait into the caller's memory (num_species * nx * ny * nz doubles), the
+ * requested species copied by several host threads as each arrives. */
+int csp_snapshot_read(csp_handle* h, double* u);
+
 /* Per (domain, species) min / max / sum(u*dV) in FP64, and the channel openness of
  * every discrete boundary in boundary order (Species_output_scalar_data,
  * species.c:2785-2880).  min/max/total: [num_domains][num_species]; openness: all
