@@ -142,12 +142,18 @@ __host__ __device__ inline void rx_plain(const RxConst& k, int n, double h, doub
   dc = cc - c;
 }
 
-__host__ __device__ inline void rx_features(const RxConst& k, int d, float dtr, float c, const float* b,
-                                            float* x) {
+__host__ __device__ inline float rx_feature_dt(float dtr) { return log10f(dtr) * 0.25f; }
+
+// (x6 = rx_feature_dt(dtr): the same for all voxels of a realisation)
+__host__ __device__ inline void rx_features_at(const RxConst& k, int d, float x6, float c, const float* b, float* x) {
   x[0] = log10f(fmaxf(c, 1e-3f)) * (1.f / 3.f);
   for (int q = 0; q < MLP_SLOTS; q++) x[1 + q] = k.tot[q] > 0.f ? b[q] / k.tot[q] : 0.f;
-  x[6] = log10f(dtr) * 0.25f;
+  x[6] = x6;
   x[7] = 0.25f * (float)d;
+}
+
+__host__ __device__ inline void rx_features(const RxConst& k, int d, float dtr, float c, const float* b, float* x) {
+  rx_features_at(k, d, rx_feature_dt(dtr), c, b, x);
 }
 
 // Training target of one sample: the correction t_s that turns the single explicit step
@@ -210,9 +216,13 @@ __device__ __forceinline__ void mlp_forward(const MlpW& W, const float* x, float
 // Weights sit in shared memory as TF32 bit patterns (converted once per CTA) in fragment
 // order: for k-block kb and n-tile pair np, lane l's four words (b0, b1 of n-tile 2np, then
 // of 2np + 1) are contiguous, so a lane fetches two B fragments with one 16-byte load
-// (the output layer, a single n-tile: two words).  Activations are staged per warp in a
-// [32][MLP_TC_LD] tile whose padded rows put the A-fragment loads in 32 different banks.
-constexpr int MLP_TC_LD = MLP_H + 4;     // padded row length (floats)
+// (the output layer, a single n-tile: two words).  The activations stay in registers: a
+// layer's C fragment of n-tile kb is the next layer's A fragment of k-block kb when the
+// units 8 kb + (2q, 2q + 1) of a lane take the columns (q, q + 4) of A, so the weights of
+// layers 2 and 3 have their rows in that order within a k-block (PERM).  Only inputs and
+// outputs pass through shared memory, in a [32][MLP_TC_LD] tile per warp whose rows put the
+// A-fragment loads in 32 different banks.
+constexpr int MLP_TC_LD = 12;            // row length of the inputs and outputs (floats)
 constexpr int MLP_TC_N3 = 8;             // output layer padded to one n-tile
 constexpr int MLP_F1 = (MLP_IN / 8) * (MLP_H / 16) * 32 * 4;
 constexpr int MLP_F2 = (MLP_H / 8) * (MLP_H / 16) * 32 * 4;
@@ -222,7 +232,7 @@ struct MlpTC {
   float b1[MLP_H], b2[MLP_H], b3[MLP_TC_N3];
 };
 static_assert(sizeof(MlpTC) % 16 == 0, "activation tiles follow the weights");
-constexpr int MLP_TC_STAGE = 32 * MLP_TC_LD;   // floats of one warp's activation tile
+constexpr int MLP_TC_STAGE = 32 * MLP_TC_LD;   // floats of one warp's inputs and outputs
 
 __device__ __forceinline__ unsigned tf32_bits(float f) {
   unsigned r;
@@ -232,7 +242,7 @@ __device__ __forceinline__ unsigned tf32_bits(float f) {
 
 // Fragment-order word i of a layer with K inputs, NT n-tiles and W = [K][NV] (columns
 // beyond NV read as 0).
-template <int K, int NT, int NV>
+template <int K, int NT, int NV, bool PERM>
 __device__ __forceinline__ unsigned mlp_frag_word(const float* W, int i) {
   int kb, nt, lane, h;
   if constexpr (NT >= 2) {
@@ -247,15 +257,15 @@ __device__ __forceinline__ unsigned mlp_frag_word(const float* W, int i) {
     kb = i >> 6;
     nt = 0;
   }
-  const int k = kb * 8 + (lane & 3) + 4 * h, n = nt * 8 + (lane >> 2);
+  const int q = lane & 3, k = kb * 8 + (PERM ? 2 * q + h : q + 4 * h), n = nt * 8 + (lane >> 2);
   return n < NV ? tf32_bits(W[k * NV + n]) : 0u;
 }
 
 __device__ __forceinline__ void mlp_tc_load(MlpTC& T, const float* __restrict__ p) {
   const MlpW& W = *reinterpret_cast<const MlpW*>(p);
-  for (int i = threadIdx.x; i < MLP_F1; i += blockDim.x) T.f1[i] = mlp_frag_word<MLP_IN, MLP_H / 8, MLP_H>(W.w1, i);
-  for (int i = threadIdx.x; i < MLP_F2; i += blockDim.x) T.f2[i] = mlp_frag_word<MLP_H, MLP_H / 8, MLP_H>(W.w2, i);
-  for (int i = threadIdx.x; i < MLP_F3; i += blockDim.x) T.f3[i] = mlp_frag_word<MLP_H, 1, MLP_OUT>(W.w3, i);
+  for (int i = threadIdx.x; i < MLP_F1; i += blockDim.x) T.f1[i] = mlp_frag_word<MLP_IN, MLP_H / 8, MLP_H, false>(W.w1, i);
+  for (int i = threadIdx.x; i < MLP_F2; i += blockDim.x) T.f2[i] = mlp_frag_word<MLP_H, MLP_H / 8, MLP_H, true>(W.w2, i);
+  for (int i = threadIdx.x; i < MLP_F3; i += blockDim.x) T.f3[i] = mlp_frag_word<MLP_H, 1, MLP_OUT, true>(W.w3, i);
   for (int i = threadIdx.x; i < MLP_H; i += blockDim.x) {
     T.b1[i] = W.b1[i];
     T.b2[i] = W.b2[i];
@@ -271,71 +281,88 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// out[32][NT*8] = act(in[32][K] W[K][NT*8] + bias), in / out: [32][MLP_TC_LD] warp tiles
-// (out may be in: every read of a tile precedes its writes, and mma.sync converges the warp)
-template <int K, int NT, bool RELU>
-__device__ __forceinline__ void mlp_tc_layer(const float* in, const unsigned* F, const float* bias, float* out,
+// acc (16 rows x 64 units, C fragments) = bias + A W over KB k-blocks; a(kb): the A fragment
+template <int KB, class A>
+__device__ __forceinline__ void mlp_tc_layer(A a, const unsigned* F, const float* bias, float (&acc)[MLP_H / 8][4],
                                              int lane) {
-  const int g = lane >> 2, q = lane & 3;
 #pragma unroll
-  for (int mt = 0; mt < 2; mt++) {
-    float acc[NT][4];
+  for (int nt = 0; nt < MLP_H / 8; nt++) {
+    const float2 bb = *reinterpret_cast<const float2*>(bias + nt * 8 + 2 * (lane & 3));
+    acc[nt][0] = acc[nt][2] = bb.x;
+    acc[nt][1] = acc[nt][3] = bb.y;
+  }
 #pragma unroll
-    for (int nt = 0; nt < NT; nt++) {
-      const float2 bb = *reinterpret_cast<const float2*>(bias + nt * 8 + 2 * q);
-      acc[nt][0] = acc[nt][2] = bb.x;
-      acc[nt][1] = acc[nt][3] = bb.y;
+  for (int kb = 0; kb < KB; kb++) {
+    unsigned av[4];
+    a(kb, av);
+#pragma unroll
+    for (int np = 0; np < MLP_H / 16; np++) {
+      const uint4 bb = *reinterpret_cast<const uint4*>(F + ((kb * (MLP_H / 16) + np) * 32 + lane) * 4);
+      const unsigned b0[2] = {bb.x, bb.y}, b1[2] = {bb.z, bb.w};
+      mma_tf32(acc[2 * np], av, b0);
+      mma_tf32(acc[2 * np + 1], av, b1);
     }
-    const float* r0 = in + (mt * 16 + g) * MLP_TC_LD;
-    const float* r1 = r0 + 8 * MLP_TC_LD;
-#pragma unroll
-    for (int kb = 0; kb < K / 8; kb++) {
-      const int k0 = kb * 8;
-      const unsigned a[4] = {tf32_bits(r0[k0 + q]), tf32_bits(r1[k0 + q]), tf32_bits(r0[k0 + q + 4]),
-                             tf32_bits(r1[k0 + q + 4])};
-      if constexpr (NT >= 2) {
-#pragma unroll
-        for (int np = 0; np < NT / 2; np++) {
-          const uint4 bb = *reinterpret_cast<const uint4*>(F + ((kb * (NT / 2) + np) * 32 + lane) * 4);
-          const unsigned b0[2] = {bb.x, bb.y}, b1[2] = {bb.z, bb.w};
-          mma_tf32(acc[2 * np], a, b0);
-          mma_tf32(acc[2 * np + 1], a, b1);
-        }
-      } else {
-        const uint2 bb = *reinterpret_cast<const uint2*>(F + (kb * 32 + lane) * 2);
-        const unsigned b0[2] = {bb.x, bb.y};
-        mma_tf32(acc[0], a, b0);
-      }
-    }
-    __syncwarp();
-    float* o0 = out + (mt * 16 + g) * MLP_TC_LD;
-    float* o1 = o0 + 8 * MLP_TC_LD;
-#pragma unroll
-    for (int nt = 0; nt < NT; nt++) {
-      float v[4] = {acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]};
-      if (RELU)
-        for (int i = 0; i < 4; i++) v[i] = fmaxf(v[i], 0.f);
-      o0[nt * 8 + 2 * q] = v[0];
-      o0[nt * 8 + 2 * q + 1] = v[1];
-      o1[nt * 8 + 2 * q] = v[2];
-      o1[nt * 8 + 2 * q + 1] = v[3];
-    }
-    __syncwarp();
   }
 }
 
-// Forward pass of the 32 lanes' samples; every lane of the warp must call it.
+// Forward pass of the 32 lanes' samples; every lane of the warp must call it.  The row tiles
+// one after the other: together they read each weight once (LSU busy 34 % instead of 57 %), but
+// their 64 activations per lane leave no registers for the voxel's values, whose loads then
+// wait (k_react_network 473 us instead of 405 for 3 M voxels; 419 with those values copied to
+// shared memory a tile ahead).
 __device__ __forceinline__ void mlp_forward_tc(const MlpTC& T, float* stage, const float* x, float* y) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   float* row = stage + lane * MLP_TC_LD;
-#pragma unroll
-  for (int i = 0; i < MLP_IN; i++) row[i] = x[i];
+  *reinterpret_cast<float4*>(row) = make_float4(x[0], x[1], x[2], x[3]);
+  *reinterpret_cast<float4*>(row + 4) = make_float4(x[4], x[5], x[6], x[7]);
   __syncwarp();
-  mlp_tc_layer<MLP_IN, MLP_H / 8, true>(stage, T.f1, T.b1, stage, lane);
-  mlp_tc_layer<MLP_H, MLP_H / 8, true>(stage, T.f2, T.b2, stage, lane);
-  mlp_tc_layer<MLP_H, 1, false>(stage, T.f3, T.b3, stage, lane);
+#pragma unroll 1
+  for (int mt = 0; mt < 2; mt++) {
+    float* r0 = stage + (mt * 16 + g) * MLP_TC_LD;
+    float* r1 = r0 + 8 * MLP_TC_LD;
+    float acc[MLP_H / 8][4];
+    unsigned h[MLP_H / 8][4];
+    // the activations of a lane as the next layer's A fragments
+    auto relu = [&]() {
 #pragma unroll
-  for (int i = 0; i < MLP_OUT; i++) y[i] = row[i];
+      for (int nt = 0; nt < MLP_H / 8; nt++) {
+        h[nt][0] = tf32_bits(fmaxf(acc[nt][0], 0.f));
+        h[nt][1] = tf32_bits(fmaxf(acc[nt][2], 0.f));
+        h[nt][2] = tf32_bits(fmaxf(acc[nt][1], 0.f));
+        h[nt][3] = tf32_bits(fmaxf(acc[nt][3], 0.f));
+      }
+    };
+    auto hidden = [&](int kb, unsigned (&a)[4]) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = h[kb][i];
+    };
+    mlp_tc_layer<MLP_IN / 8>(
+        [&](int, unsigned (&a)[4]) {
+          a[0] = tf32_bits(r0[q]);
+          a[1] = tf32_bits(r1[q]);
+          a[2] = tf32_bits(r0[q + 4]);
+          a[3] = tf32_bits(r1[q + 4]);
+        },
+        T.f1, T.b1, acc, lane);
+    relu();
+    mlp_tc_layer<MLP_H / 8>(hidden, T.f2, T.b2, acc, lane);
+    relu();
+    const float2 b3 = *reinterpret_cast<const float2*>(T.b3 + 2 * q);
+    float o[4] = {b3.x, b3.y, b3.x, b3.y};
+#pragma unroll
+    for (int kb = 0; kb < MLP_H / 8; kb++) {
+      const uint2 bb = *reinterpret_cast<const uint2*>(T.f3 + (kb * 32 + lane) * 2);
+      const unsigned b[2] = {bb.x, bb.y};
+      mma_tf32(o, h[kb], b);
+    }
+    __syncwarp();                                        // the tile's rows have been read
+    *reinterpret_cast<float2*>(r0 + 2 * q) = make_float2(o[0], o[1]);
+    *reinterpret_cast<float2*>(r1 + 2 * q) = make_float2(o[2], o[3]);
+  }
+  __syncwarp();
+  const float4 o = *reinterpret_cast<const float4*>(row);
+  y[0] = o.x; y[1] = o.y; y[2] = o.z; y[3] = o.w;
+  y[4] = row[4];
   __syncwarp();
 }
 
@@ -775,12 +802,20 @@ __device__ __forceinline__ void rx_load_old(const RxDom& K, const float* const* 
   }
 }
 
-// Replace the explicit increments the voxel kernel applied to voxel v by the surrogate's
-// (db[], dc): the explicit ones are recomputed from the same deviations and constants,
-// so they are the ones that were added.
+// The voxel's new values that rx_correct replaces, read beside the old ones: one trip to
+// memory instead of two.
+__device__ __forceinline__ void rx_load_new(const RxDom& K, float* const* un, long long v, float* now) {
+#pragma unroll
+  for (int s = 0; s < MLP_RX_NS; s++) now[s] = (K.store >> s & 1u) ? un[s][v] : 0.f;
+}
+
+// Replace the explicit increments the voxel kernel applied to voxel v (its new values now[])
+// by the surrogate's (db[], dc): the explicit ones are recomputed from the same deviations
+// and constants, so they are the ones that were added.
 template <unsigned FQ>
 __device__ __forceinline__ void rx_correct(const RxDom& K, const RealDesc& D, float* const* un, long long v,
-                                           unsigned fqs, const float* dev, float c, const float* db, float dc) {
+                                           unsigned fqs, const float* dev, const float* now, float c, const float* db,
+                                           float dc) {
   float sdj = 0.f;
 #pragma unroll
   for (int q = 0; q < MLP_SLOTS; q++) {
@@ -788,11 +823,15 @@ __device__ __forceinline__ void rx_correct(const RxDom& K, const RealDesc& D, fl
     const float4 k = K.rk[q + 1];
     const float dJ = buffer_dj(k.x, k.y, k.z, k.w, dev[q + 1], dev[0], c);
     sdj = __fadd_rn(sdj, dJ);
-    if (K.store >> (q + 1) & 1u) un[q + 1][v] = rx_add<FQ>(K, q + 1, un[q + 1][v], __fsub_rn(db[q], dJ), fqs);
+    if (K.store >> (q + 1) & 1u) un[q + 1][v] = rx_add<FQ>(K, q + 1, now[q + 1], __fsub_rn(db[q], dJ), fqs);
   }
   if (K.store & 1u) {
-    const int vi = (int)v, xq = vi / D.P;
-    if (!(D.dirichlet && rx_on_face(D, xq, vi - xq * D.P))) un[0][v] = __fadd_rn(un[0][v], __fadd_rn(sdj, dc));
+    bool face = false;
+    if (D.dirichlet) {
+      const int vi = (int)v, xq = vi / D.P;
+      face = rx_on_face(D, xq, vi - xq * D.P);
+    }
+    if (!face) un[0][v] = __fadd_rn(now[0], __fadd_rn(sdj, dc));
   }
 }
 
@@ -906,6 +945,7 @@ struct RxWarpCache {
   RxDom dom[8];
   const float* uo[MLP_RX_NS];
   float* un[MLP_RX_NS];
+  float dtr, x6;                         // the reaction's step and its feature
 };
 __device__ __forceinline__ void rx_cache_fill(const RealDesc& D, const RealCtl& C, RxWarpCache& W, int lane) {
   __syncwarp();
@@ -916,7 +956,47 @@ __device__ __forceinline__ void rx_cache_fill(const RealDesc& D, const RealCtl& 
     const unsigned cur = C.cur_mask[C.step & 1];
     W.uo[t] = t < D.ns ? D.u[(cur >> t) & 1u][t] : nullptr;
     W.un[t] = t < D.ns ? D.u[((cur >> t) & 1u) ^ 1u][t] : nullptr;
+  } else if (lane == 8 + MLP_RX_NS) {
+    W.dtr = (float)(D.dt * D.reaction_substep);
+    W.x6 = rx_feature_dt(W.dtr);
   }
+  __syncwarp();
+}
+
+// A warp's voxels whose network output was rejected, kept until they fill its 32 lanes: with 8 %
+// rejected nearly every tile held one, and the whole warp waited for its FP64 integration.
+// Together with activations in registers (mlp_forward_tc) and the new values read beside the
+// old ones, 200 steps of 24 100x100x50 grids, 20 of them reactions with 5.2 M network voxels
+// each: 42.5 -> 34.5 ms (k_react_network 20 -> 12 ms of it).
+struct RxRejects {
+  int v[64];
+  unsigned char d[64];
+};
+__device__ __forceinline__ void rx_reject(RxRejects& J, int& n, bool rejected, long long v, int d, int lane) {
+  const unsigned m = __ballot_sync(0xffffffffu, rejected);
+  if (rejected) {
+    const int i = n + __popc(m & ((1u << lane) - 1u));
+    J.v[i] = (int)v;
+    J.d[i] = (unsigned char)d;
+  }
+  n += __popc(m);
+  __syncwarp();
+}
+// The last min(n, 32) of them through the plain integrator, from the old state.
+template <unsigned FQ>
+__device__ __forceinline__ void rx_integrate_rejected(const RealDesc& D, const RxWarpCache& W, const RxRejects& J, int& n,
+                                                      int lane) {
+  const int first = n > 32 ? n - 32 : 0;
+  if (first + lane < n) {
+    const long long v = J.v[first + lane];
+    const RxDom& K = W.dom[J.d[first + lane]];
+    float dev[MLP_RX_NS], now[MLP_RX_NS], c, b[MLP_SLOTS], dc, db[MLP_SLOTS];
+    rx_load_old<FQ>(K, W.uo, v, D.fixq, dev, c, b);
+    rx_load_new(K, W.un, v, now);
+    rx_fallback(K.k, D.reaction_substep, D.dt, c, b, dc, db);
+    rx_correct<FQ>(K, D, W.un, v, D.fixq, dev, now, c, db, dc);
+  }
+  n = first;
   __syncwarp();
 }
 
@@ -932,12 +1012,12 @@ __device__ __forceinline__ RxTile rx_fetch_tile(const RealDesc* __restrict__ des
                                                 const unsigned* __restrict__ counts, unsigned td, int chunks,
                                                 int back, int lane) {
   RxTile f;
-  const long long seg = td >> MLP_TILE_BITS;
+  const unsigned seg = td >> MLP_TILE_BITS;
   const unsigned i = (td & ((1u << MLP_TILE_BITS) - 1u)) * 32u + lane;
-  f.r = (int)(seg / chunks);
-  f.have = i < counts[2 * seg + back];
-  const unsigned e = f.have ? list[seg * MLP_DEPLOY_SPAN + (back ? MLP_DEPLOY_SPAN - 1 - i : i)] : 0u;
-  f.v = (seg - (long long)f.r * chunks) * MLP_DEPLOY_SPAN + e;
+  f.r = (int)(seg / (unsigned)chunks);
+  f.have = i < counts[2 * (size_t)seg + back];
+  const unsigned e = f.have ? list[(long long)seg * MLP_DEPLOY_SPAN + (back ? MLP_DEPLOY_SPAN - 1 - i : i)] : 0u;
+  f.v = (long long)(seg - (unsigned)f.r * (unsigned)chunks) * MLP_DEPLOY_SPAN + e;
   f.d = f.have ? (descs[f.r].dom[f.v] & DOMAIN_BITS) : 0;
   return f;
 }
@@ -949,6 +1029,8 @@ __device__ __forceinline__ RxTile rx_fetch_tile(const RealDesc* __restrict__ des
 // queued tiles (tiles of one list are queued together, so a warp's realisation rarely
 // changes); a CTA without a tile returns before it loads the weights.  The next tile's
 // index chain is fetched while a tile runs.  chunks = the segments per realisation.
+// Bound by instructions in flight: some 2,000 per tile, 500 of them the network's, at half
+// of the issue slots with the 16 warps that 128 registers allow; LSU 57 % busy.
 template <unsigned FQ>
 __global__ void __launch_bounds__(MLP_DEPLOY_T, 2) k_react_network(const RealDesc* __restrict__ descs,
                                                                    const RealCtl* __restrict__ ctl,
@@ -963,6 +1045,7 @@ __global__ void __launch_bounds__(MLP_DEPLOY_T, 2) k_react_network(const RealDes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* stage = dsm + sizeof(MlpTC) / sizeof(float) + warp * MLP_TC_STAGE;
   __shared__ RxWarpCache s_wc[MLP_DEPLOY_T / 32];
+  __shared__ RxRejects s_rej[MLP_DEPLOY_T / 32];
   __shared__ unsigned s_net, s_fall, s_total;
   if (threadIdx.x == 0) { s_total = queue[0]; s_net = 0; s_fall = 0; }
   __syncthreads();
@@ -974,39 +1057,44 @@ __global__ void __launch_bounds__(MLP_DEPLOY_T, 2) k_react_network(const RealDes
     RxWarpCache& W = s_wc[warp];
     const unsigned t_lo = (blockIdx.x * (MLP_DEPLOY_T / 32) + warp) * per, t_hi = min(total, t_lo + per);
     unsigned n_net = 0, n_fall = 0;
+    int n_rej = 0;
     int rc = -1;                                         // realisation whose constants are cached
     RxTile nx{};
     if (t_lo < t_hi) nx = rx_fetch_tile(descs, list, counts, tiles[t_lo], chunks, 0, lane);
-    for (unsigned tw = t_lo; tw < t_hi; tw++) {
+    for (unsigned tw = t_lo;; tw++) {
       const RxTile cu = nx;
+      const bool flush = tw >= t_hi || cu.r != rc;       // warp-uniform
+      while (n_rej >= (flush ? 1 : 32)) rx_integrate_rejected<FQ>(descs[rc], W, s_rej[warp], n_rej, lane);
+      if (tw >= t_hi) break;
       if (tw + 1 < t_hi) nx = rx_fetch_tile(descs, list, counts, tiles[tw + 1], chunks, 0, lane);
       const RealDesc& D = descs[cu.r];
-      if (cu.r != rc) {                                  // warp-uniform
+      if (cu.r != rc) {
         rx_cache_fill(D, ctl[cu.r], W, lane);
         rc = cu.r;
       }
-      const float dtr = (float)(D.dt * D.reaction_substep);
+      const float dtr = W.dtr;
       const unsigned fqs = D.fixq;
       const RxDom& K = W.dom[cu.d];
-      float dev[MLP_RX_NS], c = 0.f, b[MLP_SLOTS], x[MLP_IN], t[MLP_OUT];
+      float dev[MLP_RX_NS], now[MLP_RX_NS], c = 0.f, b[MLP_SLOTS], x[MLP_IN], t[MLP_OUT];
 #pragma unroll
       for (int i = 0; i < MLP_IN; i++) x[i] = 0.f;
 #pragma unroll
       for (int q = 0; q < MLP_SLOTS; q++) b[q] = 0.f;
       if (cu.have) {
         rx_load_old<FQ>(K, W.uo, cu.v, fqs, dev, c, b);
-        rx_features(K.k, cu.d, dtr, c, b, x);
+        rx_load_new(K, W.un, cu.v, now);
+        rx_features_at(K.k, cu.d, W.x6, c, b, x);
       }
       mlp_forward_tc(T, stage, x, t);
+      bool rejected = false;
       if (cu.have) {
         float dc, db[MLP_SLOTS];
         n_net++;
-        if (!rx_apply_output(K.k, dtr, c, b, t, tol, dc, db)) {
-          n_fall++;
-          rx_fallback(K.k, D.reaction_substep, D.dt, c, b, dc, db);
-        }
-        rx_correct<FQ>(K, D, W.un, cu.v, fqs, dev, c, db, dc);
+        rejected = !rx_apply_output(K.k, dtr, c, b, t, tol, dc, db);
+        if (rejected) n_fall++;
+        else rx_correct<FQ>(K, D, W.un, cu.v, fqs, dev, now, c, db, dc);
       }
+      rx_reject(s_rej[warp], n_rej, rejected, cu.v, cu.d, lane);
     }
     if (n_net) atomicAdd(&s_net, n_net);
     if (n_fall) atomicAdd(&s_fall, n_fall);
@@ -1039,6 +1127,7 @@ __global__ void __launch_bounds__(UM_T * UM_NET_WGS, 2) k_react_network_umma(con
                                                                           int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char um_sm[];
   __shared__ RxWarpCache s_wc[UM_NET_WGS * UM_T / 32];
+  __shared__ RxRejects s_rej[UM_NET_WGS * UM_T / 32];
   __shared__ unsigned s_net, s_fall, s_total;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wi = warp & 3, wg = warp >> 2;
   if (threadIdx.x == 0) { s_total = queue[0]; s_net = 0; s_fall = 0; }
@@ -1057,19 +1146,23 @@ __global__ void __launch_bounds__(UM_T * UM_NET_WGS, 2) k_react_network_umma(con
     const unsigned tmem = um_tmem_alloc(um_sm, UM_NET_WGS * UM_TMEM_COLS);
     const UmWg G = um_wg(um_sm, wg, tmem);
     unsigned phase = 0, n_net = 0, n_fall = 0;
+    int n_rej = 0;
     RxWarpCache& W = s_wc[warp];
     int rc = -1;                                         // realisation whose constants this warp caches
     RxTile nx{};
     const unsigned g0 = g_lo + (unsigned)wg;
     if (g0 < g_hi && 4 * g0 + wi < total) nx = rx_fetch_tile(descs, list, counts, tiles[4 * g0 + wi], chunks, 0, lane);
-    for (unsigned g = g0; g < g_hi; g += UM_NET_WGS) {  // uniform over the warpgroup
-      const bool tile = 4 * g + wi < total;              // warp-uniform
+    for (unsigned g = g0;; g += UM_NET_WGS) {            // uniform over the warpgroup
+      const bool end = g >= g_hi, tile = !end && 4 * g + wi < total;   // warp-uniform
       RxTile cu = nx;
       if (!tile) cu.have = false;
+      const bool flush = end || (tile && cu.r != rc);
+      while (n_rej >= (flush ? 1 : 32)) rx_integrate_rejected<FQ>(descs[rc], W, s_rej[warp], n_rej, lane);
+      if (end) break;
       const unsigned gn = g + UM_NET_WGS;
       if (gn < g_hi && 4 * gn + wi < total)
         nx = rx_fetch_tile(descs, list, counts, tiles[4 * gn + wi], chunks, 0, lane);
-      float dev[MLP_RX_NS], c = 0.f, b[MLP_SLOTS], x[MLP_IN], t[MLP_OUT];
+      float dev[MLP_RX_NS], now[MLP_RX_NS], c = 0.f, b[MLP_SLOTS], x[MLP_IN], t[MLP_OUT];
 #pragma unroll
       for (int i = 0; i < MLP_IN; i++) x[i] = 0.f;
 #pragma unroll
@@ -1079,12 +1172,13 @@ __global__ void __launch_bounds__(UM_T * UM_NET_WGS, 2) k_react_network_umma(con
         rx_cache_fill(D, ctl[cu.r], W, lane);
         rc = cu.r;
       }
-      const float dtr = (float)(D.dt * D.reaction_substep);
+      const float dtr = W.dtr;
       const unsigned fqs = D.fixq;
       const RxDom& K = W.dom[cu.d];
       if (cu.have) {
         rx_load_old<FQ>(K, W.uo, cu.v, fqs, dev, c, b);
-        rx_features(K.k, cu.d, dtr, c, b, x);
+        rx_load_new(K, W.un, cu.v, now);
+        rx_features_at(K.k, cu.d, W.x6, c, b, x);
       }
       if (!mlp_forward_umma(um_sm, G, phase, x, t)) {
         if ((threadIdx.x & 127) == 0) {
@@ -1093,15 +1187,15 @@ __global__ void __launch_bounds__(UM_T * UM_NET_WGS, 2) k_react_network_umma(con
         }
         break;
       }
+      bool rejected = false;
       if (cu.have) {
         float dc, db[MLP_SLOTS];
         n_net++;
-        if (!rx_apply_output(K.k, dtr, c, b, t, tol, dc, db)) {
-          n_fall++;
-          rx_fallback(K.k, D.reaction_substep, D.dt, c, b, dc, db);
-        }
-        rx_correct<FQ>(K, D, W.un, cu.v, fqs, dev, c, db, dc);
+        rejected = !rx_apply_output(K.k, dtr, c, b, t, tol, dc, db);
+        if (rejected) n_fall++;
+        else rx_correct<FQ>(K, D, W.un, cu.v, fqs, dev, now, c, db, dc);
       }
+      rx_reject(s_rej[warp], n_rej, rejected, cu.v, cu.d, lane);
     }
     um_tmem_free(tmem, UM_NET_WGS * UM_TMEM_COLS);
     if (n_net) atomicAdd(&s_net, n_net);
@@ -1153,10 +1247,12 @@ __global__ void __launch_bounds__(MLP_DEPLOY_T, 4) k_react_plain(const RealDesc*
         const RxDom& K = W.dom[cu.d];
         const unsigned fqs = D.fixq;
         float dev[MLP_RX_NS], c, b[MLP_SLOTS], dc, db[MLP_SLOTS];
+        float now[MLP_RX_NS];
         rx_load_old<FQ>(K, W.uo, cu.v, fqs, dev, c, b);
         n_fall++;
         rx_fallback(K.k, D.reaction_substep, D.dt, c, b, dc, db);
-        rx_correct<FQ>(K, D, W.un, cu.v, fqs, dev, c, db, dc);
+        rx_load_new(K, W.un, cu.v, now);
+        rx_correct<FQ>(K, D, W.un, cu.v, fqs, dev, now, c, db, dc);
       }
     }
     if (n_fall) atomicAdd(&s_fall, n_fall);

@@ -1342,7 +1342,9 @@ static cudaError_t launch_march(csp_handle* h, const MarchPlan& pl, long long ns
   a.flag_stride = h->n;
   a.err = h->d_err;
   a.inject = h->inject_wait;
-  MarchKernel k = march_kernel(h->ms, h->fixq, h->surrogate != 0);
+  // the classification belongs to a reaction step, which is launched alone (launch_steps); the
+  // stretches between take the kernel without it
+  MarchKernel k = march_kernel(h->ms, h->fixq, h->surrogate != 0 && !(what & (MARCH_ADVANCE | MARCH_REPEAT)));
   const unsigned grid = (unsigned)(pl.teams * pl.size);
   if (pl.size == 1 || !(what & (MARCH_ADVANCE | MARCH_REPEAT))) {
     k<<<grid, MARCH_T, sizeof(MarchShared), h->stream>>>(a);
