@@ -93,7 +93,8 @@ struct MarchStep {
 struct MarchShared {
   alignas(16) VoxDesc desc;
   MarchStep step;
-  // the same on every step: the segments, and the entries of every warp's first boundary tile
+  int next;                          // items of the step that a warp has taken beyond its first
+  // the same on every step: the segments, and the entries of the CTA's first boundary tiles
   int cut[MARCH_CUTS];
   alignas(16) int4 tile[MARCH_T][2];
 };
@@ -692,7 +693,7 @@ __device__ __forceinline__ void mixed_voxel(const VoxDesc& D, const MarchStep& U
 }
 
 // A CTA's share of a realisation's step: units [u0, u1) and boundary tiles [t0, t1) (of 32
-// voxels, those with channels first), dealt to its warps in turn, units first.  Contiguous
+// voxels, those with channels first), taken by its warps as they come free, units first.  Contiguous
 // units share their columns' rows in L1; the tiles, whose lanes touch a line each, are spread
 // evenly over the CTAs (16 of them on one SM took twice the time of one).
 struct MarchShare {
@@ -723,22 +724,36 @@ __device__ __forceinline__ bool march_entry(const MarchArgs& A, const MarchReal&
   return true;
 }
 
-// The boundary tiles of a warp, from t on, a CTA's warps apart: the first one's entries are in
-// S.tile, the next tile's are on their way while one runs.
+// A warp's next item of the step: the CTA's units, then its boundary tiles, are taken as warps
+// come free.  Dealt in turn, the warps with a unit also got the later tiles while those that
+// began with a tile were idle (us per step: 64 grids of 36x36x32 43.4 -> 41.9, 16 of 2.9 M
+// voxels 309 -> 290, 40 of 100x100x50 185 -> 183, one of 100x100x50 7.5 -> 7.3).
+__device__ __forceinline__ int march_next(MarchShared& S, int items) {
+  int i = 0;
+  if (items <= MARCH_T / 32) return items;
+  if ((threadIdx.x & 31u) == 0) i = atomicAdd(&S.next, 1);
+  return __shfl_sync(0xffffffffu, i, 0) + MARCH_T / 32;
+}
+
+// Boundary tiles (from tile k of the CTA on, then those the warp takes next; nu: the CTA's units).
 template <int MS, bool SUR>
-__device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R, const MarchShare& H, int t) {
+__device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R, const MarchShare& H, int nu, int k) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const MarchShared& S = *reinterpret_cast<const MarchShared*>(smem);
-  int4 e0 = S.tile[threadIdx.x][0], e1 = S.tile[threadIdx.x][1], n0, n1;
-  bool have = e0.x >= 0;
-  constexpr int W = MARCH_T / 32;
-  for (; t < H.t1; t += W) {
-    const bool next = march_entry(A, R, H, t + W, n0, n1);
+  MarchShared& S = *reinterpret_cast<MarchShared*>(smem);
+  const int items = nu + H.t1 - H.t0;
+  for (; k < items - nu; k = march_next(S, items) - nu) {
+    int4 e0, e1;
+    bool have;
+    if (k < MARCH_T / 32) {
+      const int i = k * 32 + (int)(threadIdx.x & 31u);
+      e0 = S.tile[i][0];
+      e1 = S.tile[i][1];
+      have = e0.x >= 0;
+    } else {
+      have = march_entry(A, R, H, H.t0 + k, e0, e1);
+    }
     if (have) mixed_voxel<MS, SUR>(S.desc, S.step, A.descs[R.r], A.ctl[R.r], A.mix, e0, e1);
     __syncwarp();
-    have = next;
-    e0 = n0;
-    e1 = n1;
   }
 }
 
@@ -748,7 +763,6 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
   MarchShared& S = *reinterpret_cast<MarchShared*>(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int team = blockIdx.x / A.size, rank = blockIdx.x - team * A.size;
-  constexpr int W = MARCH_T / 32;
   unsigned target = 0;                   // arrivals after which the team's next barrier opens
   if (A.inject && blockIdx.x == 0) {
     // test hook: one thread waits for an arrival that nothing makes; this CTA then leaves and
@@ -771,12 +785,11 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
       for (int i = tid; i < (int)(sizeof(VoxDesc) / 16); i += MARCH_T) dst[i] = __ldg(src + i);
     }
     const MarchShare H(R, A.what, rank, A.size);
-    // the warp's first item is a unit or, after the CTA's last unit, a tile
-    const int nu = H.u1 - H.u0, tile0 = H.t0 + ((warp - nu) % W + W) % W;
+    const int nu = H.u1 - H.u0, items = nu + H.t1 - H.t0;
     for (int c = tid; c <= R.nseg; c += MARCH_T) S.cut[c] = __ldg(A.cuts + R.cut0 + c);
     {
       int4 e0 = make_int4(-1, 0, 0, 0), e1 = e0;
-      if (!march_entry(A, R, H, tile0, e0, e1)) e0.x = -1;
+      if (!march_entry(A, R, H, H.t0 + warp, e0, e1)) e0.x = -1;
       S.tile[tid][0] = e0;
       S.tile[tid][1] = e1;
     }
@@ -785,6 +798,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
     double last_closed = 0.0, dt = 0.0, tabort = 0.0;
     long long total = 0;
     int stopped = 0;
+    if (tid == 0) S.next = 0;
     if (warp == 0) {
       const long long k = C.step;
       const unsigned cur = C.cur_mask[k & 1];
@@ -811,12 +825,13 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
     long long i = 0;
     for (; i < A.nsteps && S.step.go > 0; i++) {
       if (S.step.updated) {
-        for (int u = H.u0 + warp; u < H.u1; u += W) {
-          const int seg = u / R.ncol, col = u - seg * R.ncol;
+        int item = warp;
+        for (; item < nu; item = march_next(S, items)) {
+          const int u = H.u0 + item, seg = u / R.ncol, col = u - seg * R.ncol;
           march_dispatch<MS, FQ, SUR>(S, A.descs, R.r, col, S.cut[seg], S.cut[seg + 1]);
           __syncwarp();
         }
-        if (tile0 < H.t1) march_mixed<MS, SUR>(A, R, H, tile0);
+        if (item < items) march_mixed<MS, SUR>(A, R, H, nu, item - nu);
       }
       if (!(A.what & (MARCH_ADVANCE | MARCH_REPEAT))) break;
       __syncthreads();
@@ -850,7 +865,10 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
           S.step.cur ^= done;
           S.step.pre = pre; S.step.updated = updated; S.step.sub = dsi; S.step.flags = flags;
         }
-        if (lane == 0) S.step.go = !ok ? -1 : stopped ? 0 : 1;
+        if (lane == 0) {
+          S.next = 0;
+          S.step.go = !ok ? -1 : stopped ? 0 : 1;
+        }
         if (adv && lane < NS && (done >> lane & 1u)) {
           const float* o = S.step.uo[lane];
           S.step.uo[lane] = S.step.un[lane];
