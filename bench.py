@@ -43,6 +43,7 @@ sys.path.insert(0, ROOT)
 N_REAL = 256
 SHAPE = (100, 100, 50)
 BYTES_PER_VOXEL_STEP = 41     # 5 species x (4 B read + 4 B written) + 1 B domain id, FP32
+MARCH_STEPS_MAX = 4096     # steps of one launch of the step kernel (csp_runtime.cu)
 
 
 def dist_env():
@@ -139,12 +140,12 @@ def measured_peaks():
 
 
 def profiled_traffic(nvox):
-    """DRAM bytes per launch of the voxel kernel from the committed ncu summary, scaled
-    from the captured case to this launch by voxel count (traffic grows in proportion)."""
-    p = os.path.join(ROOT, "profiles", "k_voxels_staged_config3.md")
+    """DRAM bytes per step of the step kernel from the committed ncu summary, scaled from the
+    captured case by voxel count (traffic grows in proportion)."""
+    p = os.path.join(ROOT, "profiles", "k_march_config3.md")
     if not os.path.exists(p):
         return None
-    m = re.search(r"dram_bytes_per_voxel:\s*([0-9.]+)", open(p).read())
+    m = re.search(r"dram_bytes_per_voxel_step:\s*([0-9.]+)", open(p).read())
     return float(m.group(1)) * nvox if m else None
 
 
@@ -394,10 +395,10 @@ def main():
     nvox = sum(int(np.prod(s["voxels"].shape)) for s in specs)
     W, K = max(3, args.warmup), args.steps
 
-    # ---- tile shape of the staged voxel kernel: the autotuner's pick ----
+    # ---- teams and segments of the step kernel: the autotuner's pick ----
     tune = sim.autotune(repeats=3)
 
-    # ---- device-timed steps (graph replay, CUDA events on the handle stream) ----
+    # ---- device-timed steps (CUDA events on the handle stream) ----
     sim.advance(W)
     D.barrier()
     clocks = Clocks(local)
@@ -413,10 +414,12 @@ def main():
     # total of every species) of every rank on every rank: one all_gather
     gathered = int(len(ens.statistics()["index"]))
 
-    # ---- roofline of the dominant kernel: per-launch CUDA events ----
+    # ---- roofline of the dominant kernel.  The step kernel takes every step of a call in one
+    # launch, so its time per step is the timed region's; the direct kernel launches per step ----
+    direct = tune["chosen"]["segment"] < 0
     nprof = min(K, 100)
     vms, bms = sim.profile(nprof)
-    t_launch = vms / nprof / 1e3
+    t_launch = vms / nprof / 1e3 if direct else ms_max / K / 1e3
     achieved = BYTES_PER_VOXEL_STEP * nvox / t_launch / 1e9
     peak, peak_kind = measured_peaks()
     traffic = profiled_traffic(nvox)
@@ -481,9 +484,9 @@ def main():
                    "sample": f"{steps} steps of one 100x100x50 realisation of the workload "
                              f"({dt:.1f} s), FP64 port of the reference"}
 
-    # per step: voxel kernel, density-row flux kernel, channel-row gating/flux kernel, step
-    # epilogue (the workload has both kinds of flux rows), in the device-timed region
-    kernels = 4 * K
+    # in the device-timed region: one launch of the step kernel per MARCH_STEPS_MAX steps; the
+    # direct kernel with its density-row, channel-row and epilogue kernels on every step
+    kernels = 4 * K if direct else -(-K // MARCH_STEPS_MAX)
     if rank == 0:
         line = {
             "metric": "ensemble voxel-steps/s", "value": value, "unit": "voxel-steps/s",
@@ -498,7 +501,7 @@ def main():
                                 "autotuned_from": len(tune["candidates"])}},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "k_voxels_direct" if tune["chosen"]["segment"] < 0 else "k_voxels_staged",
+                         "kernel": "k_voxels_direct" if direct else "k_march",
                          "launch_ms": t_launch * 1e3,
                          "bytes_per_voxel": BYTES_PER_VOXEL_STEP, "peak_source": peak_kind,
                          "boundary_kernel_ms": bms / nprof},
