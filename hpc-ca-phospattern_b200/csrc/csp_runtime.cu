@@ -201,14 +201,13 @@ struct csp_handle {
   int* d_stepflags = nullptr;
   size_t stepflags_elems = 0;
   StepRec* d_rec = nullptr;          // per realisation: what its running step does
-  int max_plane_vox = 0;
   long long max_vox = 0;
   long long max_field = 0;           // max n0*P (padded planes)
   int kernel = 0;                 // 0 march, 1 direct
-  int inject_wait = 0;            // csp_test_wait_timeout armed (direct launches, no graph)
-  // csp_set_phase_timing: the first steps of every advance call run as direct launches
-  // with events between the step's kernels; the sample's per-phase device time, scaled to
-  // the steps of the call, is added to phase_ms at the call's wait
+  int inject_wait = 0;            // csp_test_wait_timeout armed
+  // csp_set_phase_timing: the first steps of every advance call run as one launch per phase
+  // with events between them; the call's device time, in the phases' proportions in that
+  // sample, is added to phase_ms at the call's wait
   int phase_timing = 0;
   cudaEvent_t phase_ev[PHASE_SAMPLE * (CSP_NUM_PHASES + 1)] = {};
   int phase_sampled = 0;
@@ -557,7 +556,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     hr0.field_elems = (size_t)n0 * P;
     field_total += hr0.field_elems * 2 * models[r].num_species;
     dom_total += hr0.field_elems;
-    h->max_plane_vox = std::max(h->max_plane_vox, plane);
     h->max_vox = std::max(h->max_vox, (long long)n0 * plane);
     h->max_field = std::max(h->max_field, (long long)n0 * P);
   }
