@@ -845,6 +845,8 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
         if (adv) count.next(lane, pre, updated, dsi, flags);
         bool ok = true;
         if (A.size > 1 && lane == 0) ok = march_wait(A.arrived + team * 32, target, A.err);
+        // every lane has read the step's masks (votes and reductions are no memory barriers)
+        __syncwarp();
         // the step is taken: every CTA of the team follows the same rules (see k_epilogue)
         if (adv && lane == 0) {
           if (tabort != 0) {
