@@ -137,18 +137,40 @@ __device__ __forceinline__ unsigned rx_classify4(const VoxDesc& D, int d, F2 ca0
          ((neg1 >> 63) ? nt : e) << 24;
 }
 
-// General reactions of a group (models whose buffers do not all bind species 0): local
-// arrays, so that the fast path's registers stay registers.
+// General reactions (react_general) of a group in domain d, the four voxels of a species
+// together (models whose buffers do not all bind species 0): local arrays indexed by the
+// buffers' species, so that the fast path's registers stay registers.  24 grids of 100x100x50
+// with such a buffer: 616 us per step with a voxel at a time and the masks at run time, now 249.
 template <int MS>
-__device__ __noinline__ void react_group(const RealDesc* Dp, const int* dj, const float* val, float* out, unsigned pre,
+__device__ __noinline__ void react_group(const RealDesc& D, int d, const float4* val, float4* out, unsigned pre,
                                          unsigned fq) {
-  for (int j = 0; j < 4; j++) {
-    float vj[MS], oj[MS];
-    for (int s = 0; s < MS; s++) { vj[s] = val[s * 4 + j]; oj[s] = out[s * 4 + j]; }
-    react_general<MS>(*Dp, dj[j], vj, oj, pre, fq);
-    for (int s = 0; s < MS; s++) out[s * 4 + j] = oj[s];
+  for (int bi = 0; bi < D.nbuf; bi++) {
+    const int t = bi * D.nd + d;
+    const int s0 = D.bsp0[t], s1 = D.bsp1[t];
+    const float nkon = -D.kon_dt[t], nkoff = -D.koff_dt[t], a = D.a_dt[t], j0 = D.j0_dt[t], base = D.fbase[d][s1];
+    const float4 b0 = val[s0], b1 = val[s1];
+    auto dj = [&](float x0, float x1) { return buffer_dj(nkon, nkoff, a, j0, x0, x1, __fadd_rn(base, x1)); };
+    const float4 J = make_float4(dj(b0.x, b1.x), dj(b0.y, b1.y), dj(b0.z, b1.z), dj(b0.w, b1.w));
+    float4 r = (pre >> s0 & 1u) ? out[s0] : b0;
+    if ((fq & ~pre) >> s0 & 1u) r = J;
+    else r = make_float4(__fadd_rn(r.x, J.x), __fadd_rn(r.y, J.y), __fadd_rn(r.z, J.z), __fadd_rn(r.w, J.w));
+    out[s0] = r;
+    r = (pre >> s1 & 1u) ? out[s1] : b1;
+    out[s1] = make_float4(__fsub_rn(r.x, J.x), __fsub_rn(r.y, J.y), __fsub_rn(r.z, J.z), __fsub_rn(r.w, J.w));
   }
 }
+
+// What a kernel's bodies know at compile time: every mask of the step (MARCH_KNOWN, for batches
+// of the reference model's shape, see march_masks_known), or the species that diffuse
+// (MARCH_MASKS, any other model of up to five species; masks it has no body for run on one with
+// run-time masks), or nothing (MARCH_RUNTIME, up to eight species).  us per step of 24 grids of
+// 100x100x50 with run-time masks and on MARCH_MASKS: Dirichlet faces 256 -> 126, two
+// fixed-point species 261 -> 116, three species 161 -> 90; the reference model on MARCH_KNOWN
+// 104.  The bodies are kernels of their own: in one kernel the run-time body's registers and
+// spills (1,008 bytes of loads) became everyone's.
+enum : int { MARCH_KNOWN = 0, MARCH_MASKS = 1, MARCH_RUNTIME = 2 };
+// A body's reactions: none, fast (STEP_REACT_FAST), general, or as the step says.
+enum : int { REACT_NONE = 0, REACT_FAST = 1, REACT_GENERAL = 2, REACT_ANY = 3 };
 
 // Whether every step of a realisation runs on the variants with compile-time masks (see
 // march_dispatch): the reference model's shape.
@@ -167,11 +189,11 @@ struct GroupPlace {
   int dym, dyp, dzm, dzp;
 };
 
-// One unit.  PRE >= 0: the step's masks are known at compile time -- the species of PRE
-// diffuse, with REACT every species is updated by the fast reactions, without it only those of
-// PRE are; FQ are exactly the fixed-point species and nothing is fixed -- so the loop has no
-// mask test and only its own species' registers.  PRE < 0: masks at run time, any model.
-template <int MS, unsigned FQ, bool SUR, int PRE, bool REACT>
+// One unit.  PRE >= 0: the species of PRE diffuse and the reactions are REACT, known at compile
+// time, so the loop has no test of them and three planes of registers for the species of PRE
+// alone.  EXACT: so is the rest -- with reactions every species is updated, FQ are exactly the
+// fixed-point species and nothing is fixed.  PRE < 0: all at run time, any model.
+template <int MS, unsigned FQ, bool SUR, int PRE, int REACT, bool EXACT>
 __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, int r_, int col, int x0, int x1) {
   constexpr bool DYN = PRE < 0;
   // from the shared array itself, not by argument: the compiler then knows the address space
@@ -180,10 +202,14 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
   const VoxDesc& D = S.desc;
   const MarchStep& U = S.step;
   const unsigned pre = DYN ? U.pre : (unsigned)PRE;
-  const unsigned lmask = DYN ? U.updated : REACT ? (1u << MS) - 1u : (unsigned)PRE;
-  const bool react = DYN ? (U.flags & STEP_REACT) != 0u : REACT;
-  const bool react_fast = DYN ? (U.flags & STEP_REACT_FAST) != 0u : REACT;
-  const unsigned fq = DYN ? FQ & D.fixq & lmask : FQ & lmask;       // fixed-point species
+  const unsigned lmask = DYN                   ? U.updated
+                         : REACT == REACT_NONE ? (unsigned)PRE
+                         : EXACT               ? (1u << MS) - 1u
+                                               : U.updated | (unsigned)PRE;
+  const bool react = DYN ? (U.flags & STEP_REACT) != 0u : REACT != REACT_NONE;
+  const bool react_fast = DYN ? (U.flags & STEP_REACT_FAST) != 0u : REACT == REACT_FAST;
+  // fixed-point species (never diffusing ones)
+  const unsigned fq = EXACT ? FQ & lmask : FQ & D.fixq & lmask & ~pre;
   const int nz = D.nz;
   const int p0 = col * MARCH_COL + 4 * (int)(threadIdx.x & 31u);
   const unsigned lanes = __ballot_sync(0xffffffffu, p0 < D.plane);
@@ -256,7 +282,7 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
       auto dn = [&](int kk) -> int { return (int)(pt.code >> (3 + 3 * kk)) & 7; };
       const bool allyx = !REG || ((pt.code >> 9) & 0xfffu) == (unsigned)d0 * 0x249u;
       const bool uni0 = allyx && dn(0) == d0, uni3 = allyx && dn(1) == d0;
-      const unsigned fixed = DYN ? D.fixed_mask[d0] : 0u;
+      const unsigned fixed = EXACT ? 0u : D.fixed_mask[d0];
       // value and diffusion of species s: v = the stored values (fixed point: converted),
       // o2 = diffused value (fixed point: the increment so far, 0)
       auto load_diffuse = [&](int s, float4& v, F2 (&o2)[2]) {
@@ -319,7 +345,7 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
         float4 r;
         f2_split(o2[0], r.x, r.y);
         f2_split(o2[1], r.z, r.w);
-        if (DYN && (fixed >> s & 1u)) {
+        if (!EXACT && (fixed >> s & 1u)) {
           float iv = D.dinit[d0][s];
           if (fq >> s & 1u) iv = q_set(iv, D.qinv[d0][s]);
           r = make_float4(iv, iv, iv, iv);
@@ -327,7 +353,7 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
           const float qi = D.qinv[d0][s];
           r = make_float4(q_add(st.x, r.x, qi), q_add(st.y, r.y, qi), q_add(st.z, r.z, qi), q_add(st.w, r.w, qi));
         }
-        if (DYN && s == 0 && D.dirichlet) {
+        if (!EXACT && s == 0 && D.dirichlet) {
           const bool face = x == 0 || x + 1 == nx || G.dym == 0 || G.dyp == 0;
           const float iv = D.dinit[d0][0];
           if (face || G.z0 == 0) r.x = iv;
@@ -336,8 +362,9 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
           if (face || G.lastj == 2) r.z = iv;
           if (face || G.lastj == 3) r.w = iv;
         }
-        if (REG && s == 0 && pt.flux != PAT_NONE) {
-          // SERCA across one face (boundaryfluxes.c:60-84), from the old Ca of its two sides
+        if (REG && s == 0 && pt.flux != PAT_NONE && (!DYN || (pre & 1u))) {
+          // SERCA across one face (boundaryfluxes.c:60-84) on the steps on which Ca diffuses, from
+          // the old Ca of its two sides
           const int kk = (int)(pt.flux & 7u);
           const float4 q = kk == 2 ? ym[0] : kk == 3 ? yp[0] : kk == 4 ? prv[0] : nxt[0];
           const double bs = D.base0[d0], bo = D.base0[dn(kk)], scale = D.serca;
@@ -351,22 +378,19 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
         }
         *reinterpret_cast<float4*>(field(U.un[s]) + off) = r;
       };
-      if (DYN && react && !react_fast) {
-        float tv[MS * 4], to[MS * 4];
-        const int dj[4] = {d0, d0, d0, d0};
+      if (react && !react_fast) {
+        float4 tv[MS], to[MS];
 #pragma unroll
         for (int s = 0; s < MS; s++) {
-          float4 v;
           F2 o2[2];
-          load_diffuse(s, v, o2);
-          tv[s * 4] = v.x; tv[s * 4 + 1] = v.y; tv[s * 4 + 2] = v.z; tv[s * 4 + 3] = v.w;
-          f2_split(o2[0], to[s * 4], to[s * 4 + 1]);
-          f2_split(o2[1], to[s * 4 + 2], to[s * 4 + 3]);
+          load_diffuse(s, tv[s], o2);
+          f2_split(o2[0], to[s].x, to[s].y);
+          f2_split(o2[1], to[s].z, to[s].w);
         }
-        react_group<MS>(descs + r_, dj, tv, to, pre, fq);
+        react_group<MS>(descs[r_], d0, tv, to, pre, fq);
 #pragma unroll
         for (int s = 0; s < MS; s++) {
-          const F2 o2[2] = {f2(to[s * 4], to[s * 4 + 1]), f2(to[s * 4 + 2], to[s * 4 + 3])};
+          const F2 o2[2] = {f2(to[s].x, to[s].y), f2(to[s].z, to[s].w)};
           if (lmask >> s & 1u) store(s, cur[s], o2);
           fetch_next(s);
         }
@@ -420,9 +444,8 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
         }
       }
     };
-    // (a realisation of the run-time masks has no regular groups)
     const bool mine = code != CODE_MIXED;
-    if (DYN || __all_sync(lanes, code < (unsigned)ND || code == CODE_MIXED)) {
+    if (__all_sync(lanes, code < (unsigned)ND || code == CODE_MIXED)) {
       if (mine) group(std::false_type{});
     } else {
       if (mine) group(std::true_type{});
@@ -442,33 +465,28 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
   }
 }
 
-// The variants of march_unit by the step's masks: in a five-species model whose species 4 is
-// the fixed-point one, Ca and any of the species 1-3 diffusing, with and without the
-// reactions; everything else at run time.
-template <int MS, unsigned FQ, bool SUR>
+// The body of a step: Ca and any of the species 1-3 diffusing; everything else at run time.
+template <int MS, unsigned FQ, bool SUR, int BODY>
 __device__ __forceinline__ void march_dispatch(const MarchShared& S, const RealDesc* __restrict__ descs, int r, int col,
                                                int x0, int x1) {
-  if constexpr (MS == 5 && FQ == 1u << 4) {
-    const VoxDesc& D = S.desc;
-    const MarchStep& U = S.step;
-    const bool plain = D.fixq == FQ && !D.any_fixed && !D.dirichlet;
-    const bool rf = (U.flags & STEP_REACT_FAST) && U.updated == 0x1Fu;
-    const bool nr = !(U.flags & STEP_REACT) && U.updated == U.pre;
-    if (plain && (rf || nr)) {
-#define CSP_UNIT(p)                                                                           \
-  case p:                                                                                     \
-    if (rf) march_unit<MS, FQ, SUR, p, true>(descs, r, col, x0, x1);                          \
-    else march_unit<MS, FQ, SUR, p, false>(descs, r, col, x0, x1);                            \
+  const MarchStep& U = S.step;
+  if constexpr (BODY != MARCH_RUNTIME) {
+    constexpr bool EXACT = BODY == MARCH_KNOWN;
+    const bool none = !(U.flags & STEP_REACT), fast = U.flags & STEP_REACT_FAST;
+#define CSP_UNIT(p)                                                                                     \
+  case p:                                                                                               \
+    if (fast) march_unit<MS, FQ, SUR, p, REACT_FAST, EXACT>(descs, r, col, x0, x1);                     \
+    else if (EXACT || none) march_unit<MS, FQ, SUR, p, REACT_NONE, EXACT>(descs, r, col, x0, x1);       \
+    else if constexpr (!EXACT) march_unit<MS, FQ, SUR, p, REACT_GENERAL, EXACT>(descs, r, col, x0, x1); \
     return;
-      switch (U.pre) {
-        CSP_UNIT(0x1) CSP_UNIT(0x3) CSP_UNIT(0x5) CSP_UNIT(0x7)
-        CSP_UNIT(0x9) CSP_UNIT(0xB) CSP_UNIT(0xD) CSP_UNIT(0xF)
-        default: break;
-      }
-#undef CSP_UNIT
+    switch (U.pre) {
+      CSP_UNIT(0x1) CSP_UNIT(0x3) CSP_UNIT(0x5) CSP_UNIT(0x7)
+      CSP_UNIT(0x9) CSP_UNIT(0xB) CSP_UNIT(0xD) CSP_UNIT(0xF)
+      default: break;
     }
+#undef CSP_UNIT
   }
-  march_unit<MS, FQ, SUR, -1, false>(descs, r, col, x0, x1);
+  if constexpr (BODY != MARCH_KNOWN) march_unit<MS, FQ, SUR, -1, REACT_ANY, false>(descs, r, col, x0, x1);
 }
 
 // The step counters of a realisation, on the lanes of a warp: lane l < 30 holds the step index
@@ -757,7 +775,7 @@ __device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R,
   }
 }
 
-template <int MS, unsigned FQ, bool SUR>
+template <int MS, unsigned FQ, bool SUR, int BODY>
 __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ MarchArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   MarchShared& S = *reinterpret_cast<MarchShared*>(smem);
@@ -828,7 +846,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
         int item = warp;
         for (; item < nu; item = march_next(S, items)) {
           const int u = H.u0 + item, seg = u / R.ncol, col = u - seg * R.ncol;
-          march_dispatch<MS, FQ, SUR>(S, A.descs, R.r, col, S.cut[seg], S.cut[seg + 1]);
+          march_dispatch<MS, FQ, SUR, BODY>(S, A.descs, R.r, col, S.cut[seg], S.cut[seg + 1]);
           __syncwarp();
         }
         if (item < items) march_mixed<MS, SUR>(A, R, H, nu, item - nu);
@@ -897,12 +915,12 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
 
 using MarchKernel = void (*)(const MarchArgs);
 
-// The kernel variants built: five species with fixed point only for species 4 (the reference
-// model: TRPN); five species with any of species 1-4 fixed; eight species with any of 1-7.
-inline MarchKernel march_kernel(int ms, unsigned fixq, bool sur) {
-  if (ms == 5 && (fixq & ~(1u << 4)) == 0) return sur ? k_march<5, 1u << 4, true> : k_march<5, 1u << 4, false>;
-  if (ms == 5) return sur ? k_march<5, 0x1Eu, true> : k_march<5, 0x1Eu, false>;
-  return sur ? k_march<8, 0xFEu, true> : k_march<8, 0xFEu, false>;
+// The kernel of a batch: models of at most ms species, all of the reference model's shape
+// (known: fixed point for species 4 alone) or not.
+inline MarchKernel march_kernel(int ms, bool known, bool sur) {
+  if (known) return sur ? k_march<5, 1u << 4, true, MARCH_KNOWN> : k_march<5, 1u << 4, false, MARCH_KNOWN>;
+  if (ms == 5) return sur ? k_march<5, 0x1Eu, true, MARCH_MASKS> : k_march<5, 0x1Eu, false, MARCH_MASKS>;
+  return sur ? k_march<8, 0xFEu, true, MARCH_RUNTIME> : k_march<8, 0xFEu, false, MARCH_RUNTIME>;
 }
 
 // Teams and units of a launch over realisations [r0, r1).
@@ -910,6 +928,7 @@ struct MarchPlan {
   int r0 = 0, r1 = 0;
   int teams = 0, size = 0;
   int nseg = 0;                      // segments of the first realisation
+  bool known = false;                // march_kernel
   MarchReal* d_real = nullptr;
   int* d_first = nullptr;
   int* d_cuts = nullptr;

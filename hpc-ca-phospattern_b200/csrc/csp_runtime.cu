@@ -217,7 +217,6 @@ struct csp_handle {
   // launches of the step kernel: the variant, its resident CTAs, and the teams and units for
   // every range of realisations asked for so far
   int ms = 5;
-  unsigned fixq = 0;
   int ctas = 0;
   size_t l2 = 0;
   std::vector<MarchPlan> plans;
@@ -953,13 +952,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   for (const FluxPair& p : pairs)
     if (p.kind == FLUX_SERCA) serca[p.r] = p.param;
   {
-    // realisations that may have regular groups: the step kernel's variants with run-time
-    // masks (another realisation's model may select them for the batch) do not know them
-    bool batch = true;
-    for (int r = 0; r < n; r++)
-      batch = batch && h->real[r].desc.ns <= 5 && (h->real[r].desc.fixq & ~(1u << 4)) == 0;
-    std::vector<char> regular(n, 0);
-    for (int r = 0; r < n; r++) regular[r] = batch && march_masks_known(h->real[r].desc);
     std::vector<int> order(rows.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
@@ -975,7 +967,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       const int r = group[0].r;
       const RealDesc& D = h->real[r].desc;
       GroupPattern g;
-      if (ng == 4 && regular[r] && !chan_of[0] && !chan_of[1] && !chan_of[2] && !chan_of[3] &&
+      if (ng == 4 && !chan_of[0] && !chan_of[1] && !chan_of[2] && !chan_of[3] &&
           regular_group(D, group, g)) {
         std::vector<GroupPattern>& P = pats[r];
         size_t i = 0;
@@ -1160,19 +1152,17 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   }
   {
     int ns = 0, dev = 0, sms = 0, per_sm = 0, l2 = 0;
-    for (const RealDesc& D : descs) {
-      ns = std::max(ns, D.ns);
-      h->fixq |= D.fixq;
-    }
+    for (const RealDesc& D : descs) ns = std::max(ns, D.ns);
     h->ms = ns <= 5 ? 5 : 8;
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-    for (int sur = 0; sur < 2 && e == cudaSuccess; sur++) {
+    for (int v = 0; v < 4 && e == cudaSuccess; v++) {
+      const bool sur = v & 1, known = v >> 1;
       int k = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, march_kernel(h->ms, h->fixq, sur != 0), MARCH_T,
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, march_kernel(h->ms, known, sur), MARCH_T,
                                                         sizeof(MarchShared));
-      per_sm = sur == 0 ? k : std::min(per_sm, k);
+      per_sm = v == 0 ? k : std::min(per_sm, k);
     }
     if (e != cudaSuccess || per_sm < 1) {
       csp_destroy(h);
@@ -1252,6 +1242,8 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
   pl.r1 = r1;
   pl.teams = best;
   pl.size = size_of(best);
+  pl.known = true;
+  for (int r = r0; r < r1; r++) pl.known = pl.known && march_masks_known(desc(r));
   std::vector<std::vector<int>> team(best);
   deal(best, &team);
   std::vector<MarchReal> real;
@@ -1342,7 +1334,7 @@ static cudaError_t launch_march(csp_handle* h, const MarchPlan& pl, long long ns
   a.inject = h->inject_wait;
   // the classification belongs to a reaction step, which is launched alone (launch_steps); the
   // stretches between take the kernel without it
-  MarchKernel k = march_kernel(h->ms, h->fixq, h->surrogate != 0 && !(what & (MARCH_ADVANCE | MARCH_REPEAT)));
+  MarchKernel k = march_kernel(h->ms, pl.known, h->surrogate != 0 && !(what & (MARCH_ADVANCE | MARCH_REPEAT)));
   const unsigned grid = (unsigned)(pl.teams * pl.size);
   if (pl.size == 1 || !(what & (MARCH_ADVANCE | MARCH_REPEAT))) {
     k<<<grid, MARCH_T, sizeof(MarchShared), h->stream>>>(a);
