@@ -214,6 +214,18 @@ struct alignas(16) MixVoxel {
   MixItem item;
 };
 
+// An irregular group (CODE_MIXED) as one entry: its voxels have no channel and no flux but SERCA
+// from neighbours.  code: as MixVoxel::code, by voxel (0 outside the box).  order: the
+// six faces (directions 0-5, 3 bits each) as a voxel's pairs come, from bit 18 the number of
+// voxels.  flux: a byte per voxel, bit i a flux across the i-th of them, MIXG_TO on the
+// receiving side, MIXG_APPLY.
+enum : unsigned { MIXG_TO = 0x40u, MIXG_APPLY = 0x80u };
+struct alignas(16) MixGroup {
+  int v;                             // field index of the first voxel
+  unsigned flux, order, pad;
+  unsigned code[4];
+};
+
 struct FluxEntry {
   int pair;
   float sign;             // +1 "to" side, -1 "from" side (inner boundaries)

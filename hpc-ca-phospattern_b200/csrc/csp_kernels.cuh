@@ -482,11 +482,12 @@ __global__ void __launch_bounds__(256, 8) k_density_rows(const RealDesc* __restr
   if (any && write) unew[a.x] = (float)((double)nv + acc);
 }
 
-// The boundary work: voxels with a channel pair (the longest chains), the others, and what
-// they read.
+// The boundary work: voxels with a channel pair (the longest chains), the others, irregular
+// groups, and what they read.
 struct MixArgs {
   const MixVoxel* chan;
   const MixVoxel* vox;
+  const MixGroup* grp;
   const MixItem* items;
   const FluxPair* pairs;
   const FluxParams* params;

@@ -22,7 +22,7 @@
 // groups along domain sheets: coefficients per direction, SERCA flux from the values at hand).
 // A warp whose groups are all uniform takes the leaner of two forms of the loop body.  The
 // voxels of irregular groups and those with channels are the boundary work (mixed_voxel), in
-// tiles of 32.
+// tiles of 32; where there are many, irregular groups are, in tiles of 32 groups (mixed_group).
 //
 // The barrier's wait is bounded in time (WAIT_NS).  A CTA that gives up sets ERR_TIMEOUT in the
 // device error word, which the other waits see too, and every CTA leaves the launch; the fields
@@ -59,8 +59,16 @@ struct MarchReal {
   int r;
   int ncol, nseg;                    // columns, x segments
   int cut0;                          // segment s: planes [cuts[cut0 + s], cuts[cut0 + s + 1])
-  int chan0, nchan, vox0, nvox;
+  int chan0, nchan, vox0, nvox, grp0, ngrp;
 };
+// Irregular voxels of a batch from which they are taken as groups (MixGroup): with fewer, a
+// voxel per lane fills the GPU and its chain is shorter (us per step of random 2^3 blocks of
+// domains, by voxel and by group: one grid of 40x40x36 6.8 and 12.1, one of 100x100x50 34.7 and
+// 23.4, 24 of those 845 and 423; 8^3 blocks, 24 grids: 344 and 247).
+constexpr size_t MIX_GROUPS_MIN = 262144;
+// Share of uniform groups below which the units of such a realisation would read its planes for
+// next to nothing: all of its groups are boundary work (24 grids of 2^3 blocks: 423 -> 374 us).
+constexpr double MIX_DENSE = 1.0 / 16;
 constexpr int MARCH_CUTS = 1024;          // segments of a realisation (at most), plus one
 
 struct MarchArgs {
@@ -710,18 +718,130 @@ __device__ __forceinline__ void mixed_voxel(const VoxDesc& D, const MarchStep& U
   if (SUR && D.sur && react_fast) D.rx_class[v] = (unsigned char)cls;
 }
 
+__device__ __forceinline__ float part(const float4& q, int j) { return j == 0 ? q.x : j == 1 ? q.y : j == 2 ? q.z : q.w; }
+
+// The four voxels of an irregular group (MixGroup) as mixed_voxel takes one: the same
+// arithmetic per voxel, from values read 128 bits at a time.  A lane's chain is longer than a
+// voxel's, so only batches with many irregular voxels have such entries (MIX_GROUPS_MIN).
+// Bound by issue: 2,000 instructions per tile, half of the slots used by the 16 warps that 128
+// registers allow, 0.06 of the DRAM bandwidth.
+template <int MS, unsigned FQ, bool SUR>
+__device__ __forceinline__ void mixed_group(const VoxDesc& D, const MarchStep& U, const RealDesc& R, const int4& e0,
+                                            const int4& e1) {
+  const int v = e0.x;
+  const unsigned flux = (unsigned)e0.y, order = (unsigned)e0.z;
+  const unsigned code[4] = {(unsigned)e1.x, (unsigned)e1.y, (unsigned)e1.z, (unsigned)e1.w};
+  const int nv = (int)(order >> 18);
+  const unsigned pre = U.pre, updated = U.updated;
+  const unsigned fq = FQ & D.fixq & updated;           // fixed-point species: out[] holds the increment
+  const bool react = U.flags & STEP_REACT_FAST;   // (realisations with other reactions have no such entries)
+  const int dym = (code[0] >> 23 & 1u) ? -D.nz : 0, dyp = (code[0] >> 24 & 1u) ? D.nz : 0;
+  const int dxm = (code[0] >> 25 & 1u) ? -D.P : 0, dxp = (code[0] >> 26 & 1u) ? D.P : 0;
+  const int dzm = (code[0] >> 21 & 1u) ? -1 : 0, dzp = (code[3] >> 22 & 1u) ? 4 : 3;
+  float4 raw[MS];
+#pragma unroll
+  for (int s = 0; s < MS; s++)
+    raw[s] = (updated >> s & 1u) ? *reinterpret_cast<const float4*>(field(U.uo[s]) + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float out[MS][4];
+#pragma unroll
+  for (int s = 0; s < MS; s++) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) out[s][j] = (fq >> s & 1u) ? 0.f : part(raw[s], j);
+    if (!(pre >> s & 1u)) continue;
+    const float* u = field(U.uo[s]) + v;
+    const float4 ym = *reinterpret_cast<const float4*>(u + dym), yp = *reinterpret_cast<const float4*>(u + dyp);
+    const float4 xm = *reinterpret_cast<const float4*>(u + dxm), xp = *reinterpret_cast<const float4*>(u + dxp);
+    const float zm = u[dzm], zp = u[dzp];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const unsigned c = code[j];
+      const int d = (int)(c & 7u);
+      const float self = part(raw[s], j);
+      const float un[6] = {j == 0 ? zm : part(raw[s], j > 0 ? j - 1 : 0),
+                           !(c >> 22 & 1u) ? self : j == 3 ? zp : part(raw[s], j < 3 ? j + 1 : 3),
+                           part(ym, j), part(yp, j), part(xm, j), part(xp, j)};
+      int dn[6];
+#pragma unroll
+      for (int q = 0; q < 6; q++) dn[q] = (int)(c >> (3 + 3 * q)) & 7;
+      const bool uniform = (c >> 3 & 0x3ffffu) == (unsigned)d * 0x9249u;
+      const float* co = D.coef[s] + d * ND;
+      const float across = diffuse_general(co, dn, self, un), inside = diffuse_uniform(co[d], self, un);
+      out[s][j] = uniform ? inside : across;         // (both, no branch: the lanes differ)
+    }
+  }
+  // SERCA (boundaryfluxes.c:60-84) across the faces of all four voxels in one loop, so that a
+  // warp takes as many turns as its lane with the most (random 2^3 blocks of domains: 8, where a
+  // loop per voxel and face takes 24: 527 -> 471 us); the partner's value once more, from L1.
+  // (Two fluxes per turn 512 us, the warp's fluxes dealt to its lanes the same.)
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  if (pre & 1u) {
+    const float* u = field(U.uo[0]) + v;
+    for (unsigned m = flux & 0x3f3f3f3fu; m; m &= m - 1u) {
+      const int b = __ffs(m) - 1, j = b >> 3, k = (int)(order >> (3 * (b & 7))) & 7;
+      const unsigned c = j == 0 ? code[0] : j == 1 ? code[1] : j == 2 ? code[2] : code[3];
+      const int off = k == 0 ? -1 : k == 1 ? 1 : k == 2 ? dym : k == 3 ? dyp : k == 4 ? dxm : dxp;
+      const double us = (double)u[j] + D.base0[c & 7u], uo = (double)u[j + off] + D.base0[(c >> (3 + 3 * k)) & 7u];
+      const bool to = flux >> (8 * j) & MIXG_TO;
+      const double J = serca_flux_fast(to ? uo : us, to ? us : uo, D.serca);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (q == j) acc[q] += to ? J : -J;
+    }
+  }
+  unsigned cls = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const unsigned c = code[j];
+    const int d = (int)(c & 7u);
+    float val[MS];
+#pragma unroll
+    for (int s = 0; s < MS; s++) val[s] = (fq >> s & 1u) ? q_value(part(raw[s], j), D.qunit[d][s]) : part(raw[s], j);
+    if (react) {
+      const float dca = val[0], ca = __fadd_rn(D.fbase0[d], dca);
+      if (SUR && D.sur && j < nv) cls |= rx_classify<MS>(R, d, ca, val) << (8 * j);
+      const unsigned rm = D.rmask[d];
+#pragma unroll
+      for (int s = 1; s < MS; s++) {
+        const float4 ka = *reinterpret_cast<const float4*>(&D.rk2[d][s][0]);   // -kon, -kon, -koff, -koff
+        const float4 kb = *reinterpret_cast<const float4*>(&D.rk2[d][s][2]);   // a, a, j0, j0
+        const float dJ = buffer_dj(ka.x, ka.z, kb.x, kb.z, val[s], dca, ca);
+        const bool on = rm >> s & 1u;              // (no branch: the lanes' domains differ)
+        out[s][j] = on ? __fadd_rn(out[s][j], dJ) : out[s][j];
+        out[0][j] = on ? __fsub_rn(out[0][j], dJ) : out[0][j];
+      }
+    }
+    const unsigned fm = D.any_fixed ? D.fixed_mask[d] : 0u;
+#pragma unroll
+    for (int s = 0; s < MS; s++) {
+      float& o = out[s][j];
+      if (fm >> s & 1u) o = D.dinit[d][s];
+      if (fq >> s & 1u) o = (fm >> s & 1u) ? q_set(o, D.qinv[d][s]) : q_add(part(raw[s], j), o, D.qinv[d][s]);
+    }
+    if (D.dirichlet && (c >> 21 & 63u) != 63u) out[0][j] = D.dinit[d][0];
+    const unsigned f = flux >> (8 * j);
+    if ((pre & 1u) && (f & 63u) && (f & MIXG_APPLY)) out[0][j] = (float)((double)out[0][j] + acc[j]);
+  }
+#pragma unroll
+  for (int s = 0; s < MS; s++)
+    if (updated >> s & 1u)
+      *reinterpret_cast<float4*>(field(U.un[s]) + v) = make_float4(out[s][0], out[s][1], out[s][2], out[s][3]);
+  if (SUR && D.sur && react) *reinterpret_cast<unsigned*>(D.rx_class + v) = cls;
+}
+
 // A CTA's share of a realisation's step: units [u0, u1) and boundary tiles [t0, t1) (of 32
-// voxels, those with channels first), taken by its warps as they come free, units first.  Contiguous
+// voxels, those with channels first, then of 32 groups), taken by its warps as they come free, units first.  Contiguous
 // units share their columns' rows in L1; the tiles, whose lanes touch a line each, are spread
 // evenly over the CTAs (16 of them on one SM took twice the time of one).
 struct MarchShare {
-  int u0, u1, t0, t1, tc, nc, nv;
+  int u0, u1, t0, t1, tc, tv, nc, nv, ng;
   __device__ __forceinline__ MarchShare(const MarchReal& R, unsigned what, int rank, int size) {
     const long long units = (what & MARCH_UNITS) ? R.ncol * (long long)R.nseg : 0;
     nc = (what & MARCH_CHANNELS) ? R.nchan : 0;
     nv = (what & MARCH_VOXELS) ? R.nvox : 0;
+    ng = (what & MARCH_VOXELS) ? R.ngrp : 0;
     tc = (nc + 31) / 32;
-    const long long tiles = tc + (nv + 31) / 32;
+    tv = (nv + 31) / 32;
+    const long long tiles = tc + tv + (ng + 31) / 32;
     u0 = (int)(units * rank / size);
     u1 = (int)(units * (rank + 1) / size);
     // the CTAs with one unit less get the odd tiles
@@ -730,13 +850,17 @@ struct MarchShare {
   }
 };
 
-// The lane's entry of tile t; false: none.
+// The lane's entry (MixVoxel or MixGroup) of tile t; false: none.
 __device__ __forceinline__ bool march_entry(const MarchArgs& A, const MarchReal& R, const MarchShare& H, int t, int4& e0,
                                             int4& e1) {
-  const bool c = t < H.tc;
-  const int i = (c ? t : t - H.tc) * 32 + (int)(threadIdx.x & 31u);
-  if (t >= H.t1 || i >= (c ? H.nc : H.nv)) return false;
-  const int4* e = reinterpret_cast<const int4*>((c ? A.mix.chan + R.chan0 : A.mix.vox + R.vox0) + i);
+  const int lane = (int)(threadIdx.x & 31u);
+  const int kind = t < H.tc ? 0 : t < H.tc + H.tv ? 1 : 2;
+  const int i = (kind == 0 ? t : kind == 1 ? t - H.tc : t - H.tc - H.tv) * 32 + lane;
+  if (t >= H.t1 || i >= (kind == 0 ? H.nc : kind == 1 ? H.nv : H.ng)) return false;
+  static_assert(sizeof(MixVoxel) == 32 && sizeof(MixGroup) == 32, "two 16-byte loads");
+  const int4* e = kind == 0   ? reinterpret_cast<const int4*>(A.mix.chan + R.chan0 + i)
+                  : kind == 1 ? reinterpret_cast<const int4*>(A.mix.vox + R.vox0 + i)
+                              : reinterpret_cast<const int4*>(A.mix.grp + R.grp0 + i);
   e0 = __ldg(e);
   e1 = __ldg(e + 1);
   return true;
@@ -754,7 +878,7 @@ __device__ __forceinline__ int march_next(MarchShared& S, int items) {
 }
 
 // Boundary tiles (from tile k of the CTA on, then those the warp takes next; nu: the CTA's units).
-template <int MS, bool SUR>
+template <int MS, unsigned FQ, bool SUR>
 __device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R, const MarchShare& H, int nu, int k) {
   extern __shared__ __align__(128) unsigned char smem[];
   MarchShared& S = *reinterpret_cast<MarchShared*>(smem);
@@ -770,7 +894,10 @@ __device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R,
     } else {
       have = march_entry(A, R, H, H.t0 + k, e0, e1);
     }
-    if (have) mixed_voxel<MS, SUR>(S.desc, S.step, A.descs[R.r], A.ctl[R.r], A.mix, e0, e1);
+    if (have) {
+      if (H.t0 + k < H.tc + H.tv) mixed_voxel<MS, SUR>(S.desc, S.step, A.descs[R.r], A.ctl[R.r], A.mix, e0, e1);
+      else mixed_group<MS, FQ, SUR>(S.desc, S.step, A.descs[R.r], e0, e1);
+    }
     __syncwarp();
   }
 }
@@ -849,7 +976,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
           march_dispatch<MS, FQ, SUR, BODY>(S, A.descs, R.r, col, S.cut[seg], S.cut[seg + 1]);
           __syncwarp();
         }
-        if (item < items) march_mixed<MS, SUR>(A, R, H, nu, item - nu);
+        if (item < items) march_mixed<MS, FQ, SUR>(A, R, H, nu, item - nu);
       }
       if (!(A.what & (MARCH_ADVANCE | MARCH_REPEAT))) break;
       __syncthreads();

@@ -51,6 +51,7 @@ struct HostReal {
   std::vector<GroupPattern> pat;  // regular groups (GroupPattern)
   double serca = 0.0;             // scale of the SERCA law (FluxParams::p[9])
   FluxParams gate[2] = {};        // RyR, pRyR
+  bool dense = false;             // every group is boundary work (MIX_DENSE)
   std::vector<double> acc;        // prefix sums of the planes' costs (march_cut)
   // padded linear device index of physical species voxel (x, y, z)
   long long dev_index(int x, int y, int z) const {
@@ -191,8 +192,9 @@ struct csp_handle {
   // items; realisation-major like the rows
   MixVoxel* d_mix = nullptr;
   MixVoxel* d_mixc = nullptr;
+  MixGroup* d_grp = nullptr;
   MixItem* d_items = nullptr;
-  std::vector<int> mix_first, mixc_first;
+  std::vector<int> mix_first, mixc_first, grp_first;
   // csp_run_states: host-to-device stream, staging (two input and two output slots), per
   // step stop flags
   cudaStream_t in_stream = nullptr;
@@ -476,6 +478,39 @@ bool regular_group(const RealDesc& D, const MixVoxel* m, GroupPattern& g) {
   }
   // (across z, inside the group, the other side's base would be another voxel's)
   return k >= 2;
+}
+
+// The irregular group whose n voxels in the box are m[0..n) (n up to 4, no channels) as one
+// entry; false: a flux of it is no SERCA flux from a neighbour, or not in the order of faces.
+// faces: the directions in the order in which a voxel's pairs come when they are listed by their
+// voxels' coordinates.
+bool irregular_group(const RealDesc& D, const MixVoxel* m, int n, const std::vector<MixItem>& items, const int* faces,
+                     MixGroup& g) {
+  memset(&g, 0, sizeof g);
+  g.v = m[0].v;
+  g.order = (unsigned)n << 18;
+  for (int i = 0; i < 6; i++) g.order |= (unsigned)faces[i] << (3 * i);
+  const int off[6] = {-1, 1, -D.nz, D.nz, -D.P, D.P};
+  for (int j = 0; j < n; j++) {
+    g.code[j] = m[j].code;
+    if (m[j].item.meta & MIX_NONE) continue;
+    MixItem it = m[j].item;
+    const unsigned first = it.meta;
+    unsigned f = ((first & MIX_TO) ? MIXG_TO : 0u) | ((first & MIX_APPLY) ? MIXG_APPLY : 0u);
+    for (int i = 0;; i++) {
+      while (i < 6 && m[j].v + off[faces[i]] != it.vo) i++;
+      if (i == 6) return false;
+      const int k = faces[i];
+      if (!(it.meta & MIX_SERCA) || (it.meta >> 8 & 0xffffu) != 0 || ((it.meta ^ first) & (MIX_TO | MIX_APPLY)) ||
+          !(m[j].code >> (21 + k) & 1u) || (it.meta >> 27 & 7u) != (m[j].code >> (3 + 3 * k) & 7u))
+        return false;
+      f |= 1u << i;
+      if (it.meta & MIX_LAST) break;
+      it = items[it.more];
+    }
+    g.flux |= f << (8 * j);
+  }
+  return true;
 }
 
 }  // namespace
@@ -822,6 +857,10 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       cudaStreamSynchronize(h->stream);
       for (size_t i = pairs.size(); i-- > 0 && pairs[i].r == r;)
         codes[first + pairs[i].v0 / 4] = codes[first + pairs[i].v1 / 4] = CODE_MIXED;
+      // (kernel padding has CODE_MIXED too: the share is of the groups with voxels)
+      const size_t uniform = groups - std::count(codes.begin() + first, codes.begin() + first + groups, CODE_MIXED);
+      hr.dense = D.react_fast && dom_total >= MIX_GROUPS_MIN && (double)uniform < MIX_DENSE * D.nx * (D.plane / 4);
+      if (hr.dense) std::fill(codes.begin() + first, codes.begin() + first + groups, CODE_MIXED);
       mix_voxels(D, r, codes.data() + first, hostd, mix);
     }
     // initial channel states (BoundaryFluxes_init_stochastic_boundaries, boundaryfluxes.c:544-605)
@@ -967,7 +1006,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       const int r = group[0].r;
       const RealDesc& D = h->real[r].desc;
       GroupPattern g;
-      if (ng == 4 && !chan_of[0] && !chan_of[1] && !chan_of[2] && !chan_of[3] &&
+      if (ng == 4 && !h->real[r].dense && !chan_of[0] && !chan_of[1] && !chan_of[2] && !chan_of[3] &&
           regular_group(D, group, g)) {
         std::vector<GroupPattern>& P = pats[r];
         size_t i = 0;
@@ -1027,6 +1066,38 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     }
     if (ng) flush();
     mix.swap(rest);
+  }
+  // batches with many irregular voxels: those as groups
+  const size_t irregular = mix.size();
+  std::vector<MixGroup> grp;
+  std::vector<int> grp_of;              // their realisations
+  for (size_t i = 0, k = 0; i < mix.size();) {
+    const int r = mix[i].r;
+    size_t end = i;
+    while (end < mix.size() && mix[end].r == r) end++;
+    const HostReal& hr = h->real[r];
+    const RealDesc& D = hr.desc;
+    int faces[6];                       // x-, y-, z-, z+, y+, x+ as device directions
+    for (int a = 0; a < 3; a++) {
+      const int physical = hr.perm[a];
+      faces[physical] = (2 - a) * 2;
+      faces[5 - physical] = (2 - a) * 2 + 1;
+    }
+    const bool many = irregular >= MIX_GROUPS_MIN && D.react_fast;
+    while (i < end) {
+      size_t j = i + 1;
+      while (j < end && mix[j].v / 4 == mix[i].v / 4) j++;
+      const int z = mix[i].v % D.P % D.nz;
+      MixGroup g;
+      if (many && z % 4 == 0 && (int)(j - i) == std::min(4, D.nzv - z) &&
+          irregular_group(D, &mix[i], (int)(j - i), items, faces, g)) {
+        grp.push_back(g);
+        grp_of.push_back(r);
+        i = j;
+      }
+      for (; i < j; i++) mix[k++] = mix[i];
+    }
+    if (i == mix.size()) mix.resize(k);
   }
   h->nrows = (int)rows.size();
   // rows touched by density pairs only first (gating-free launch), channel rows after
@@ -1100,6 +1171,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     };
     firsts(h->mix_first, (int)mix.size(), [&](int i) { return mix[i].r; });
     firsts(h->mixc_first, (int)mixc.size(), [&](int i) { return mixc[i].r; });
+    firsts(h->grp_first, (int)grp.size(), [&](int i) { return grp_of[i]; });
     firsts(h->drow_first, h->ndrows, [&](int i) { return drows[i].r; });
     firsts(h->krow_first, h->nrows_density, [&](int i) { return rows[i].r; });
     firsts(h->crow_first, h->nrows - h->nrows_density, [&](int i) { return rows[h->nrows_density + i].r; });
@@ -1132,6 +1204,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
             (drows.empty() || upload((void**)&h->d_drows, drows.data(), drows.size() * sizeof(DensityRow))) &&
             upload((void**)&h->d_mix, mix.empty() ? nullptr : mix.data(), mix.size() * sizeof(MixVoxel)) &&
             upload((void**)&h->d_mixc, mixc.empty() ? nullptr : mixc.data(), mixc.size() * sizeof(MixVoxel)) &&
+            upload((void**)&h->d_grp, grp.empty() ? nullptr : grp.data(), grp.size() * sizeof(MixGroup)) &&
             upload((void**)&h->d_items, items.empty() ? nullptr : items.data(), items.size() * sizeof(MixItem)) &&
             upload((void**)&h->d_rows, rows.empty() ? nullptr : rows.data(), rows.size() * sizeof(FluxRow)) &&
             upload((void**)&h->d_entries, entries.empty() ? nullptr : entries.data(), entries.size() * sizeof(FluxEntry)) &&
@@ -1197,9 +1270,10 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
   for (int i = 0; i < n; i++) order[i] = r0 + i;
   auto desc = [&](int r) -> const RealDesc& { return h->real[r].desc; };
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return working_set(desc(a)) > working_set(desc(b)); });
-  auto columns = [&](int r) { return (desc(r).plane + MARCH_COL - 1) / MARCH_COL; };
+  auto columns = [&](int r) { return h->real[r].dense ? 0 : (desc(r).plane + MARCH_COL - 1) / MARCH_COL; };
   auto tiles_of = [&](int r) {
-    return (h->mixc_first[r + 1] - h->mixc_first[r] + 31) / 32 + (h->mix_first[r + 1] - h->mix_first[r] + 31) / 32;
+    return (h->mixc_first[r + 1] - h->mixc_first[r] + 31) / 32 + (h->mix_first[r + 1] - h->mix_first[r] + 31) / 32 +
+           (h->grp_first[r + 1] - h->grp_first[r] + 31) / 32;
   };
   int most = 0;
   for (double sum = 0.0; most < std::min(n, h->ctas);) {
@@ -1263,6 +1337,8 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
       m.nchan = h->mixc_first[r + 1] - m.chan0;
       m.vox0 = h->mix_first[r];
       m.nvox = h->mix_first[r + 1] - m.vox0;
+      m.grp0 = h->grp_first[r];
+      m.ngrp = h->grp_first[r + 1] - m.grp0;
       real.push_back(m);
     }
     first.push_back((int)real.size());
@@ -1322,6 +1398,7 @@ static cudaError_t launch_march(csp_handle* h, const MarchPlan& pl, long long ns
   a.what = what;
   a.mix.chan = h->d_mixc;
   a.mix.vox = h->d_mix;
+  a.mix.grp = h->d_grp;
   a.mix.items = h->d_items;
   a.mix.pairs = h->d_pairs;
   a.mix.params = h->d_params;
@@ -3010,7 +3087,8 @@ extern "C" void csp_destroy(csp_handle* h) {
   if (h->graph) cudaGraphExecDestroy(h->graph);
   for (MarchPlan& p : h->plans) free_plan(p);
   cudaFree(h->d_fields); cudaFree(h->d_dom); cudaFree(h->d_gcode); cudaFree(h->d_desc); cudaFree(h->d_vdesc); cudaFree(h->d_ctl);
-  cudaFree(h->d_rec); cudaFree(h->d_drows); cudaFree(h->d_mix); cudaFree(h->d_mixc); cudaFree(h->d_items);
+  cudaFree(h->d_rec); cudaFree(h->d_drows); cudaFree(h->d_mix); cudaFree(h->d_mixc); cudaFree(h->d_grp);
+  cudaFree(h->d_items);
   cudaFree(h->d_rows); cudaFree(h->d_entries); cudaFree(h->d_pairs); cudaFree(h->d_params);
   cudaFree(h->d_states); cudaFree(h->d_err); cudaFree(h->d_red); cudaFree(h->d_red_out); cudaFree(h->d_line);
   cudaFree(h->d_stage);
