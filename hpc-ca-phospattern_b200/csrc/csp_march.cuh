@@ -24,7 +24,7 @@
 // voxels of irregular groups and those with channels are the boundary work (mixed_voxel), in
 // tiles of 32; where there are many, irregular groups are, in tiles of 32 groups (mixed_group).
 //
-// The barrier's wait is bounded in time (WAIT_NS).  A CTA that gives up sets ERR_TIMEOUT in the
+// The barrier's wait is bounded in time (MarchArgs::wait_ns).  A CTA that gives up sets ERR_TIMEOUT in the
 // device error word, which the other waits see too, and every CTA leaves the launch; the fields
 // are undefined then (the host reports CSP_EDEVICE).  Nothing is in flight when a CTA leaves
 // but its own plain loads and stores.
@@ -42,7 +42,7 @@ namespace csp {
 
 constexpr int MARCH_T = 512;              // threads per CTA
 constexpr int MARCH_COL = 128;            // plane positions per unit: 4 per lane
-constexpr unsigned long long INJECT_WAIT_NS = 1000000ull;   // 1 ms for the test hook's wait
+constexpr unsigned long long INJECT_WAIT_NS = 1000000ull;   // limit of a wait with the test hook: 1 ms
 
 // What a launch does with the step of a realisation.
 enum : unsigned {
@@ -87,6 +87,7 @@ struct MarchArgs {
   int* flags;                        // nullable [nsteps][flag_stride]: stop flag of realisation r at [r - flag_r0]
   int flag_stride, flag_r0;
   int* err;
+  unsigned long long wait_ns;        // limit of a wait
   int inject;                        // test hook (csp_test_wait_timeout)
 };
 
@@ -533,7 +534,7 @@ struct MarchCount {
 __device__ __forceinline__ void march_arrive(unsigned* arrived) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
 }
-__device__ __forceinline__ bool march_wait(const unsigned* arrived, unsigned target, int* err) {
+__device__ __forceinline__ bool march_wait(const unsigned* arrived, unsigned target, unsigned long long limit_ns, int* err) {
   auto count = [&]() {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
@@ -543,7 +544,7 @@ __device__ __forceinline__ bool march_wait(const unsigned* arrived, unsigned tar
   const unsigned long long t0 = global_ns();
   while (count() < target) {
     if (*(volatile int*)err & ERR_TIMEOUT) return false;
-    if (global_ns() - t0 > WAIT_NS) {
+    if (global_ns() - t0 > limit_ns) {
       atomicOr(err, ERR_TIMEOUT);
       return false;
     }
@@ -910,14 +911,12 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
   const int team = blockIdx.x / A.size, rank = blockIdx.x - team * A.size;
   unsigned target = 0;                   // arrivals after which the team's next barrier opens
   if (A.inject && blockIdx.x == 0) {
-    // test hook: one thread waits for an arrival that nothing makes; this CTA then leaves and
-    // the waits of the others see the error word
-    if (tid == 37) {
-      const volatile unsigned* never = A.arrived + 31;
-      const unsigned long long t0 = global_ns();
-      while (*never == 0u && global_ns() - t0 < INJECT_WAIT_NS) {}
-      if (*never == 0u) atomicOr(A.err, ERR_TIMEOUT);
-    }
+    // test hook: this CTA leaves without arriving, so that the waits of its team run out.  Where
+    // no CTA will wait for it, one thread waits for an arrival that nothing makes.
+    bool waited_for = false;
+    if (A.size > 1 && A.nsteps > 0 && (A.what & (MARCH_ADVANCE | MARCH_REPEAT)))
+      for (int e = A.first[0]; e < A.first[1]; e++) waited_for = waited_for || !A.ctl[A.real[e].r].stopped;
+    if (!waited_for && tid == 37) march_wait(A.arrived + 31, 1u, A.wait_ns, A.err);
     return;
   }
   for (int e = A.first[team]; e < A.first[team + 1]; e++) {
@@ -989,7 +988,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
         unsigned pre = 0, updated = 0, dsi = 0, flags = 0;
         if (adv) count.next(lane, pre, updated, dsi, flags);
         bool ok = true;
-        if (A.size > 1 && lane == 0) ok = march_wait(A.arrived + team * 32, target, A.err);
+        if (A.size > 1 && lane == 0) ok = march_wait(A.arrived + team * 32, target, A.wait_ns, A.err);
         // every lane has read the step's masks (votes and reductions are no memory barriers)
         __syncwarp();
         // the step is taken: every CTA of the team follows the same rules (see k_epilogue)

@@ -1408,6 +1408,7 @@ static cudaError_t launch_march(csp_handle* h, const MarchPlan& pl, long long ns
   a.flags = flags;
   a.flag_stride = h->n;
   a.err = h->d_err;
+  a.wait_ns = h->inject_wait ? INJECT_WAIT_NS : WAIT_NS;
   a.inject = h->inject_wait;
   // the classification belongs to a reaction step, which is launched alone (launch_steps); the
   // stretches between take the kernel without it

@@ -301,10 +301,11 @@ int csp_set_phase_timing(csp_handle* h, int32_t on);
 int csp_get_phase_times(const csp_handle* h, double* ms, int64_t* steps);
 
 /* Test hook for the failure path of the step kernel's bounded waits.  While armed (on != 0),
- * every launch of the step kernel makes one thread of its first CTA wait for an arrival that
- * nothing makes, with a 1 ms limit; the thread then sets the timeout bit of the device error
- * word and the CTA leaves, the CTAs that wait for it at a barrier see the bit and leave too,
- * and csp_advance returns CSP_EDEVICE with csp_status naming the timeout.  The handle's fields are
+ * the limit of a wait is 1 ms and the first CTA of every launch of the step kernel leaves
+ * without arriving at its team's barrier: the CTAs that wait for it reach the limit, set the
+ * timeout bit of the device error word and leave (where none will wait for it, it waits itself
+ * for an arrival that nothing makes), and csp_advance returns CSP_EDEVICE with csp_status
+ * naming the timeout.  The handle's fields are
  * undefined afterwards and the error stays set; the device and other handles stay usable.
  * No counterpart in the reference: it has no device and aborts on any error
  * (fvm_mpi/src/utils.h:21-27). */
