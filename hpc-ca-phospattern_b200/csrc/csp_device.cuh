@@ -200,13 +200,13 @@ static_assert(sizeof(FluxRow) % 16 == 0, "whole 16-byte words");
 enum : unsigned { MIX_LAST = 1u, MIX_APPLY = 2u, MIX_TO = 4u, MIX_SERCA = 8u, MIX_OWNER = 16u, MIX_CHANNEL = 0x20u,
                   MIX_PRYR = 0x40u, MIX_NONE = 0x80u };
 struct alignas(16) MixItem {
-  int vo;
+  unsigned vo;
   unsigned meta;                     // MIX_NONE: no flux
   int pair;
   int more;                          // MixVoxel::item: index of the next one
 };
 struct alignas(16) MixVoxel {
-  int v;                             // field index
+  unsigned v;                        // field index
   unsigned code;
   int r;                             // realisation (the device copy: the channel's index in its boundary and, from
                                      // bit 24, the boundary)
@@ -221,7 +221,7 @@ struct alignas(16) MixVoxel {
 // receiving side, MIXG_APPLY.
 enum : unsigned { MIXG_TO = 0x40u, MIXG_APPLY = 0x80u };
 struct alignas(16) MixGroup {
-  int v;                             // field index of the first voxel
+  unsigned v;                        // field index of the first voxel
   unsigned flux, order, pad;
   unsigned code[4];
 };

@@ -274,11 +274,11 @@ __global__ void __launch_bounds__(256) k_voxels_direct(const RealDesc* __restric
   const StepInfo si = s_si;
   const unsigned cur = s_cur;
   const int nz = D.nz, plane = D.plane;
-  const int nvox = D.nx * plane;
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned nvox = (unsigned)D.nx * plane;
+  const unsigned v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvox || si.updated == 0) return;
-  const int x = v / plane;
-  const int p = v - x * plane;
+  const int x = (int)(v / plane);
+  const int p = (int)(v - (unsigned)x * plane);
   const int y = p / nz;
   const int z = p - y * nz;
   if (z >= D.nzv) return;

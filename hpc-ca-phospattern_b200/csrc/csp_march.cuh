@@ -235,7 +235,7 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
   }
   const int cut = D.nzv != nz && G.lastj < 3 ? G.lastj : 4;     // the row ends inside the group, after voxel cut
   const int nx = D.nx, P = D.P;
-  int off = x0 * P + p0;                         // the lane's position (fields hold < 2^31)
+  unsigned off = (unsigned)x0 * P + p0;          // the lane's position (padded fields hold < 2^32)
   // planes x-1, x, x+1 (cur: also the species that only react)
   float4 prv[MS], cur[MS], nxt[MS];
 #pragma unroll
@@ -257,7 +257,7 @@ __device__ __forceinline__ void march_unit(const RealDesc* __restrict__ descs, i
     for (int s = 0; s < MS; s++) {
       fut[s] = nxt[s];
       if ((pre >> s & 1u) && more && x + 2 < nx)
-        fut[s] = *reinterpret_cast<const float4*>(field(U.uo[s]) + (off + 2 * P));
+        fut[s] = *reinterpret_cast<const float4*>(field(U.uo[s]) + (off + 2u * P));
     }
     if (more) code_next = __ldg(D.gcode + ((off + P) >> 2));
     // every neighbour before the first store: a load that follows a store to another buffer
@@ -571,7 +571,7 @@ __device__ __noinline__ bool mix_pair_flux(const RealDesc& D, RealCtl* C, const 
 template <int MS, bool SUR>
 __device__ __forceinline__ void mixed_voxel(const VoxDesc& D, const MarchStep& U, const RealDesc& R, RealCtl& C,
                                             const MixArgs& A, const int4& e0, const int4& e1) {
-  const int v = e0.x;
+  const unsigned v = (unsigned)e0.x;
   const unsigned code = (unsigned)e0.y, valid = (code >> 21) & 63u;
   const unsigned pre = U.pre, updated = U.updated;
   const int d = (int)(code & 7u);
@@ -591,7 +591,7 @@ __device__ __forceinline__ void mixed_voxel(const VoxDesc& D, const MarchStep& U
   int ch_old = 0;
   if (!(m0 & MIX_NONE)) {
     const float* u = field(U.uo[sp0]);
-    part = u[e1.x];
+    part = u[(unsigned)e1.x];
     self = u[v];
     if (m0 & MIX_CHANNEL) ch_old = A.states[(U.k & 1) * (long long)A.nch + e0.w];
   }
@@ -607,7 +607,7 @@ __device__ __forceinline__ void mixed_voxel(const VoxDesc& D, const MarchStep& U
     for (int q = 0; q < 6; q++) un[s][q] = u[off[q]];
   }
   // fluxes of the item's species: the items of one species follow one another
-  MixItem it{e1.x, m0, e1.z, e1.w};
+  MixItem it{(unsigned)e1.x, m0, e1.z, e1.w};
   auto base = [&](unsigned dd, int s) -> double { return s == 0 ? D.base0[dd] : R.base[dd][s]; };
   auto fluxes = [&](int& sp, bool& apply, double& acc, bool& left, bool first) -> bool {
     bool any = false;
@@ -666,7 +666,7 @@ __device__ __forceinline__ void mixed_voxel(const VoxDesc& D, const MarchStep& U
         return any;
       }
       const int4 q = __ldg(reinterpret_cast<const int4*>(A.items + it.more));
-      it = MixItem{q.x, (unsigned)q.y, q.z, q.w};
+      it = MixItem{(unsigned)q.x, (unsigned)q.y, q.z, q.w};
     }
   };
   int sp = -1;
@@ -729,7 +729,7 @@ __device__ __forceinline__ float part(const float4& q, int j) { return j == 0 ? 
 template <int MS, unsigned FQ, bool SUR>
 __device__ __forceinline__ void mixed_group(const VoxDesc& D, const MarchStep& U, const RealDesc& R, const int4& e0,
                                             const int4& e1) {
-  const int v = e0.x;
+  const unsigned v = (unsigned)e0.x;
   const unsigned flux = (unsigned)e0.y, order = (unsigned)e0.z;
   const unsigned code[4] = {(unsigned)e1.x, (unsigned)e1.y, (unsigned)e1.z, (unsigned)e1.w};
   const int nv = (int)(order >> 18);
@@ -891,7 +891,7 @@ __device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R,
       const int i = k * 32 + (int)(threadIdx.x & 31u);
       e0 = S.tile[i][0];
       e1 = S.tile[i][1];
-      have = e0.x >= 0;
+      have = e0.x != -1;
     } else {
       have = march_entry(A, R, H, H.t0 + k, e0, e1);
     }

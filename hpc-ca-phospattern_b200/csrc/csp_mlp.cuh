@@ -828,8 +828,8 @@ __device__ __forceinline__ void rx_correct(const RxDom& K, const RealDesc& D, fl
   if (K.store & 1u) {
     bool face = false;
     if (D.dirichlet) {
-      const int vi = (int)v, xq = vi / D.P;
-      face = rx_on_face(D, xq, vi - xq * D.P);
+      const int xq = (int)(v / D.P);
+      face = rx_on_face(D, xq, (int)(v - (long long)xq * D.P));
     }
     if (!face) un[0][v] = __fadd_rn(now[0], __fadd_rn(sdj, dc));
   }
@@ -969,14 +969,14 @@ __device__ __forceinline__ void rx_cache_fill(const RealDesc& D, const RealCtl& 
 // old ones, 200 steps of 24 100x100x50 grids, 20 of them reactions with 5.2 M network voxels
 // each: 42.5 -> 34.5 ms (k_react_network 20 -> 12 ms of it).
 struct RxRejects {
-  int v[64];
+  unsigned v[64];
   unsigned char d[64];
 };
 __device__ __forceinline__ void rx_reject(RxRejects& J, int& n, bool rejected, long long v, int d, int lane) {
   const unsigned m = __ballot_sync(0xffffffffu, rejected);
   if (rejected) {
     const int i = n + __popc(m & ((1u << lane) - 1u));
-    J.v[i] = (int)v;
+    J.v[i] = (unsigned)v;
     J.d[i] = (unsigned char)d;
   }
   n += __popc(m);

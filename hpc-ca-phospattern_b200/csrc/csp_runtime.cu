@@ -60,12 +60,14 @@ struct HostReal {
   }
 };
 
+static int round_up(int a, int b) { return (a + b - 1) / b * b; }
+
 // Device axis order of one realisation.  The stencil is isotropic and every face has the
 // same no-flux rule, so the kernels may hold the field in any axis order.  The marching
 // axis (device axis 0) is the physical axis crossed by the most domain changes, so that
 // domain-boundary sheets (cleft, jSR, network SR at fixed z in a dyad) become whole
 // planes and the voxels sharing a warp share a neighbourhood type.
-static void choose_axes(const csp_model& m, int perm[3]) {
+static void choose_axes(const csp_model& m, int S, int perm[3]) {
   long long ch[3] = {0, 0, 0};
   const int N0 = m.N[0], N1 = m.N[1], N2 = m.N[2];
   for (int x = 0; x < N0; x++)
@@ -82,11 +84,16 @@ static void choose_axes(const csp_model& m, int perm[3]) {
   int rest[2], k = 0;
   for (int a = 0; a < 3; a++)
     if (a != a0) rest[k++] = a;
-  // contiguous last: a length that is a multiple of 4 (4-voxel groups then never straddle
-  // a row), then the fewest changes; on a tie keep the physical order
+  // contiguous last: a length that is a multiple of 4 (its rows need no padding), then the one
+  // whose rows take at least 8 % less padding (a row of 1 voxel takes 4 positions, in memory and
+  // in every step), then the fewest changes; on a tie keep the physical order
   const int n[3] = {N0, N1, N2};
   const bool a4 = n[rest[0]] % 4 == 0, b4 = n[rest[1]] % 4 == 0;
-  const bool swap = a4 != b4 ? a4 : ch[rest[0]] < ch[rest[1]];
+  auto padded = [&](int a) { return (double)round_up(n[a] * S, 4) / (n[a] * S); };
+  const double pa = padded(rest[0]), pb = padded(rest[1]);
+  const bool swap = a4 != b4                                ? a4
+                    : std::max(pa, pb) > 1.08 * std::min(pa, pb) ? pa < pb
+                                                                 : ch[rest[0]] < ch[rest[1]];
   perm[0] = a0;
   perm[1] = swap ? rest[1] : rest[0];
   perm[2] = swap ? rest[0] : rest[1];
@@ -406,11 +413,11 @@ void mix_voxels(const RealDesc& D, int r, const unsigned char* code,
                 const std::vector<unsigned char>& dom, std::vector<MixVoxel>& out) {
   for (int x = 0; x < D.nx; x++)
     for (int y = 0; y < D.ny; y++) {
-      const int row = x * D.P + y * D.nz;
+      const unsigned row = (unsigned)x * D.P + (unsigned)y * D.nz;
       for (int g = 0; g < D.nz / 4; g++) {
         if (code[row / 4 + g] != CODE_MIXED) continue;
         for (int z = 4 * g; z < std::min(4 * g + 4, D.nzv); z++) {
-          const int v = row + z;
+          const unsigned v = row + z;
           const unsigned valid = (z > 0 ? 1u : 0u) | (z < D.nzv - 1 ? 2u : 0u) | (y > 0 ? 4u : 0u) |
                                  (y < D.ny - 1 ? 8u : 0u) | (x > 0 ? 16u : 0u) | (x < D.nx - 1 ? 32u : 0u);
           const int off[6] = {-1, 1, -D.nz, D.nz, -D.P, D.P};
@@ -564,8 +571,6 @@ static void ryr_params(FluxParams& fp, const csp_ryr_params& p, double t_close) 
   fp.k1 = 0.0;
 }
 
-static int round_up(int a, int b) { return (a + b - 1) / b * b; }
-
 extern "C" int csp_create(const csp_model* models, const csp_options* options, int32_t n, csp_handle** out) {
   if (!out) return fail(nullptr, CSP_EINVAL, "out is NULL");
   *out = nullptr;
@@ -580,13 +585,18 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     int rc = derive(models[r], options[r], dv[r], err);
     if (rc) { delete h; return fail(nullptr, rc, "realisation %d: %s", r, err.c_str()); }
     HostReal& hr0 = h->real[r];
-    choose_axes(models[r], hr0.perm);
+    choose_axes(models[r], dv[r].S, hr0.perm);
     hr0.nphys[0] = dv[r].nx; hr0.nphys[1] = dv[r].ny; hr0.nphys[2] = dv[r].nz;
     const int n0 = hr0.nphys[hr0.perm[0]], n1 = hr0.nphys[hr0.perm[1]], n2 = hr0.nphys[hr0.perm[2]];
-    const long long plane_ll = (long long)n1 * round_up(n2, 4);
-    const long long P_ll = (plane_ll + PLANE_ALIGN - 1) / PLANE_ALIGN * PLANE_ALIGN;
+    // 2^31 voxels per field; with its rows' padding it stays below the 2^32 positions that the
+    // kernels index (a plane above 128 voxels grows by half at most)
+    auto plane_of = [](long long positions) { return (positions + PLANE_ALIGN - 1) / PLANE_ALIGN * PLANE_ALIGN; };
+    const long long plane_ll = (long long)n1 * round_up(n2, 4), P_ll = plane_of(plane_ll);
+    if (n0 * plane_of((long long)n1 * n2) >= (1ll << 31) || n0 * P_ll >= (1ll << 32) || P_ll >= (1ll << 31)) {
+      delete h;
+      return fail(nullptr, CSP_EINVAL, "realisation %d: grid too large (2^31 voxels per field)", r);
+    }
     const int plane = (int)plane_ll, P = (int)P_ll;
-    if (n0 * P_ll >= (1ll << 31)) { delete h; return fail(nullptr, CSP_EINVAL, "realisation %d: grid too large (2^31 voxels per field)", r); }
     hr0.field_elems = (size_t)n0 * P;
     field_total += hr0.field_elems * 2 * models[r].num_species;
     dom_total += hr0.field_elems;
@@ -1035,7 +1045,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
           const bool to = sign > 0.f, chan = p.channel >= 0;
           const unsigned d0 = p.doms & DOMAIN_BITS, d1 = (p.doms >> 3) & DOMAIN_BITS;
           MixItem it;
-          it.vo = (int)(to ? p.v0 : p.v1);
+          it.vo = (unsigned)(to ? p.v0 : p.v1);
           it.pair = pair;
           it.more = 0;
           it.meta = (rw.apply ? MIX_APPLY : 0u) | (to ? MIX_TO : 0u) |
