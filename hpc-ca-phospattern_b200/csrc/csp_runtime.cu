@@ -2791,8 +2791,9 @@ static cudaError_t mlp_grad_launch(const float* dp, const float* dx, const float
 }
 
 // csp_mlp_gradient's device memory: a pool per device that keeps up to GRAD_POOL_KEEP bytes
-// from call to call (a cudaMalloc and cudaFree of them cost 0.5 ms, the kernel 0.2) and gives
-// the rest back when a call ends; csp_destroy gives back what is not in use.
+// from call to call (a cudaMalloc and cudaFree of them cost 0.5 ms, the kernel 0.2).  What is
+// above goes back when a call ends: at its wait after the free, a pool releases memory at a
+// synchronisation.  csp_destroy gives back what is not in use.
 constexpr unsigned long long GRAD_POOL_KEEP = 64ull << 20;
 constexpr int GRAD_POOL_DEVICES = 64;
 static std::mutex g_grad_pool_mu;
@@ -2822,8 +2823,11 @@ static cudaError_t grad_pool(cudaMemPool_t* pool) {
 
 static void grad_pool_trim() {
   std::lock_guard<std::mutex> lock(g_grad_pool_mu);
-  for (cudaMemPool_t p : g_grad_pool)
-    if (p) cudaMemPoolTrimTo(p, 0);
+  for (cudaMemPool_t p : g_grad_pool) {
+    if (!p) continue;
+    cudaStreamSynchronize(0);          // (a free of a call that ended may still be queued)
+    cudaMemPoolTrimTo(p, 0);
+  }
 }
 
 extern "C" int csp_mlp_gradient(const float* params, const float* x, const float* t, int64_t n, float* grad,
@@ -2832,11 +2836,11 @@ extern "C" int csp_mlp_gradient(const float* params, const float* x, const float
   // one allocation: parameters, gradient and loss, inputs, targets
   const size_t np = (MLP_NPARAM + 1 + 63) / 64 * 64;
   const size_t nx = ((size_t)n * MLP_IN + 63) / 64 * 64;
+  const size_t bytes = (2 * np + nx + (size_t)n * MLP_OUT) * sizeof(float);
   float* dp = nullptr;
   cudaMemPool_t pool = nullptr;
   cudaError_t e = grad_pool(&pool);
-  if (e == cudaSuccess)
-    e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dp), (2 * np + nx + (size_t)n * MLP_OUT) * sizeof(float), pool, 0);
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dp), bytes, pool, 0);
   float *dg = dp + np, *dx = dg + np, *dt = dx + nx;
   std::vector<float> out(MLP_NPARAM + 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(dg, 0, np * sizeof(float), 0);
@@ -2845,7 +2849,10 @@ extern "C" int csp_mlp_gradient(const float* params, const float* x, const float
   if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, n * MLP_OUT * sizeof(float), cudaMemcpyHostToDevice, 0);
   if (e == cudaSuccess) e = mlp_grad_launch(dp, dx, dt, n, dg, dg + MLP_NPARAM, 0);
   if (e == cudaSuccess) e = cudaMemcpy(out.data(), dg, out.size() * sizeof(float), cudaMemcpyDeviceToHost);
-  if (dp) cudaFreeAsync(dp, 0);
+  if (dp) {
+    cudaFreeAsync(dp, 0);
+    if (bytes > GRAD_POOL_KEEP) cudaStreamSynchronize(0);
+  }
   if (e != cudaSuccess) return fail(nullptr, CSP_ECUDA, "mlp gradient: %s", cudaGetErrorString(e));
   std::memcpy(grad, out.data(), MLP_NPARAM * sizeof(float));
   *loss = out[MLP_NPARAM];
@@ -3093,8 +3100,8 @@ extern "C" int csp_mlp_train(csp_handle* h, int32_t r, const csp_mlp_config* cfg
 
 extern "C" void csp_destroy(csp_handle* h) {
   if (!h) return;
-  grad_pool_trim();
   if (h->stream) cudaStreamSynchronize(h->stream);
+  grad_pool_trim();
   if (h->graph) cudaGraphExecDestroy(h->graph);
   for (MarchPlan& p : h->plans) free_plan(p);
   cudaFree(h->d_fields); cudaFree(h->d_dom); cudaFree(h->d_gcode); cudaFree(h->d_desc); cudaFree(h->d_vdesc); cudaFree(h->d_ctl);
