@@ -43,7 +43,6 @@ sys.path.insert(0, ROOT)
 N_REAL = 256
 SHAPE = (100, 100, 50)
 BYTES_PER_VOXEL_STEP = 41     # 5 species x (4 B read + 4 B written) + 1 B domain id, FP32
-MARCH_STEPS_MAX = 4096     # steps of one launch of the step kernel (csp_runtime.cu)
 
 
 def dist_env():
@@ -403,8 +402,10 @@ def main():
     D.barrier()
     clocks = Clocks(local)
     clocks.start()
+    launches = sim.step_launches()
     sim.advance(K)
     ms = sim.last_ms()
+    launches = sim.step_launches() - launches
     clk = clocks.stop()
     D.barrier()
     ms_max = D.reduce(ms, "max")
@@ -414,8 +415,8 @@ def main():
     # total of every species) of every rank on every rank: one all_gather
     gathered = int(len(ens.statistics()["index"]))
 
-    # ---- roofline of the dominant kernel.  The step kernel takes every step of a call in one
-    # launch, so its time per step is the timed region's; the direct kernel launches per step ----
+    # ---- roofline of the dominant kernel.  The step kernel takes many steps per launch, so its
+    # time per step is the timed region's; the direct kernel launches per step ----
     direct = tune["chosen"]["segment"] < 0
     nprof = min(K, 100)
     vms, bms = sim.profile(nprof)
@@ -484,9 +485,9 @@ def main():
                    "sample": f"{steps} steps of one 100x100x50 realisation of the workload "
                              f"({dt:.1f} s), FP64 port of the reference"}
 
-    # in the device-timed region: one launch of the step kernel per MARCH_STEPS_MAX steps; the
-    # direct kernel with its density-row, channel-row and epilogue kernels on every step
-    kernels = 4 * K if direct else -(-K // MARCH_STEPS_MAX)
+    # in the device-timed region: the step kernel's launches; the direct kernel with its
+    # density-row, channel-row and epilogue kernels on every step
+    kernels = 4 * K if direct else launches
     if rank == 0:
         line = {
             "metric": "ensemble voxel-steps/s", "value": value, "unit": "voxel-steps/s",

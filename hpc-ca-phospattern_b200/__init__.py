@@ -293,6 +293,12 @@ class Simulation:
         self._check(self.lib.csp_snapshot_read(self.h, u.ctypes.data_as(C.POINTER(C.c_double))))
         return u
 
+    def step_launches(self):
+        """Launches of the step kernel so far (csp_step_launches)."""
+        n = C.c_int64()
+        self._check(self.lib.csp_step_launches(self.h, C.byref(n)))
+        return n.value
+
     def profile(self, nsteps):
         """Advance nsteps with per-kernel CUDA events: (voxel_ms, boundary_ms) summed."""
         a, b = C.c_float(), C.c_float()

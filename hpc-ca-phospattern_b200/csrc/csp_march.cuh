@@ -1055,6 +1055,7 @@ struct MarchPlan {
   int teams = 0, size = 0;
   int nseg = 0;                      // segments of the first realisation
   bool known = false;                // march_kernel
+  double step_us = 0.0;              // estimated time of a step
   MarchReal* d_real = nullptr;
   int* d_first = nullptr;
   int* d_cuts = nullptr;

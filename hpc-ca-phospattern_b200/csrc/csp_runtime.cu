@@ -33,7 +33,13 @@ using namespace csp;
 namespace {
 
 constexpr int STEPS_PER_GRAPH = 16;
-constexpr int64_t MARCH_STEPS_MAX = 4096;   // steps per launch of the step kernel (a launch stays below a second)
+// Steps per launch of the step kernel: it holds every SM, and other handles, threads and streams
+// on the GPU wait for its end, so a launch takes at most about MARCH_LAUNCH_US by the plan's
+// estimate (measured / estimated: the reference model's shape 0.9 to 1.2, a single grid beyond
+// L2 1.7, eight species 5) and the fields' way through HBM at its start stays below 1 % of it
+// (256 grids of 100x100x50, 85 steps per launch, 0.8 of 95 ms).
+constexpr int64_t MARCH_STEPS_MAX = 4096;
+constexpr double MARCH_LAUNCH_US = 1e5;
 constexpr int PHASE_SAMPLE = 16;            // steps timed per advance call (csp_set_phase_timing)
 thread_local char g_create_error[512];
 
@@ -229,6 +235,7 @@ struct csp_handle {
   int ctas = 0;
   size_t l2 = 0;
   std::vector<MarchPlan> plans;
+  int64_t march_launches = 0;        // csp_step_launches
   cudaGraphExec_t graph = nullptr;
   int graph_surrogate = 0;
   int graph_sur_tc = 0;
@@ -1329,7 +1336,7 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
   pl.known = true;
   for (int r = r0; r < r1; r++) pl.known = pl.known && march_masks_known(desc(r));
   std::vector<std::vector<int>> team(best);
-  deal(best, &team);
+  pl.step_us = deal(best, &team);
   std::vector<MarchReal> real;
   std::vector<int> first(1, 0), cuts, one;
   for (const auto& t : team) {
@@ -1422,6 +1429,7 @@ static cudaError_t launch_march(csp_handle* h, const MarchPlan& pl, long long ns
   a.inject = h->inject_wait;
   // the classification belongs to a reaction step, which is launched alone (launch_steps); the
   // stretches between take the kernel without it
+  h->march_launches++;
   MarchKernel k = march_kernel(h->ms, pl.known, h->surrogate != 0 && !(what & (MARCH_ADVANCE | MARCH_REPEAT)));
   const unsigned grid = (unsigned)(pl.teams * pl.size);
   if (pl.size == 1 || !(what & (MARCH_ADVANCE | MARCH_REPEAT))) {
@@ -1582,8 +1590,8 @@ static int64_t steps_without_reaction(const csp_handle* h, int r0, int r1, int64
 }
 
 // nsteps steps of [r0, r1); step_flags (nullable, device): every realisation's stop flag after
-// every step, [nsteps][n].  The step kernel takes all of them in one launch; with the
-// surrogate on, those between two reaction steps.
+// every step, [nsteps][n].  The step kernel takes as many as a launch may (MARCH_LAUNCH_US), with
+// the surrogate on those between two reaction steps.
 static int launch_steps(csp_handle* h, int r0, int r1, int64_t nsteps, int* step_flags) {
   if (nsteps <= 0) return CSP_OK;
   if (h->kernel == 1) {
@@ -1596,8 +1604,9 @@ static int launch_steps(csp_handle* h, int r0, int r1, int64_t nsteps, int* step
   const MarchPlan* pl;
   int rc = plan_for(h, r0, r1, &pl);
   if (rc) return rc;
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(MARCH_STEPS_MAX, (int64_t)(MARCH_LAUNCH_US / pl->step_us)));
   for (int64_t i = 0; i < nsteps;) {
-    int64_t m = std::min<int64_t>(nsteps - i, MARCH_STEPS_MAX);
+    int64_t m = std::min<int64_t>(nsteps - i, most);
     if (h->surrogate) m = steps_without_reaction(h, r0, r1, i, m);
     if (m > 0) {
       CUDA_TRY(h, launch_march(h, *pl, m, MARCH_STEP, step_flags ? step_flags + i * h->n : nullptr));
@@ -2479,6 +2488,12 @@ extern "C" int csp_get_stream(const csp_handle* h, void** stream) {
 extern "C" int csp_last_advance_ms(const csp_handle* h, float* ms) {
   if (!h || !ms) return CSP_EINVAL;
   *ms = h->last_ms;
+  return CSP_OK;
+}
+
+extern "C" int csp_step_launches(const csp_handle* h, int64_t* n) {
+  if (!h || !n) return CSP_EINVAL;
+  *n = h->march_launches;
   return CSP_OK;
 }
 

@@ -277,6 +277,10 @@ int csp_get_stream(const csp_handle* h, void** stream);
 /* Device time in ms of the last csp_advance call (CUDA events on the handle stream). */
 int csp_last_advance_ms(const csp_handle* h, float* ms);
 
+/* Launches of the step kernel by this handle so far.  A call takes its steps in as few launches
+ * as keep each at about 0.1 s, since a launch holds the whole GPU. */
+int csp_step_launches(const csp_handle* h, int64_t* n);
+
 /* Advance like csp_advance, but with a launch per step and CUDA events around its parts:
  * voxel_ms receives the summed device times of the voxels' updates with their boundary fluxes
  * and gating, boundary_ms those of the surrogate's corrections and the step counter. */
