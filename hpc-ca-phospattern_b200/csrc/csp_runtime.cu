@@ -1536,7 +1536,7 @@ static void launch_surrogate(csp_handle* h, int r0, int r1) {
 }
 
 static void launch_epilogue(csp_handle* h, int r0, int r1, int* step_flags) {
-  k_epilogue<<<(r1 - r0 + 127) / 128, 128, 0, h->stream>>>(h->d_desc + r0, h->d_ctl + r0, h->d_rec + r0, r1 - r0,
+  k_epilogue<<<std::max(1, (r1 - r0 + 127) / 128), 128, 0, h->stream>>>(h->d_desc + r0, h->d_ctl + r0, h->d_rec + r0, r1 - r0,
                                                            step_flags, h->surrogate ? h->d_sur_queue : nullptr);
 }
 
@@ -2536,11 +2536,13 @@ extern "C" int csp_set_kernel(csp_handle* h, int32_t which) {
 
 // ---- autotuner ----
 // Candidates: the number of teams of the step kernel (realisations in flight) and the x
-// segments per realisation, around the estimate's choice, and the direct kernel.  Each runs TUNE_STEPS steps
-// `repeats` times at the current step without going on (MARCH_REPEAT: the buffers read stay
-// current, the next ones are written again; the channels' gating is left out), so that the
-// fields' place in L2 or HBM counts as in a run; no side effect stays, and every candidate
-// gives bitwise equal fields.
+// segments per realisation, around the estimate's choice, and the direct kernel.  Each runs
+// TUNE_STEPS whole steps `repeats` times at the current step without going on (MARCH_REPEAT: the
+// buffers read stay current, the next ones are written again, the channels draw the same), so
+// that the fields' place in L2 or HBM counts as in a run.  Both kinds are timed as a run has
+// them: the step kernel without its launch, which a run has once for many steps, the direct
+// kernel with all of its launches per step.  The channels counted are put back; no side effect
+// stays, and every candidate gives bitwise equal fields.
 constexpr int TUNE_STEPS = 4;
 extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep) {
   if (!h) return CSP_EINVAL;
@@ -2577,15 +2579,18 @@ extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep
   int best = -1;
   MarchPlan best_plan;
   bool direct = false;
-  cudaError_t e = cudaSuccess;
-  auto timed = [&](auto launch, float* ms) {
+  float launch_ms = 0.f;                  // of a launch of the step kernel without a step
+  std::vector<RealCtl> ctl(h->n);
+  cudaError_t e = cudaMemcpyAsync(ctl.data(), h->d_ctl, h->n * sizeof(RealCtl), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  auto timed = [&](auto launch, float over, float* ms) {
     cudaEventRecord(e0, h->stream);
     launch();                                                   // warm-up
     cudaEventRecord(e1, h->stream);
     cudaError_t w = cudaEventSynchronize(e1);
     if (w != cudaSuccess) return w;
     cudaEventElapsedTime(ms, e0, e1);
-    *ms /= TUNE_STEPS;
+    *ms = std::max(*ms - over, 0.f) / TUNE_STEPS;
     if (best >= 0 && *ms > 2.f * local.ms[best]) return cudaGetLastError();    // far behind already
     cudaEventRecord(e0, h->stream);
     for (int k = 0; k < repeats; k++) launch();
@@ -2593,9 +2598,14 @@ extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep
     cudaError_t x = cudaEventSynchronize(e1);
     if (x == cudaSuccess) x = cudaGetLastError();
     cudaEventElapsedTime(ms, e0, e1);
-    *ms /= (float)repeats * TUNE_STEPS;
+    *ms = std::max(*ms / repeats - over, 0.f) / TUNE_STEPS;
     return x;
   };
+  const unsigned what = (MARCH_STEP & ~MARCH_ADVANCE) | MARCH_REPEAT;
+  if (e == cudaSuccess) {
+    e = timed([&]() { launch_march(h, *def, 0, what); }, 0.f, &launch_ms);
+    launch_ms *= TUNE_STEPS;
+  }
   for (int i = 0; i < ncand && e == cudaSuccess && rc == CSP_OK; i++) {
     MarchPlan pl;
     rc = make_plan(h, 0, h->n, cand[i][0], cand[i][1], pl);
@@ -2603,7 +2613,7 @@ extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep
     const int k = local.n++;
     local.threads[k] = MARCH_T;
     local.segment[k] = (nx0 + pl.nseg - 1) / pl.nseg;
-    e = timed([&]() { launch_march(h, pl, TUNE_STEPS, MARCH_UNITS | MARCH_VOXELS | MARCH_REPEAT); }, &local.ms[k]);
+    e = timed([&]() { launch_march(h, pl, TUNE_STEPS, what); }, launch_ms, &local.ms[k]);
     if (e == cudaSuccess && (best < 0 || local.ms[k] < local.ms[best])) {
       free_plan(best_plan);
       best = k;
@@ -2613,7 +2623,8 @@ extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep
     }
   }
   if (e == cudaSuccess && rc == CSP_OK) {
-    // the direct kernel with its density rows, which only write the next buffers too
+    // the direct kernel with its rows, which only write the next buffers and channel states
+    // too, and an epilogue over no realisation
     const int k = local.n++;
     local.threads[k] = 256;
     local.segment[k] = -1;
@@ -2621,12 +2632,16 @@ extern "C" int csp_autotune(csp_handle* h, int32_t repeats, csp_tune_report* rep
       for (int s = 0; s < TUNE_STEPS; s++) {
         launch_direct(h, 0, h->n);
         launch_density_rows(h, 0, h->n);
+        launch_channel_rows(h, 0, h->n);
+        launch_epilogue(h, 0, 0, nullptr);
       }
-    }, &local.ms[k]);
+    }, 0.f, &local.ms[k]);
     direct = e == cudaSuccess && local.ms[k] < local.ms[best];
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(h->d_ctl, ctl.data(), h->n * sizeof(RealCtl), cudaMemcpyHostToDevice, h->stream);
   if (e != cudaSuccess || rc != CSP_OK) {
     free_plan(best_plan);
     return rc != CSP_OK ? rc : fail(h, CSP_ECUDA, "autotune: %s", cudaGetErrorString(e));
