@@ -184,10 +184,8 @@ struct FluxRow {
   unsigned char species, dsi, kind, owner, boundary, apply;
   unsigned char doms;     // first pair: domain ids of v0 (bits 0-2) and v1 (bits 3-5)
   unsigned char pad1;
-  int first_pair;         // index of the first pair
-  int pad2[3];
 };
-static_assert(sizeof(FluxRow) % 16 == 0, "whole 16-byte words");
+static_assert(sizeof(FluxRow) == 64, "a flux row is one 64-byte line");
 
 // A voxel of a group with CODE_MIXED.  code: bits 0-2 its domain id, bits 3-20 the ids of the
 // neighbours z-, z+, y-, y+, x-, x+ (3 bits each, its own for those outside the box), bits

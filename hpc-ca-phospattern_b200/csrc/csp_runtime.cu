@@ -958,6 +958,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     return a.pair < b.pair;
   });
   std::vector<FluxRow> rows;
+  std::vector<int> first_pair;          // by row
   std::vector<FluxEntry> entries;
   for (size_t i = 0; i < sides.size();) {
     size_t j = i;
@@ -971,7 +972,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       row.local_channel = p0.local_channel; row.sign = sides[i].sign;
       row.dsi = (unsigned char)p0.dsi; row.kind = (unsigned char)p0.kind; row.owner = (unsigned char)sides[i].owner;
       row.boundary = (unsigned char)p0.boundary;
-      row.first_pair = sides[i].pair;
+      first_pair.push_back(sides[i].pair);
       row.doms = (unsigned char)p0.doms;
     }
     j = i + 1;
@@ -1073,7 +1074,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
           }
           channel = channel || chan;
         };
-        add(rw.first_pair, rw.sign, rw.owner);
+        add(first_pair[order[q - 1]], rw.sign, rw.owner);
         for (int e = rw.more_begin; e < rw.more_end; e++) add(entries[e].pair, entries[e].sign, entries[e].owner);
       }
       if (!(m.item.meta & MIX_NONE)) (first ? m.item : items.back()).meta |= MIX_LAST;
