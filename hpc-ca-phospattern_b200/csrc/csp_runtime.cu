@@ -417,7 +417,7 @@ int derive(const csp_model& m, const csp_options& o, Derived& dv, std::string& e
 
 // The voxels of realisation r's groups that carry CODE_MIXED, in index order.
 void mix_voxels(const RealDesc& D, int r, const unsigned char* code,
-                const std::vector<unsigned char>& dom, std::vector<MixVoxel>& out) {
+                const unsigned char* dom, std::vector<MixVoxel>& out) {
   for (int x = 0; x < D.nx; x++)
     for (int y = 0; y < D.ny; y++) {
       const unsigned row = (unsigned)x * D.P + (unsigned)y * D.nz;
@@ -637,9 +637,8 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   std::vector<unsigned char> states0;
   std::vector<RealCtl> ctl(n);
   size_t foff = 0, doff = 0;
-  std::vector<unsigned char> hostd;
+  std::vector<unsigned char> doms(dom_total);           // domain bytes of every realisation
   std::vector<unsigned char> codes(dom_total / 4);      // group codes of every realisation
-  std::vector<MixVoxel> mix;
   for (int r = 0; r < n; r++) {
     const csp_model& m = models[r];
     const csp_options& o = options[r];
@@ -767,7 +766,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     doff += hr.field_elems;
     hr.dV = d.h * d.h * d.h;
     // species voxel domains (species.c:596-605) and the initial state (species.c:887-935)
-    hostd.assign(hr.field_elems, 0);
+    unsigned char* const hostd = doms.data() + (D.dom - h->d_dom);
     long gcount[ND] = {0};
     for (int x = 0; x < d.nx; x++)
       for (int y = 0; y < d.ny; y++)
@@ -849,7 +848,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
         pairs.push_back(p);
       }
     }
-    cudaMemcpyAsync((void*)D.dom, hostd.data(), hr.field_elems, cudaMemcpyHostToDevice, h->stream);
+    cudaMemcpyAsync((void*)D.dom, hostd, hr.field_elems, cudaMemcpyHostToDevice, h->stream);
     {
       InitTable init;
       for (int dd = 0; dd < ND; dd++)
@@ -864,7 +863,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       k_init_fields<<<dim3((unsigned)((quads + 255) / 256), (unsigned)D.ns), 256, 0, h->stream>>>(
           D.dom, D.u[0][0], hr.field_elems, quads, init);
     }
-    // group codes, then the voxels of the groups that are not uniform or receive flux
+    // group codes: uniform, or CODE_MIXED for now
     {
       const long long groups = (long long)D.nx * (D.P / 4);
       const size_t first = (size_t)(D.dom - h->d_dom) / 4;
@@ -878,7 +877,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       const size_t uniform = groups - std::count(codes.begin() + first, codes.begin() + first + groups, CODE_MIXED);
       hr.dense = D.react_fast && dom_total >= MIX_GROUPS_MIN && (double)uniform < MIX_DENSE * D.nx * (D.plane / 4);
       if (hr.dense) std::fill(codes.begin() + first, codes.begin() + first + groups, CODE_MIXED);
-      mix_voxels(D, r, codes.data() + first, hostd, mix);
     }
     // initial channel states (BoundaryFluxes_init_stochastic_boundaries, boundaryfluxes.c:544-605)
     int ndiscrete = 0;
@@ -1003,6 +1001,9 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   // order, the items of a voxel in (species, pair) order
   std::vector<MixItem> items;
   std::vector<MixVoxel> mixc;           // voxels with a channel pair
+  std::vector<MixVoxel> mix;            // the others
+  std::vector<MixGroup> grp;            // irregular groups
+  std::vector<int> grp_of;              // their realisations
   std::vector<int> places;              // MixVoxel::r of their device copies
   std::vector<std::vector<GroupPattern>> pats(n);
   std::vector<int> serca(n, -1);
@@ -1011,9 +1012,9 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   {
     std::vector<int> order(rows.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-      return rows[a].r != rows[b].r ? rows[a].r < rows[b].r : rows[a].v < rows[b].v;
-    });
+    auto before = [&](int a, int b) { return rows[a].r != rows[b].r ? rows[a].r < rows[b].r : rows[a].v < rows[b].v; };
+    if (!std::is_sorted(order.begin(), order.end(), before))     // (fluxes of several species)
+      std::stable_sort(order.begin(), order.end(), before);
     std::vector<MixVoxel> rest;
     size_t q = 0;
     MixVoxel group[4] = {};             // the voxels of the group in hand
@@ -1042,80 +1043,85 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       }
       ng = 0;
     };
-    for (MixVoxel m : mix) {
-      bool channel = false, first = true;      // first: only the inline item so far
-      int place = 0;
-      if (ng > 0 && (group[0].r != m.r || group[0].v / 4 != m.v / 4)) flush();
-      while (q < order.size() && rows[order[q]].r == m.r && rows[order[q]].v == m.v) {
-        const FluxRow& rw = rows[order[q++]];
-        auto add = [&](int pair, float sign, int owner) {
-          const FluxPair& p = pairs[pair];
-          const bool to = sign > 0.f, chan = p.channel >= 0;
-          const unsigned d0 = p.doms & DOMAIN_BITS, d1 = (p.doms >> 3) & DOMAIN_BITS;
-          MixItem it;
-          it.vo = (unsigned)(to ? p.v0 : p.v1);
-          it.pair = pair;
-          it.more = 0;
-          it.meta = (rw.apply ? MIX_APPLY : 0u) | (to ? MIX_TO : 0u) |
-                    (p.kind == FLUX_SERCA && !chan && p.param == serca[m.r] ? MIX_SERCA : 0u) | (owner ? MIX_OWNER : 0u) |
-                    (unsigned)p.species << 8 | (unsigned)p.dsi << 16 | (to ? d1 : d0) << 24 | (to ? d0 : d1) << 27;
-          if (m.item.meta & MIX_NONE) {
-            if (chan && p.kind != FLUX_SERCA && p.local_channel < (1 << 24) && p.boundary < 128) {
-              it.meta |= MIX_CHANNEL | (p.kind == FLUX_P_RYR ? MIX_PRYR : 0u);
-              m.chan = p.channel;
-              place = p.local_channel | p.boundary << 24;
-            }
-            m.item = it;
-          } else {
-            MixItem& prev = first ? m.item : items.back();
-            prev.more = (int)items.size();
-            first = false;
-            items.push_back(it);
+    // irregular groups of `rest` as groups where the batch has many
+    bool many = false;
+    auto regroup = [&]() {
+      for (size_t i = 0; i < rest.size();) {
+        const int r = rest[i].r;
+        const HostReal& hr = h->real[r];
+        const RealDesc& D = hr.desc;
+        int faces[6];                   // x-, y-, z-, z+, y+, x+ as device directions
+        for (int a = 0; a < 3; a++) {
+          const int physical = hr.perm[a];
+          faces[physical] = (2 - a) * 2;
+          faces[5 - physical] = (2 - a) * 2 + 1;
+        }
+        while (i < rest.size() && rest[i].r == r) {
+          size_t j = i + 1;
+          while (j < rest.size() && rest[j].r == r && rest[j].v / 4 == rest[i].v / 4) j++;
+          const int z = rest[i].v % D.P % D.nz;
+          MixGroup g;
+          if (D.react_fast && z % 4 == 0 && (int)(j - i) == std::min(4, D.nzv - z) &&
+              irregular_group(D, &rest[i], (int)(j - i), items, faces, g)) {
+            grp.push_back(g);
+            grp_of.push_back(r);
+            i = j;
           }
-          channel = channel || chan;
-        };
-        add(first_pair[order[q - 1]], rw.sign, rw.owner);
-        for (int e = rw.more_begin; e < rw.more_end; e++) add(entries[e].pair, entries[e].sign, entries[e].owner);
+          for (; i < j; i++) mix.push_back(rest[i]);
+        }
       }
-      if (!(m.item.meta & MIX_NONE)) (first ? m.item : items.back()).meta |= MIX_LAST;
-      group[ng] = m;
-      place_of[ng] = place;
-      chan_of[ng++] = channel;
-    }
-    if (ng) flush();
-    mix.swap(rest);
-  }
-  // batches with many irregular voxels: those as groups
-  const size_t irregular = mix.size();
-  std::vector<MixGroup> grp;
-  std::vector<int> grp_of;              // their realisations
-  for (size_t i = 0, k = 0; i < mix.size();) {
-    const int r = mix[i].r;
-    size_t end = i;
-    while (end < mix.size() && mix[end].r == r) end++;
-    const HostReal& hr = h->real[r];
-    const RealDesc& D = hr.desc;
-    int faces[6];                       // x-, y-, z-, z+, y+, x+ as device directions
-    for (int a = 0; a < 3; a++) {
-      const int physical = hr.perm[a];
-      faces[physical] = (2 - a) * 2;
-      faces[5 - physical] = (2 - a) * 2 + 1;
-    }
-    const bool many = irregular >= MIX_GROUPS_MIN && D.react_fast;
-    while (i < end) {
-      size_t j = i + 1;
-      while (j < end && mix[j].v / 4 == mix[i].v / 4) j++;
-      const int z = mix[i].v % D.P % D.nz;
-      MixGroup g;
-      if (many && z % 4 == 0 && (int)(j - i) == std::min(4, D.nzv - z) &&
-          irregular_group(D, &mix[i], (int)(j - i), items, faces, g)) {
-        grp.push_back(g);
-        grp_of.push_back(r);
-        i = j;
+      rest.clear();
+    };
+    std::vector<MixVoxel> mine;         // the voxels of a realisation's CODE_MIXED groups
+    for (int r = 0; r < n; r++) {
+      mine.clear();
+      const size_t at = (size_t)(h->real[r].desc.dom - h->d_dom);
+      mix_voxels(h->real[r].desc, r, codes.data() + at / 4, doms.data() + at, mine);
+      for (MixVoxel m : mine) {
+        bool channel = false, first = true;      // first: only the inline item so far
+        int place = 0;
+        if (ng > 0 && (group[0].r != m.r || group[0].v / 4 != m.v / 4)) flush();
+        while (q < order.size() && rows[order[q]].r == m.r && rows[order[q]].v == m.v) {
+          const FluxRow& rw = rows[order[q++]];
+          auto add = [&](int pair, float sign, int owner) {
+            const FluxPair& p = pairs[pair];
+            const bool to = sign > 0.f, chan = p.channel >= 0;
+            const unsigned d0 = p.doms & DOMAIN_BITS, d1 = (p.doms >> 3) & DOMAIN_BITS;
+            MixItem it;
+            it.vo = (unsigned)(to ? p.v0 : p.v1);
+            it.pair = pair;
+            it.more = 0;
+            it.meta = (rw.apply ? MIX_APPLY : 0u) | (to ? MIX_TO : 0u) |
+                      (p.kind == FLUX_SERCA && !chan && p.param == serca[m.r] ? MIX_SERCA : 0u) | (owner ? MIX_OWNER : 0u) |
+                      (unsigned)p.species << 8 | (unsigned)p.dsi << 16 | (to ? d1 : d0) << 24 | (to ? d0 : d1) << 27;
+            if (m.item.meta & MIX_NONE) {
+              if (chan && p.kind != FLUX_SERCA && p.local_channel < (1 << 24) && p.boundary < 128) {
+                it.meta |= MIX_CHANNEL | (p.kind == FLUX_P_RYR ? MIX_PRYR : 0u);
+                m.chan = p.channel;
+                place = p.local_channel | p.boundary << 24;
+              }
+              m.item = it;
+            } else {
+              MixItem& prev = first ? m.item : items.back();
+              prev.more = (int)items.size();
+              first = false;
+              items.push_back(it);
+            }
+            channel = channel || chan;
+          };
+          add(first_pair[order[q - 1]], rw.sign, rw.owner);
+          for (int e = rw.more_begin; e < rw.more_end; e++) add(entries[e].pair, entries[e].sign, entries[e].owner);
+        }
+        if (!(m.item.meta & MIX_NONE)) (first ? m.item : items.back()).meta |= MIX_LAST;
+        group[ng] = m;
+        place_of[ng] = place;
+        chan_of[ng++] = channel;
       }
-      for (; i < j; i++) mix[k++] = mix[i];
+      if (ng) flush();
+      many = many || rest.size() >= MIX_GROUPS_MIN;
+      if (many) regroup();
     }
-    if (i == mix.size()) mix.resize(k);
+    if (!many) mix.swap(rest);
   }
   h->nrows = (int)rows.size();
   // rows touched by density pairs only first (gating-free launch), channel rows after
