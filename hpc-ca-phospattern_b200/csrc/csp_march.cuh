@@ -1056,10 +1056,11 @@ struct MarchPlan {
   int nseg = 0;                      // segments of the first realisation
   bool known = false;                // march_kernel
   double step_us = 0.0;              // estimated time of a step
-  MarchReal* d_real = nullptr;
-  int* d_first = nullptr;
-  int* d_cuts = nullptr;
+  // one allocation, from d_arrived on
   unsigned* d_arrived = nullptr;
+  const MarchReal* d_real = nullptr;
+  const int* d_first = nullptr;
+  const int* d_cuts = nullptr;
 };
 
 // Cost of a plane by what its warps meet, and of the rest of a step, in us of a warp with the
@@ -1086,16 +1087,25 @@ inline double march_cut(const std::vector<double>& acc, int n, std::vector<int>*
   return worst;
 }
 
-// Estimated time (us) of one step of a realisation (columns ncol, cost sums acc, `tiles`
+// march_cut's largest segment for 1, 2, ... segments: made once per realisation, since a plan asks
+// for it for every number of teams.
+inline std::vector<double> march_largest(const std::vector<double>& acc) {
+  const int nx = (int)acc.size() - 1, most = std::min(nx, MARCH_CUTS - 1);
+  std::vector<double> w(most);
+  for (int n = 1; n <= most; n++) w[n - 1] = march_cut(acc, n, nullptr);
+  return w;
+}
+
+// Estimated time (us) of one step of a realisation (columns ncol, march_largest, `tiles`
 // boundary tiles) by a team of `size` CTAs: its items per CTA in rounds of its warps, and the
 // barrier.  *nseg: the segments that give it (in: those to use, if positive).
-inline double march_cost(long long ncol, const std::vector<double>& acc, long long tiles, int size, int* nseg) {
-  const int nx = (int)acc.size() - 1, W = MARCH_T / 32;
+inline double march_cost(long long ncol, const std::vector<double>& largest, long long tiles, int size, int* nseg) {
+  const int W = MARCH_T / 32;
   double best = 1e300;
-  const int most = std::min(nx, MARCH_CUTS - 1), given = nseg ? *nseg : 0;
+  const int most = (int)largest.size(), given = nseg ? *nseg : 0;
   int found = 1;
   for (int n = given > 0 ? std::min(given, most) : 1; n <= most; n++) {
-    const double unit = MARCH_US_START + march_cut(acc, n, nullptr);
+    const double unit = MARCH_US_START + largest[n - 1];
     const long long nu = (ncol * n + size - 1) / size, nt = (tiles + size - 1) / size;
     const long long full = nu / W, part = nu % W;      // rounds of units, then the tiles
     double t = full * unit;

@@ -59,6 +59,7 @@ struct HostReal {
   FluxParams gate[2] = {};        // RyR, pRyR
   bool dense = false;             // every group is boundary work (MIX_DENSE)
   std::vector<double> acc;        // prefix sums of the planes' costs (march_cut)
+  std::vector<double> largest;    // march_largest
   // padded linear device index of physical species voxel (x, y, z)
   long long dev_index(int x, int y, int z) const {
     const int c[3] = {x, y, z};
@@ -1293,6 +1294,8 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
   std::vector<int> order(n);
   for (int i = 0; i < n; i++) order[i] = r0 + i;
   auto desc = [&](int r) -> const RealDesc& { return h->real[r].desc; };
+  for (int r = r0; r < r1; r++)
+    if (h->real[r].largest.empty()) h->real[r].largest = march_largest(h->real[r].acc);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return working_set(desc(a)) > working_set(desc(b)); });
   auto columns = [&](int r) { return h->real[r].dense ? 0 : (desc(r).plane + MARCH_COL - 1) / MARCH_COL; };
   auto tiles_of = [&](int r) {
@@ -1314,13 +1317,9 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
   auto deal = [&](int t, std::vector<std::vector<int>>* out) {
     const int size = size_of(t);
     std::vector<double> load(t, 0.0);
-    double last = 0.0;
     for (int i = 0; i < n; i++) {
-      const RealDesc& D = desc(order[i]);
-      const bool same = i > 0 && D.nx == desc(order[i - 1]).nx && D.plane == desc(order[i - 1]).plane;
-      if (!same) last = march_cost(columns(order[i]), h->real[order[i]].acc, tiles_of(order[i]), size, nullptr);
       const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-      load[k] += last;
+      load[k] += march_cost(columns(order[i]), h->real[order[i]].largest, tiles_of(order[i]), size, nullptr);
       if (out) (*out)[k].push_back(order[i]);
     }
     return *std::max_element(load.begin(), load.end());
@@ -1352,7 +1351,7 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
       m.r = r;
       m.ncol = columns(r);
       m.nseg = nseg;
-      march_cost(m.ncol, h->real[r].acc, tiles_of(r), pl.size, &m.nseg);
+      march_cost(m.ncol, h->real[r].largest, tiles_of(r), pl.size, &m.nseg);
       if (real.empty()) pl.nseg = m.nseg;
       march_cut(h->real[r].acc, m.nseg, &one);
       m.cut0 = (int)cuts.size();
@@ -1367,23 +1366,25 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
     }
     first.push_back((int)real.size());
   }
-  if (cudaMalloc(&pl.d_real, real.size() * sizeof(MarchReal)) != cudaSuccess ||
-      cudaMalloc(&pl.d_first, first.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&pl.d_cuts, cuts.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&pl.d_arrived, (size_t)best * 32 * sizeof(unsigned)) != cudaSuccess)
+  // one allocation and one copy: arrivals (0), realisations, teams, cuts
+  static_assert(sizeof(MarchReal) % sizeof(int) == 0, "an array of ints");
+  const size_t n_arrived = (size_t)best * 32, n_real = real.size() * (sizeof(MarchReal) / sizeof(int));
+  std::vector<int> mem(n_arrived + n_real, 0);
+  memcpy(mem.data() + n_arrived, real.data(), n_real * sizeof(int));
+  mem.insert(mem.end(), first.begin(), first.end());
+  mem.insert(mem.end(), cuts.begin(), cuts.end());
+  if (cudaMalloc(&pl.d_arrived, mem.size() * sizeof(int)) != cudaSuccess)
     return fail(h, CSP_ENOMEM, "launch plan of %d realisations", n);
-  CUDA_TRY(h, cudaMemcpyAsync(pl.d_real, real.data(), real.size() * sizeof(MarchReal), cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(pl.d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(pl.d_cuts, cuts.data(), cuts.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(h, cudaMemsetAsync(pl.d_arrived, 0, (size_t)best * 32 * sizeof(unsigned), h->stream));
+  const int* d = reinterpret_cast<const int*>(pl.d_arrived);
+  pl.d_real = reinterpret_cast<const MarchReal*>(d + n_arrived);
+  pl.d_first = d + n_arrived + n_real;
+  pl.d_cuts = pl.d_first + first.size();
+  CUDA_TRY(h, cudaMemcpyAsync(pl.d_arrived, mem.data(), mem.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return CSP_OK;
 }
 
 static void free_plan(MarchPlan& p) {
-  cudaFree(p.d_real);
-  cudaFree(p.d_first);
-  cudaFree(p.d_cuts);
   cudaFree(p.d_arrived);
   p = MarchPlan();
 }
@@ -2038,6 +2039,12 @@ static int run_states(csp_handle* h, const T* const* uin, int64_t nsteps, T* con
       return fail(h, CSP_ENOMEM, "per-step flags of %lld steps", (long long)nsteps);
     h->stepflags_elems = (size_t)nsteps * h->n;
   }
+  // the plans before the pipeline: making one allocates and waits
+  if (h->kernel != 1 && nsteps > 0)
+    for (int g = 0; g < G; g++) {
+      const MarchPlan* pl;
+      if (const int rc = plan_for(h, gb[g], gb[g + 1], &pl)) return rc;
+    }
   if (!h->in_stream) CUDA_TRY(h, cudaStreamCreateWithFlags(&h->in_stream, cudaStreamNonBlocking));
   if (!h->snap_stream) {
     CUDA_TRY(h, cudaStreamCreateWithFlags(&h->snap_stream, cudaStreamNonBlocking));
