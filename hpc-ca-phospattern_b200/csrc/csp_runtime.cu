@@ -2760,6 +2760,8 @@ extern "C" int csp_set_surrogate(csp_handle* h, const float* params, double tol)
     }
     CUDA_TRY(h, cudaMemcpyAsync(h->d_mlp, params, MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     h->surrogate_tol = (float)tol;
+    // the direct kernel's graph holds the tolerance of its capture
+    if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
   }
   if (on && !h->d_rx_class) {
     size_t bytes = 0;
