@@ -32,23 +32,32 @@ def blocks(synth, spec, seed, size, all_serca=True):
     ((48, 40, 43), 3, False, dict(dt_update_react=3.01 * DT)),
     ((47, 48, 37), 2, True, dict(fixed=[(0, 0), (1, 1), (3, 0)], dt_update_stoch=2.01 * DT)),
     ((34, 52, 49), 5, True, dict(surrogate=True, dt_update_react=3.01 * DT)),
+    ((46, 40, 47), 2, True, dict(surrogate=True, dt_update_react=2.01 * DT)),
+    ((44, 46, 42), 2, True, dict(species=6)),
 ])
 def test_bitwise(pkg, synth, shape, size, all_serca, o):
-    o = dict(o)
+    """Five realisations: 400,000 voxels, above the irregular ones from which groups are taken."""
+    o, n = dict(o), 5
     spec = blocks(synth, synth.tiny(shape), 7, size, all_serca)
+    for k in range(5, o.pop("species", 5)):                  # further fixed-point buffers
+        spec["species"] = list(spec["species"]) + ["X%d" % k]
+        spec["domain_species"] = {d: dict(v, init=list(v["init"]) + [5.0 if d == "cyt" else 0.0],
+                                          buffers=list(v["buffers"]) + (d == "cyt") * [
+                                              dict(species=[k, 0], k_on=0.02, k_off=0.1, tot=30.0)])
+                                  for d, v in spec["domain_species"].items()}
     spec["fixed_domain_species"] = o.pop("fixed", [])
     surrogate = o.pop("surrogate", False)
     opts = dict(h=6.0, tstop=5.0, seed=3, open_states={"ryr": [0, 1, 2]}, **o)
     got = []
     for kernel in (0, 1):
-        sim = pkg.Simulation([spec, spec], [opts, dict(opts, seed=5)])
+        sim = pkg.Simulation([spec] * n, [dict(opts, seed=3 + r) for r in range(n)])
         sim.set_kernel(kernel)
         if surrogate:
             sim.set_surrogate(pkg.mlp_init(5), 1e-4)
         sim.advance(24)
-        got.append([sim.state(r) for r in range(2)])
+        got.append([sim.state(r) for r in range(n)])
         sim.close()
-    for r in range(2):
+    for r in range(n):
         assert np.isfinite(got[0][r]).all()
         np.testing.assert_array_equal(got[0][r], got[1][r])
 
