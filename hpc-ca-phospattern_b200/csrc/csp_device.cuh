@@ -5,8 +5,7 @@
 // u1 / du pair, species.h:52-53, become a double buffer: a step reads the current
 // buffer and writes the other one) and one uint8 domain-id field.  Every field is
 // [nx][P] with P = ny*nz rounded up to a multiple of 128 elements, so each x-plane
-// starts on a 512-byte boundary (float) / 128-byte boundary (uint8) and can be moved by
-// 16-byte aligned bulk copies.  Within a plane the index is p = y*nz + z (z fastest,
+// starts on a 512-byte boundary (float) / 128-byte boundary (uint8).  Within a plane the index is p = y*nz + z (z fastest,
 // species.c:1513), where nz is the row length nzv of the grid rounded up to a multiple of
 // 4: a group of 4 positions lies in one row, and every row starts on a 16-byte boundary
 // whatever the grid's size (the positions z >= nzv hold no voxel).
@@ -125,19 +124,17 @@ struct RealCtl {
   double last_closed;                // abort rule bookkeeping
 };
 
-// What a realisation's running step does (flags: STEP_*), for the voxel and density-row kernels: written at
-// creation and by the step epilogue for the next step (16-byte loads).
+// Flags of a step: a reaction step, its reactions by the per-species tables, a gating step.
 enum : unsigned { STEP_REACT = 1u, STEP_REACT_FAST = 2u, STEP_GATE = 4u };
+// What a realisation's running step does, for the density-row kernel and the epilogue: written at
+// creation, by the step kernel and by the epilogue for the next step (a 16-byte load).
 struct alignas(16) StepRec {
   unsigned active;                   // not stopped
   unsigned cur;                      // bit s: index of the current buffer of species s
   unsigned updated;                  // species written by the step
   unsigned sub;                      // bit dsi: diffusive index dsi takes its substep (and its fluxes)
-  unsigned pre;                      // species that diffuse this step
-  unsigned flags;                    // STEP_REACT: a reaction step; STEP_REACT_FAST: by the per-species tables
-  unsigned pad[2];
 };
-static_assert(sizeof(StepRec) == 32, "two 16-byte loads");
+static_assert(sizeof(StepRec) == 16, "one 16-byte load");
 
 // A density-boundary row in 32 bytes (two 16-byte loads): the receiving voxel, the other
 // voxel of its first pair, the first pair's law with the SERCA scale inline, and the
@@ -248,7 +245,6 @@ struct alignas(16) VoxDesc {
   // of being packed by two moves per use
   unsigned long long rk2[ND][NS][4];
   float* u[2][NS];
-  const unsigned char* dom;
   const unsigned char* gcode;
   unsigned char* rx_class;
   float cdiag[ND][NS];

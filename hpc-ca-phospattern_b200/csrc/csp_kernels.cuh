@@ -415,13 +415,10 @@ __global__ void __launch_bounds__(256, CH ? 4 : 8) k_boundaries(const RealDesc* 
 __host__ __device__ inline void write_steprec(const RealDesc& D, const RealCtl& C, StepRec& R) {
   unsigned pre, updated, sub;
   step_masks(D, C.step + 1, pre, updated, sub);
-  const StepInfo si = step_info(D, C.step + 1);
   R.active = C.stopped ? 0u : 1u;
   R.cur = C.cur_mask[C.step & 1];
   R.updated = updated;
   R.sub = sub;
-  R.pre = si.pre;
-  R.flags = (si.react ? STEP_REACT : 0u) | (si.react_fast ? STEP_REACT_FAST : 0u);
 }
 
 // Density-boundary rows (voxels touched by density pairs only: the SERCA sheets), one

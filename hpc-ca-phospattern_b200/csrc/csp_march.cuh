@@ -21,8 +21,8 @@
 // neighbourhood lie in it and no voxel of it receives boundary flux, or a pattern (regular
 // groups along domain sheets: coefficients per direction, SERCA flux from the values at hand).
 // A warp whose groups are all uniform takes the leaner of two forms of the loop body.  The
-// voxels of irregular groups and those with channels are the boundary work (mixed_voxel), in
-// tiles of 32; where there are many, irregular groups are, in tiles of 32 groups (mixed_group).
+// voxels of irregular groups and those with channels are the boundary work, in tiles of 32
+// (mixed_voxel); a batch with many irregular voxels has them in tiles of 32 groups (mixed_group).
 //
 // The barrier's wait is bounded in time (MarchArgs::wait_ns).  A CTA that gives up sets ERR_TIMEOUT in the
 // device error word, which the other waits see too, and every CTA leaves the launch; the fields
@@ -84,8 +84,8 @@ struct MarchArgs {
   unsigned what;                     // MARCH_*
   MixArgs mix;
   unsigned* arrived;                 // [teams * 32]: CTAs arrived at the team's barriers, 0 before the launch
-  int* flags;                        // nullable [nsteps][flag_stride]: stop flag of realisation r at [r - flag_r0]
-  int flag_stride, flag_r0;
+  int* flags;                        // nullable [nsteps][flag_stride]: stop flag of realisation r at [r]
+  int flag_stride;
   int* err;
   unsigned long long wait_ns;        // limit of a wait
   int inject;                        // test hook (csp_test_wait_timeout)
@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
           if (ti >= total) stopped = 1;
           if (rank == 0) {
             C.open_count[(ti + 2) % 3] = 0;      // read after the previous barrier, counted next in two steps
-            if (A.flags) A.flags[i * A.flag_stride + R.r - A.flag_r0] = stopped;
+            if (A.flags) A.flags[i * A.flag_stride + R.r] = stopped;
           }
           S.step.k = ti;
           S.step.cur ^= done;
@@ -1031,7 +1031,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
       C.stopped = stopped;
       write_steprec(D, C, A.rec[R.r]);
       if (A.flags)
-        for (; i < A.nsteps; i++) A.flags[i * A.flag_stride + R.r - A.flag_r0] = stopped;
+        for (; i < A.nsteps; i++) A.flags[i * A.flag_stride + R.r] = stopped;
     }
     __syncthreads();                     // S is filled for the next realisation
   }

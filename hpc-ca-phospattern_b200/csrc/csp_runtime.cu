@@ -145,7 +145,7 @@ static VoxDesc make_vox_desc(const HostReal& hr) {
   for (int s = 0; s < NS; s++)
     if (D.dsi_of[s] >= 0) memcpy(v.coef[s], D.coef[D.dsi_of[s]], sizeof v.coef[s]);
   memcpy(v.u, D.u, sizeof v.u);
-  v.dom = D.dom; v.gcode = D.gcode; v.rx_class = D.rx_class;
+  v.gcode = D.gcode; v.rx_class = D.rx_class;
   memcpy(v.cdiag, D.cdiag, sizeof v.cdiag);
   memcpy(v.qunit, D.qunit, sizeof v.qunit);
   memcpy(v.qinv, D.qinv, sizeof v.qinv);
@@ -1255,12 +1255,15 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-    for (int v = 0; v < 4 && e == cudaSuccess; v++) {
-      const bool sur = v & 1, known = v >> 1;
+    // of the kernels that this batch's cooperative launches may take (asking loads a kernel)
+    for (int known = 0; known < 2 && e == cudaSuccess; known++) {
+      bool any = false;
+      for (const RealDesc& D : descs) any = any || march_masks_known(D) == (known != 0);
+      if (!any) continue;
       int k = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, march_kernel(h->ms, known, sur), MARCH_T,
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, march_kernel(h->ms, known != 0, false), MARCH_T,
                                                         sizeof(MarchShared));
-      per_sm = v == 0 ? k : std::min(per_sm, k);
+      per_sm = per_sm == 0 ? k : std::min(per_sm, k);
     }
     if (e != cudaSuccess || per_sm < 1) {
       csp_destroy(h);
@@ -1275,9 +1278,6 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
   return CSP_OK;
 }
 
-// The kernels of one step, for the realisations [r0, r1) (r1 < 0: all of them, the
-// launches csp_advance captures).  Realisations are independent, so stepping a range
-// gives that range exactly what a step of the whole batch gives it.
 // The fields of a realisation that its steps read and write: both buffers of every species,
 // group codes.
 static double working_set(const RealDesc& D) { return (double)D.nx * D.P * (8.0 * D.ns + 0.25); }
