@@ -64,8 +64,12 @@ struct MarchReal {
 // Irregular voxels of a batch from which they are taken as groups (MixGroup): with fewer, a
 // voxel per lane fills the GPU and its chain is shorter (us per step of random 2^3 blocks of
 // domains, by voxel and by group: one grid of 40x40x36 6.8 and 12.1, one of 100x100x50 34.7 and
-// 23.4, 24 of those 845 and 423; 8^3 blocks, 24 grids: 344 and 247).
+// 23.4, 24 of those 845 and 423; 8^3 blocks, 24 grids: 344 and 247).  Realisations count where
+// they are at least a share of the voxels: the sheets of a dyad leave 1 %, and their kernel
+// (MARCH_KNOWN) is the faster for having no code for groups (64 grids of 100x100x50 278 us per
+// step, with that code and their 1 % as groups 345).
 constexpr size_t MIX_GROUPS_MIN = 262144;
+constexpr double MIX_GROUPS_SHARE = 1.0 / 8;
 // Share of uniform groups below which the units of such a realisation would read its planes for
 // next to nothing: all of its groups are boundary work (24 grids of 2^3 blocks: 423 -> 374 us).
 constexpr double MIX_DENSE = 1.0 / 16;
@@ -103,6 +107,7 @@ struct MarchShared {
   alignas(16) VoxDesc desc;
   MarchStep step;
   int next;                          // items of the step that a warp has taken beyond its first
+  int next_group;                    // tiles of irregular groups taken
   // the same on every step: the segments, and the entries of the CTA's first boundary tiles
   int cut[MARCH_CUTS];
   alignas(16) int4 tile[MARCH_T][2];
@@ -830,19 +835,17 @@ __device__ __forceinline__ void mixed_group(const VoxDesc& D, const MarchStep& U
 }
 
 // A CTA's share of a realisation's step: units [u0, u1) and boundary tiles [t0, t1) (of 32
-// voxels, those with channels first, then of 32 groups), taken by its warps as they come free, units first.  Contiguous
+// voxels, those with channels first), taken by its warps as they come free, units first.  Contiguous
 // units share their columns' rows in L1; the tiles, whose lanes touch a line each, are spread
 // evenly over the CTAs (16 of them on one SM took twice the time of one).
 struct MarchShare {
-  int u0, u1, t0, t1, tc, tv, nc, nv, ng;
+  int u0, u1, t0, t1, tc, nc, nv;
   __device__ __forceinline__ MarchShare(const MarchReal& R, unsigned what, int rank, int size) {
     const long long units = (what & MARCH_UNITS) ? R.ncol * (long long)R.nseg : 0;
     nc = (what & MARCH_CHANNELS) ? R.nchan : 0;
     nv = (what & MARCH_VOXELS) ? R.nvox : 0;
-    ng = (what & MARCH_VOXELS) ? R.ngrp : 0;
     tc = (nc + 31) / 32;
-    tv = (nv + 31) / 32;
-    const long long tiles = tc + tv + (ng + 31) / 32;
+    const long long tiles = tc + (nv + 31) / 32;
     u0 = (int)(units * rank / size);
     u1 = (int)(units * (rank + 1) / size);
     // the CTAs with one unit less get the odd tiles
@@ -851,21 +854,18 @@ struct MarchShare {
   }
 };
 
-// The lane's entry (MixVoxel or MixGroup) of tile t; false: none.
+// The lane's entry of tile t; false: none.
 __device__ __forceinline__ bool march_entry(const MarchArgs& A, const MarchReal& R, const MarchShare& H, int t, int4& e0,
                                             int4& e1) {
-  const int lane = (int)(threadIdx.x & 31u);
-  const int kind = t < H.tc ? 0 : t < H.tc + H.tv ? 1 : 2;
-  const int i = (kind == 0 ? t : kind == 1 ? t - H.tc : t - H.tc - H.tv) * 32 + lane;
-  if (t >= H.t1 || i >= (kind == 0 ? H.nc : kind == 1 ? H.nv : H.ng)) return false;
-  static_assert(sizeof(MixVoxel) == 32 && sizeof(MixGroup) == 32, "two 16-byte loads");
-  const int4* e = kind == 0   ? reinterpret_cast<const int4*>(A.mix.chan + R.chan0 + i)
-                  : kind == 1 ? reinterpret_cast<const int4*>(A.mix.vox + R.vox0 + i)
-                              : reinterpret_cast<const int4*>(A.mix.grp + R.grp0 + i);
+  const bool c = t < H.tc;
+  const int i = (c ? t : t - H.tc) * 32 + (int)(threadIdx.x & 31u);
+  if (t >= H.t1 || i >= (c ? H.nc : H.nv)) return false;
+  const int4* e = reinterpret_cast<const int4*>((c ? A.mix.chan + R.chan0 : A.mix.vox + R.vox0) + i);
   e0 = __ldg(e);
   e1 = __ldg(e + 1);
   return true;
 }
+static_assert(sizeof(MixVoxel) == 32 && sizeof(MixGroup) == 32, "two 16-byte loads");
 
 // A warp's next item of the step: the CTA's units, then its boundary tiles, are taken as warps
 // come free.  Dealt in turn, the warps with a unit also got the later tiles while those that
@@ -879,7 +879,7 @@ __device__ __forceinline__ int march_next(MarchShared& S, int items) {
 }
 
 // Boundary tiles (from tile k of the CTA on, then those the warp takes next; nu: the CTA's units).
-template <int MS, unsigned FQ, bool SUR>
+template <int MS, bool SUR>
 __device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R, const MarchShare& H, int nu, int k) {
   extern __shared__ __align__(128) unsigned char smem[];
   MarchShared& S = *reinterpret_cast<MarchShared*>(smem);
@@ -895,9 +895,30 @@ __device__ __noinline__ void march_mixed(const MarchArgs& A, const MarchReal& R,
     } else {
       have = march_entry(A, R, H, H.t0 + k, e0, e1);
     }
-    if (have) {
-      if (H.t0 + k < H.tc + H.tv) mixed_voxel<MS, SUR>(S.desc, S.step, A.descs[R.r], A.ctl[R.r], A.mix, e0, e1);
-      else mixed_group<MS, FQ, SUR>(S.desc, S.step, A.descs[R.r], e0, e1);
+    if (have) mixed_voxel<MS, SUR>(S.desc, S.step, A.descs[R.r], A.ctl[R.r], A.mix, e0, e1);
+    __syncwarp();
+  }
+}
+
+// The CTA's share of the irregular groups (entry e of the team), in tiles of 32 that its warps
+// take as they come free.  A function and a counter of their own, not in MARCH_KNOWN.
+template <int MS, unsigned FQ, bool SUR>
+__device__ __noinline__ void march_groups(const MarchArgs& A, int e, int rank) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  MarchShared& S = *reinterpret_cast<MarchShared*>(smem);
+  const int r = A.real[e].r, n = A.real[e].ngrp, lane = (int)(threadIdx.x & 31u);
+  const MixGroup* entries = A.mix.grp + A.real[e].grp0;
+  const long long tiles = (n + 31) / 32;
+  const int t0 = (int)(tiles * rank / A.size), t1 = (int)(tiles * (rank + 1) / A.size);
+  while (true) {
+    int t = 0;
+    if (lane == 0) t = t0 + atomicAdd(&S.next_group, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= t1) break;
+    if (t * 32 + lane < n) {
+      const int4* g = reinterpret_cast<const int4*>(entries + t * 32 + lane);
+      const int4 e0 = __ldg(g), e1 = __ldg(g + 1);
+      mixed_group<MS, FQ, SUR>(S.desc, S.step, A.descs[r], e0, e1);
     }
     __syncwarp();
   }
@@ -942,7 +963,10 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
     double last_closed = 0.0, dt = 0.0, tabort = 0.0;
     long long total = 0;
     int stopped = 0;
-    if (tid == 0) S.next = 0;
+    if (tid == 0) {
+      S.next = 0;
+      if (BODY != MARCH_KNOWN) S.next_group = 0;
+    }
     if (warp == 0) {
       const long long k = C.step;
       const unsigned cur = C.cur_mask[k & 1];
@@ -975,7 +999,10 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
           march_dispatch<MS, FQ, SUR, BODY>(S, A.descs, R.r, col, S.cut[seg], S.cut[seg + 1]);
           __syncwarp();
         }
-        if (item < items) march_mixed<MS, FQ, SUR>(A, R, H, nu, item - nu);
+        if (item < items) march_mixed<MS, SUR>(A, R, H, nu, item - nu);
+        if constexpr (BODY != MARCH_KNOWN) {
+          if (R.ngrp > 0 && (A.what & MARCH_VOXELS)) march_groups<MS, FQ, SUR>(A, e, rank);
+        }
       }
       if (!(A.what & (MARCH_ADVANCE | MARCH_REPEAT))) break;
       __syncthreads();
@@ -1013,6 +1040,7 @@ __global__ void __launch_bounds__(MARCH_T, 1) k_march(const __grid_constant__ Ma
         }
         if (lane == 0) {
           S.next = 0;
+          if (BODY != MARCH_KNOWN) S.next_group = 0;
           S.step.go = !ok ? -1 : stopped ? 0 : 1;
         }
         if (adv && lane < NS && (done >> lane & 1u)) {

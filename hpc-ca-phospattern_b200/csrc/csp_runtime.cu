@@ -1044,8 +1044,9 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
       }
       ng = 0;
     };
-    // irregular groups of `rest` as groups where the batch has many
-    bool many = false;
+    // irregular groups of `rest` as groups, of realisations with many of them in such a batch
+    std::vector<char> share(n, 0);
+    size_t irregular = 0;               // voxels of those realisations
     auto regroup = [&]() {
       for (size_t i = 0; i < rest.size();) {
         const int r = rest[i].r;
@@ -1062,7 +1063,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
           while (j < rest.size() && rest[j].r == r && rest[j].v / 4 == rest[i].v / 4) j++;
           const int z = rest[i].v % D.P % D.nz;
           MixGroup g;
-          if (D.react_fast && z % 4 == 0 && (int)(j - i) == std::min(4, D.nzv - z) &&
+          if (share[r] && z % 4 == 0 && (int)(j - i) == std::min(4, D.nzv - z) &&
               irregular_group(D, &rest[i], (int)(j - i), items, faces, g)) {
             grp.push_back(g);
             grp_of.push_back(r);
@@ -1076,6 +1077,7 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     std::vector<MixVoxel> mine;         // the voxels of a realisation's CODE_MIXED groups
     for (int r = 0; r < n; r++) {
       mine.clear();
+      const size_t before_r = rest.size();
       const size_t at = (size_t)(h->real[r].desc.dom - h->d_dom);
       mix_voxels(h->real[r].desc, r, codes.data() + at / 4, doms.data() + at, mine);
       for (MixVoxel m : mine) {
@@ -1119,10 +1121,13 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
         chan_of[ng++] = channel;
       }
       if (ng) flush();
-      many = many || rest.size() >= MIX_GROUPS_MIN;
-      if (many) regroup();
+      const RealDesc& D = h->real[r].desc;
+      const size_t mine_left = rest.size() - before_r;
+      share[r] = D.react_fast && (double)mine_left >= MIX_GROUPS_SHARE * D.nx * D.ny * D.nzv;
+      if (share[r]) irregular += mine_left;
+      if (irregular >= MIX_GROUPS_MIN) regroup();
     }
-    if (!many) mix.swap(rest);
+    if (irregular < MIX_GROUPS_MIN) mix.swap(rest);
   }
   h->nrows = (int)rows.size();
   // rows touched by density pairs only first (gating-free launch), channel rows after
@@ -1258,7 +1263,8 @@ extern "C" int csp_create(const csp_model* models, const csp_options* options, i
     // of the kernels that this batch's cooperative launches may take (asking loads a kernel)
     for (int known = 0; known < 2 && e == cudaSuccess; known++) {
       bool any = false;
-      for (const RealDesc& D : descs) any = any || march_masks_known(D) == (known != 0);
+      for (int r = 0; r < n; r++)
+        any = any || (march_masks_known(descs[r]) && h->grp_first[r] == h->grp_first[r + 1]) == (known != 0);
       if (!any) continue;
       int k = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, march_kernel(h->ms, known != 0, false), MARCH_T,
@@ -1339,7 +1345,7 @@ static int make_plan(csp_handle* h, int r0, int r1, int teams, int nseg, MarchPl
   pl.r1 = r1;
   pl.teams = best;
   pl.size = size_of(best);
-  pl.known = true;
+  pl.known = h->grp_first[r0] == h->grp_first[r1];
   for (int r = r0; r < r1; r++) pl.known = pl.known && march_masks_known(desc(r));
   std::vector<std::vector<int>> team(best);
   pl.step_us = deal(best, &team);
