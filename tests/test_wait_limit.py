@@ -32,7 +32,7 @@ def test_waits_run_out(pkg, synth, n, stopped):
     with pytest.raises(pkg.CspError) as e:
         sim.advance(3)
     assert e.value.code == -5 and "bounded wait timed out" in str(e.value)
-    assert time.perf_counter() - t < 0.5               # the hook's limit, not the one second of other launches
+    assert time.perf_counter() - t < 0.9               # the hook's limit, not the one second of other launches
     sim.close()
     fresh = pkg.Simulation(synth.tiny((12, 12, 16)), dict(h=6.0, tstop=5.0, seed=1))
     fresh.advance(20)
